@@ -142,7 +142,7 @@ __device__ __forceinline__ int runnable(const Ctrl *c) {
 // their faces with the member's flags (BatchMember::flags), which the
 // batched indicator launch between two launches of this kernel writes.
 template <typename T, int SCHEME, int TI, int NT, bool WITHHOLD = false, bool ROUTE = false>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? 3 : 1) : 1) k_batch(BatchArgs b) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? 3 : 1) : 2) k_batch(BatchArgs b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BatchMember sM;
   constexpr int TJ = 32;

@@ -9,6 +9,7 @@
 // infinity-07/FD-WENO-EulerEquation.
 #pragma once
 
+#include "int_f64.cuh"
 #include "wenofd_internal.h"
 
 namespace wenofd {
@@ -325,19 +326,6 @@ struct Float4Stencil {  // AoS: one float4 per node, nodes `ss` float4s apart
 
 template <typename T, int DIR, int SCHEME, typename St>
 __device__ __forceinline__ void face_flux_st(T gamma, T zp_lambda, const T um[4], const T u0[4], const St &fp,
-                                             const St &fm, T out[4]);
-
-// fp / fm point at F+ of node face-3 and F- of node face-2, component 0;
-// consecutive stencil nodes are `ss` elements apart, components `cs` apart.
-template <typename T, int DIR, int SCHEME>
-__device__ __forceinline__ void face_flux(T gamma, T zp_lambda, const T um[4], const T u0[4],
-                                          const T *fp, const T *fm, int ss, int cs, T out[4]) {
-  face_flux_st<T, DIR, SCHEME>(gamma, zp_lambda, um, u0, StridedStencil<T>{fp, ss, cs},
-                               StridedStencil<T>{fm, ss, cs}, out);
-}
-
-template <typename T, int DIR, int SCHEME, typename St>
-__device__ __forceinline__ void face_flux_st(T gamma, T zp_lambda, const T um[4], const T u0[4], const St &fp,
                                              const St &fm, T out[4]) {
   T ave[4];
 #pragma unroll
@@ -407,6 +395,214 @@ __device__ __forceinline__ void face_flux_st(T gamma, T zp_lambda, const T um[4]
     f += R[r][3] * vh[3];
     out[r] = f;
   }
+}
+
+// ------------------------------------ FP64 on the FP64 and integer pipes
+//
+// The FP64 parity tile's flux split, reconstruction and face flux, bit for bit
+// flux_split, weno and face_flux_st on the values they take: sums and
+// FMAs stay on the FP64 pipe, products, reciprocals and quotients run on the
+// integer pipes (int_f64.cuh).  Fewer operations as well, each change exact:
+//  - a product by a power of two is exact, so a - 2b, the sum with
+//    (1/4 t2) t2 = 1/4 (t2 t2), 0.5 (F -+ P) and the like are one FMA;
+//  - quotients by one divisor share its reciprocal;
+//  - entries of L and R that are 0 or +-1 cost nothing (the reference adds
+//    their products, which can only change the sign of a zero; no zero's sign
+//    reaches the state, since rhs starts at +0);
+//  - rows 0, 2 and 3 of L share the products B1 u_n f_n, B1 u_t f_t and B1 f_3
+//    (times 1 or +-1/2).
+// Values outside the integer forms' domain (huge, tiny, infinite or NaN; far
+// from any flow) take the plain functions above.
+
+// One WENO-JS or WENO-Z reconstruction.  Out of line: some 1,500 instructions,
+// called eight times per face from both sweeps.
+// Stencil values are zeros or at least 2^-200, so differences are zeros or at
+// least 2^-253 and the indicators zeros or at least 2^-506; below 2^75, so no
+// product overflows.  tau/beta may be tiny: its square is taken flushing
+// subnormals to zero, which 1 + square rounds away.
+template <int SCHEME>
+__device__ __noinline__ double weno_plain(double a, double b, double c, double d, double e, double zp_lambda) {
+  return weno<double, SCHEME>(a, b, c, d, e, zp_lambda);
+}
+template <int SCHEME>
+__device__ __noinline__ double weno_int(double a, double b, double c, double d, double e) {
+  if (!(in_range<-200, 75>(a) && in_range<-200, 75>(b) && in_range<-200, 75>(c) && in_range<-200, 75>(d) &&
+        in_range<-200, 75>(e)))
+    return weno_plain<SCHEME>(a, b, c, d, e, 0.0);
+  const double c1312 = 13.0 / 12.0;
+  const double c3 = int_mul(3.0, c);
+  double t1 = fma(-2.0, b, a) + c, t2 = fma(-4.0, b, a) + c3;
+  const double bm = fma(0.25, int_mul(t2, t2), int_mul(int_mul(c1312, t1), t1));
+  t1 = fma(-2.0, c, b) + d;
+  t2 = b - d;
+  const double b0 = fma(0.25, int_mul(t2, t2), int_mul(int_mul(c1312, t1), t1));
+  t1 = fma(-2.0, d, c) + e;
+  t2 = fma(-4.0, d, c3) + e;
+  const double bp = fma(0.25, int_mul(t2, t2), int_mul(int_mul(c1312, t1), t1));
+  double w0, w1, w2;
+  if constexpr (SCHEME == kWenoZ) {
+    const double tau = fabs(bm - bp);
+    auto weight = [tau](double linear, double beta) {
+      const double ib = IntDivisor(beta + 1.0e-20).reciprocal();
+      const double r = int_mul_ftz(int_mul_ftz(int_mul(tau, ib), tau), ib);
+      return int_mul(linear, 1.0 + r);
+    };
+    w0 = weight(0.1, bm);
+    w1 = weight(0.6, b0);
+    w2 = weight(0.3, bp);
+  } else {
+    auto weight = [](double linear, double beta) {
+      const double x = 1.0e-6 + beta;
+      return IntDivisor(int_mul(x, x)).quotient(linear);
+    };
+    w0 = weight(0.1, bm);
+    w1 = weight(0.6, b0);
+    w2 = weight(0.3, bp);
+  }
+  const IntDivisor by_sum(w0 + w1 + w2);
+  w0 = by_sum.quotient(w0);
+  w1 = by_sum.quotient(w1);
+  w2 = by_sum.quotient(w2);
+  const double c13 = 1.0 / 3.0, c16 = 1.0 / 6.0, c56 = 5.0 / 6.0, c76 = 7.0 / 6.0, c116 = 11.0 / 6.0;
+  const double p0 = int_mul(c13, a) - int_mul(c76, b) + int_mul(c116, c);
+  const double p1 = int_mul(c56, c) - int_mul(c16, b) + int_mul(c13, d);
+  const double p2 = int_mul(c13, c) + int_mul(c56, d) - int_mul(c16, e);
+  return int_mul(w0, p0) + int_mul(w1, p1) + int_mul(w2, p2);
+}
+
+// Conserved variables whose primitives the integer forms take: density and
+// energy in [2^-60, 2^60), momenta zeros or [2^-200, 2^60).
+__device__ __forceinline__ bool state_in_range(double rho, double mu, double mv, double E) {
+  return positive_in_range<-60, 60>(rho) && in_range<-200, 60>(mu) && in_range<-200, 60>(mv) &&
+         positive_in_range<-60, 60>(E);
+}
+
+// flux_split in direction dir (0: x, 1: y).  False: a value outside the range
+// of the face fluxes' integer forms (the split fluxes are right either way).
+__device__ __forceinline__ bool flux_split_f64(int dir, double gamma, const double U[4], double fm[4], double fp[4]) {
+  const double rho = U[0], E = U[3];
+  bool ok = state_in_range(rho, U[1], U[2], E);
+  if (ok) {
+    const IntDivisor by_rho(rho);
+    const double u = by_rho.quotient(U[1]), v = by_rho.quotient(U[2]);
+    const double p = int_mul(gamma - 1.0, fma(-0.5, int_mul(rho, int_mul(u, u) + int_mul(v, v)), E));
+    ok = positive_in_range<-60, 60>(p);
+    if (ok) {
+      const double un = dir == 0 ? u : v;  // normal velocity
+      double F[4];
+      F[0] = int_mul(rho, un);
+      const double a = int_mul(F[0], un) + p;
+      // rho u v in the reference's order: (rho u) v
+      const double b = int_mul(dir == 0 ? F[0] : int_mul(rho, u), v);
+      F[1] = dir == 0 ? a : b;
+      F[2] = dir == 0 ? b : a;
+      F[3] = int_mul(E + p, un);
+      const double ws = fabs(un) + int_sqrt(by_rho.quotient(int_mul(gamma, p)));
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double P = int_mul(ws, U[r]), h = int_half(F[r]);
+        fm[r] = fma(-0.5, P, h);
+        fp[r] = fma(0.5, P, h);
+        ok = ok && in_range<-200, 70>(fm[r]) && in_range<-200, 70>(fp[r]);
+      }
+      return ok;
+    }
+  }
+  if (dir == 0) flux_split<double, 0>(gamma, U, fm, fp);
+  else flux_split<double, 1>(gamma, U, fm, fp);
+  return false;
+}
+
+// The face flux (face_flux_st) in direction dir.  fp / fm point at F+ of node
+// face-3 and F- of node face-2, component 0; stencil nodes `ss` elements apart,
+// components `cs` apart.  False: a value left the integer forms' domain and
+// `out` is not set.  One body for both directions: the normal and tangential
+// components change places, and the reference's row 1 of L and column 1 of R
+// change sign together in y, which changes no result.
+template <int SCHEME>
+__device__ __forceinline__ bool face_flux_f64(int dir, double gamma, double zp_lambda, const double um[4],
+                                              const double u0[4], const double *fp, const double *fm, int ss, int cs,
+                                              double out[4]) {
+  const double rho = int_half(um[0] + u0[0]), E = int_half(um[3] + u0[3]);
+  const double mu = int_half(um[1] + u0[1]), mv = int_half(um[2] + u0[2]);
+  if (!state_in_range(rho, mu, mv, E)) return false;
+  const IntDivisor by_rho(rho);
+  const double u = by_rho.quotient(mu), v = by_rho.quotient(mv);
+  const double K = int_mul(u, u) + int_mul(v, v);
+  const double p = int_mul(gamma - 1.0, fma(-0.5, int_mul(rho, K), E));
+  if (!positive_in_range<-60, 60>(p)) return false;
+  const double c = int_sqrt(by_rho.quotient(int_mul(gamma, p)));
+  const double H = by_rho.quotient(E + p);
+  const double un = dir == 0 ? u : v, ut = dir == 0 ? v : u;  // normal and tangential velocity
+  const IntDivisor by_c(c);
+  const double ic = by_c.reciprocal(), nc = by_c.quotient(un);
+  const double B1 = IntDivisor(int_mul(c, c)).quotient(gamma - 1.0);
+  const double B2 = int_half(int_mul(B1, K)), B1n = int_mul(B1, un), B1t = int_mul(B1, ut);
+  // column 0 and the normal momentum's of rows 0 and 3, column 0 of row 2; the
+  // tangential momentum's are -1/2 B1t in rows 0 and 3
+  const double l00 = int_half(B2 + nc), l30 = int_half(B2 - nc), l20 = 1.0 - B2;
+  const double l0n = -int_half(B1n + ic), l3n = -int_half(B1n - ic);
+  const int cn = dir == 0 ? cs : 2 * cs, ct = dir == 0 ? 2 * cs : cs;
+
+  double vh[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    // the - side is mirrored: from its last node down
+    const double *f = side == 0 ? fp : fm + 4 * ss;
+    const int step = side == 0 ? ss : -ss;
+    double x[4][5];
+#pragma unroll 1
+    for (int q = 0; q < 5; ++q, f += step) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[k][j] = x[k][j + 1];
+      const double f0 = f[0], fn = f[cn], ft = f[ct], f3 = f[3 * cs];
+      const double Pn = int_mul(B1n, fn), Pt = int_mul(B1t, ft), P3 = int_mul(B1, f3);
+      const double a0 = int_mul(l00, f0), b0 = int_mul(l0n, fn), a3 = int_mul(l30, f0), b3 = int_mul(l3n, fn);
+      const double a2 = int_mul(l20, f0);
+      // the momenta's terms in the order x, y
+      x[0][4] = fma(0.5, P3, dir == 0 ? fma(-0.5, Pt, a0 + b0) : fma(-0.5, Pt, a0) + b0);
+      x[1][4] = int_mul(ut, f0) - ft;
+      x[2][4] = (a2 + (dir == 0 ? Pn : Pt)) + (dir == 0 ? Pt : Pn) - P3;
+      x[3][4] = fma(0.5, P3, dir == 0 ? fma(-0.5, Pt, a3 + b3) : fma(-0.5, Pt, a3) + b3);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if constexpr (SCHEME == kWenoJS || SCHEME == kWenoZ)
+        vh[k] += weno_int<SCHEME>(x[k][0], x[k][1], x[k][2], x[k][3], x[k][4]);
+      else
+        vh[k] += weno_plain<SCHEME>(x[k][0], x[k][1], x[k][2], x[k][3], x[k][4], zp_lambda);
+    }
+  }
+  if (!(in_range<-400, 200>(vh[0]) && in_range<-400, 200>(vh[1]) && in_range<-400, 200>(vh[2]) &&
+        in_range<-400, 200>(vh[3])))
+    return false;
+
+  // R * vh, rows in the reference's order (utils/equations.hpp:239-299)
+  const double q2 = int_half(K), cun = int_mul(c, un);
+  out[0] = (vh[0] + vh[2]) + vh[3];
+  const double on = int_mul(un - c, vh[0]) + int_mul(un, vh[2]) + int_mul(un + c, vh[3]);
+  const double ot = int_mul(ut, vh[0]) - vh[1] + int_mul(ut, vh[2]) + int_mul(ut, vh[3]);
+  out[1] = dir == 0 ? on : ot;
+  out[2] = dir == 0 ? ot : on;
+  out[3] = int_mul(H - cun, vh[0]) - int_mul(ut, vh[1]) + int_mul(q2, vh[2]) + int_mul(H + cun, vh[3]);
+  return true;
+}
+
+// face_flux_st out of line, for faces outside the integer forms' domain.
+struct Flux4 {
+  double v[4];
+};
+template <int DIR, int SCHEME>
+__device__ __noinline__ Flux4 face_flux_plain(double gamma, double zp_lambda, double um0, double um1, double um2,
+                                              double um3, double u00, double u01, double u02, double u03,
+                                              const double *fp, const double *fm, int ss, int cs) {
+  const double um[4] = {um0, um1, um2, um3}, u0[4] = {u00, u01, u02, u03};
+  Flux4 o;
+  face_flux_st<double, DIR, SCHEME>(gamma, zp_lambda, um, u0, StridedStencil<double>{fp, ss, cs},
+                                    StridedStencil<double>{fm, ss, cs}, o.v);
+  return o;
 }
 
 }  // namespace dev

@@ -127,93 +127,96 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
   }
   __syncthreads();
 
-  // --- x sweep: split fluxes of halo rows 0..HI-1, columns 3..3+TJ
-  for (int t = threadIdx.x; t < HI * TJ; t += NT) {
-    const int hi = t / TJ, j = t - hi * TJ;
-    T q[4], fm[4], fp[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) q[r] = Us[WENOFD_IX(g.guard, S::u(r, hi, j + 3), S::kU)];
-    flux_split<T, 0>(gamma, q, fm, fp);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      Fp[WENOFD_IX(g.guard, (r * HI + hi) * TJ + j, S::kSplit)] = fp[r];
-      Fm[WENOFD_IX(g.guard, (r * HI + hi) * TJ + j, S::kSplit)] = fm[r];
-    }
-  }
-  __syncthreads();
-  // x faces f = 0..TI: face between tile nodes f-1 and f (halo rows f+2, f+3)
-  for (int t = threadIdx.x; t < (TI + 1) * TJ; t += NT) {
-    const int f = t / TJ, j = t - f * TJ;
-    if (i0 + f > g.nx || j0 + j >= g.ny) continue;
-    T um[4], u0[4], out[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      um[r] = Us[WENOFD_IX(g.guard, S::u(r, f + 2, j + 3), S::kU)];
-      u0[r] = Us[WENOFD_IX(g.guard, S::u(r, f + 3, j + 3), S::kU)];
-    }
-    // stencils: nodes 0..4 TJ apart, components HI TJ apart
-    face_flux<T, 0, SCHEME>(gamma, zpl, um, u0,
-                            Fp + WENOFD_SPAN(g.guard, f * TJ + j, f * TJ + j + 4 * TJ + 3 * HI * TJ, S::kSplit),
-                            Fm + WENOFD_SPAN(g.guard, (f + 1) * TJ + j, (f + 5) * TJ + j + 3 * HI * TJ, S::kSplit),
-                            TJ, HI * TJ, out);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) Hf[WENOFD_IX(g.guard, (r * (TI + 1) + f) * TJ + j, S::kFace)] = out[r];
-  }
-  __syncthreads();
-
-  // rhs = 0 + x term  (rhs zeroed in assembleRHS, then += in the x sweep)
+  // --- the x sweep, then the y sweep, one body: most of it is integer
+  // instructions (int_f64.cuh), and two copies would not fit the instruction
+  // caches.
+  // Bound: the FP64 pipe, with the integer pipes close behind.  At 1024^2
+  // (WENO-Z, one stage): all arithmetic on the FP64 pipe 98.7 M warp
+  // instructions on it and 6.11 ms; with fewer operations, still all there, 79.9
+  // M and 4.95 ms; with products, quotients and roots on the integer pipes 33.0
+  // M and 2.47 ms (FP64 pipe at 82 % of the rate it reaches, ALU pipe 56 %).
+  // 4096^2 SSP-RK3 step: 285 -> 115 ms.
   constexpr int PPT = (TI * TJ + NT - 1) / NT;
   T rhs[PPT][4];
-  const T dx = g.dx, dy = g.dy;
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int t = threadIdx.x + k * NT;
-    const int i = t / TJ, j = t - (t / TJ) * TJ;
+  for (int k = 0; k < PPT; ++k)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (t < TI * TJ) {
-        const T hr = Hf[WENOFD_IX(g.guard, (r * (TI + 1) + i + 1) * TJ + j, S::kFace)],
-                hl = Hf[WENOFD_IX(g.guard, (r * (TI + 1) + i) * TJ + j, S::kFace)];
-        rhs[k][r] = T(0.0) + tdiv(-(hr - hl), dx);
+    for (int r = 0; r < 4; ++r) rhs[k][r] = T(0.0);
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    const bool xdir = dir == 0;
+    // split fluxes: x, halo rows 0..HI-1 of the tile's columns; y, halo
+    // columns 0..HJ-1 of the tile's rows
+    const int sw = xdir ? TJ : HJ, scount = xdir ? HI * TJ : TI * HJ;
+    bool outside = false;  // a split flux outside the integer forms' range
+    for (int t = threadIdx.x; t < scount; t += NT) {
+      const int row = t / sw, col = t - row * sw;
+      const int hi = xdir ? row : row + 3, hj = xdir ? col + 3 : col;
+      T q[4], fm[4] = {0, 0, 0, 0}, fp[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) q[r] = Us[WENOFD_IX(g.guard, S::u(r, hi, hj), S::kU)];
+      // (nodes past the array, which no face of the grid needs, stay zero)
+      if (1 + i0 + hi < g.nxt && 1 + j0 + hj < g.nyt) outside = !flux_split_f64(dir, gamma, q, fm, fp) || outside;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        Fp[WENOFD_IX(g.guard, r * scount + t, S::kSplit)] = fp[r];
+        Fm[WENOFD_IX(g.guard, r * scount + t, S::kSplit)] = fm[r];
       }
     }
-  }
-  __syncthreads();
-
-  // --- y sweep: split fluxes of tile rows, halo columns 0..HJ-1
-  for (int t = threadIdx.x; t < TI * HJ; t += NT) {
-    const int i = t / HJ, hj = t - i * HJ;
-    T q[4], fm[4], fp[4];
+    const bool plain = __syncthreads_or(outside);
+    // faces: x, f = 0..TI between tile nodes f-1 and f (halo rows f+2, f+3);
+    // y, f = 0..TJ of row i
+    const int fw = xdir ? TJ : TJ + 1, fcount = xdir ? (TI + 1) * TJ : TI * (TJ + 1);
+    const int ss = xdir ? TJ : 1;  // stencil nodes apart; components scount apart
+    for (int t = threadIdx.x; t < fcount; t += NT) {
+      const int row = t / fw, col = t - row * fw;
+      // x: i0 + row is the face, j0 + col the node; y: the other way round
+      if (i0 + row >= g.nx + (xdir ? 1 : 0) || j0 + col >= g.ny + (xdir ? 0 : 1)) continue;
+      const int hi = xdir ? row + 2 : row + 3, hj = xdir ? col + 3 : col + 2;
+      T um[4], u0[4], out[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) q[r] = Us[WENOFD_IX(g.guard, S::u(r, i + 3, hj), S::kU)];
-    flux_split<T, 1>(gamma, q, fm, fp);
+      for (int r = 0; r < 4; ++r) {
+        um[r] = Us[WENOFD_IX(g.guard, S::u(r, hi, hj), S::kU)];
+        u0[r] = Us[WENOFD_IX(g.guard, S::u(r, xdir ? hi + 1 : hi, xdir ? hj : hj + 1), S::kU)];
+      }
+      const int s0 = row * sw + col;
+      const T *fp = Fp + WENOFD_SPAN(g.guard, s0, s0 + 4 * ss + 3 * scount, S::kSplit);
+      const T *fm = Fm + WENOFD_SPAN(g.guard, s0 + ss, s0 + 5 * ss + 3 * scount, S::kSplit);
+      if (plain || !face_flux_f64<SCHEME>(dir, gamma, zpl, um, u0, fp, fm, ss, scount, out)) {
+        const Flux4 o = xdir ? face_flux_plain<0, SCHEME>(gamma, zpl, um[0], um[1], um[2], um[3], u0[0], u0[1], u0[2],
+                                                          u0[3], fp, fm, ss, scount)
+                             : face_flux_plain<1, SCHEME>(gamma, zpl, um[0], um[1], um[2], um[3], u0[0], u0[1], u0[2],
+                                                          u0[3], fp, fm, ss, scount);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      Fp[WENOFD_IX(g.guard, (r * TI + i) * HJ + hj, S::kSplit)] = fp[r];
-      Fm[WENOFD_IX(g.guard, (r * TI + i) * HJ + hj, S::kSplit)] = fm[r];
+        for (int r = 0; r < 4; ++r) out[r] = o.v[r];
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) Hf[WENOFD_IX(g.guard, r * fcount + t, S::kFace)] = out[r];
     }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < TI * (TJ + 1); t += NT) {
-    const int i = t / (TJ + 1), f = t - i * (TJ + 1);
-    if (i0 + i >= g.nx || j0 + f > g.ny) continue;
-    T um[4], u0[4], out[4];
+    __syncthreads();
+    // rhs = 0 + x term, then + y term (rhs zeroed in assembleRHS, += in the sweeps)
+    const T h = xdir ? g.dx : g.dy;
+    const IntDivisor by_h(h);
+    const bool h_ok = in_range<-200, 200>(h);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      um[r] = Us[WENOFD_IX(g.guard, S::u(r, i + 3, f + 2), S::kU)];
-      u0[r] = Us[WENOFD_IX(g.guard, S::u(r, i + 3, f + 3), S::kU)];
+    for (int k = 0; k < PPT; ++k) {
+      const int t = threadIdx.x + k * NT;
+      const int i = t / TJ, j = t - (t / TJ) * TJ;
+      if (t < TI * TJ) {
+        const int left = i * fw + j, right = xdir ? left + TJ : left + 1;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const T hr = Hf[WENOFD_IX(g.guard, r * fcount + right, S::kFace)],
+                  hl = Hf[WENOFD_IX(g.guard, r * fcount + left, S::kFace)];
+          const T d = -(hr - hl);
+          rhs[k][r] = rhs[k][r] + (h_ok && in_range<-700, 300>(d) ? by_h.quotient(d) : tdiv(d, h));
+        }
+      }
     }
-    // stencils: nodes 0..4 adjacent, components TI HJ apart
-    face_flux<T, 1, SCHEME>(gamma, zpl, um, u0,
-                            Fp + WENOFD_SPAN(g.guard, i * HJ + f, i * HJ + f + 4 + 3 * TI * HJ, S::kSplit),
-                            Fm + WENOFD_SPAN(g.guard, i * HJ + f + 1, i * HJ + f + 5 + 3 * TI * HJ, S::kSplit), 1,
-                            TI * HJ, out);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) Hf[WENOFD_IX(g.guard, (r * TI + i) * (TJ + 1) + f, S::kFace)] = out[r];
+    __syncthreads();
   }
-  __syncthreads();
 
-  // --- y term, source, RK combination, store
+  // --- source, RK combination, store
   const double dt = COH ? __ldcg(a.dt) : *a.dt;
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
@@ -223,11 +226,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
     if (i0 + i >= g.nx || j0 + j >= g.ny) continue;
     T rr[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const T hr = Hf[WENOFD_IX(g.guard, (r * TI + i) * (TJ + 1) + j + 1, S::kFace)],
-              hl = Hf[WENOFD_IX(g.guard, (r * TI + i) * (TJ + 1) + j, S::kFace)];
-      rr[r] = rhs[k][r] + tdiv(-(hr - hl), dy);
-    }
+    for (int r = 0; r < 4; ++r) rr[r] = rhs[k][r];
     const long long gidx = WENOFD_NODE(g, i0 + i, j0 + j);
     if (g.gravity) {  // RTI, g = 1 (src/WENOFD.cpp:807-813)
       const T g_g0 = T(1.0);
@@ -250,11 +249,12 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
 // Residency: the FP32 tiles read their FP64 inputs back in the epilogue
 // instead of staging them, and ask for four (routed) or three resident
 // 256-thread blocks per SM: the stage is issue-bound and latency-bound, and
-// trading registers for resident warps pays.  The FP64 tile is bound by the
-// FP64 pipe and keeps the registers.
+// trading registers for resident warps pays.  The FP64 tile runs two blocks
+// (shared memory's limit), so that one block's sums on the FP64 pipe overlap
+// another's products on the integer pipes.
 template <typename T, bool ROUTE, int NT>
 __host__ __device__ constexpr int stage_blocks_per_sm() {
-  if constexpr (sizeof(T) == 8) return 1;
+  if constexpr (sizeof(T) == 8) return 2;
   else return NT <= 256 ? (ROUTE ? 4 : 3) : (ROUTE ? 2 : 1);
 }
 // FP32 tiles stage their FP64 inputs in shared memory only at one block per SM.

@@ -1,0 +1,75 @@
+"""The FP64 parity tile forms products, quotients and roots on the integer
+pipes where its operands lie in a wide range of exponents and leaves the rest to
+the FP64 instructions.  Both, and tiles that mix them, are the oracle's bits:
+states scaled to the ranges' edges and past them, zeros, roundoff-sized momenta,
+exact powers of two, on tiles of one node, full tiles and remainders."""
+import numpy as np
+import pytest
+
+import oracle as orc
+import wenofd
+from conftest import assert_same
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(p, kind):
+    U = p.interior()
+    rng = np.random.default_rng(3)
+    if kind == "zeros":
+        U[1:3] = 0.0
+    elif kind == "roundoff":
+        U[2] = 1e-17 * rng.standard_normal(U[2].shape)
+    elif kind == "tiny":  # momenta below 2^-200 in part of the grid
+        U[1][::3] = 1e-70
+        U[2][:, ::5] = -1e-90
+    elif kind == "dense":  # above the range: every value times 2^70
+        U *= 2.0 ** 70
+    elif kind == "thin":  # below it: every value times 2^-80
+        U *= 2.0 ** -80
+    elif kind == "edge":  # pressure jumps across the upper bound
+        U[3][U.shape[1] // 2:] *= 2.0 ** 59
+    elif kind == "binary":  # exact powers of two: quotients and roots are exact
+        U[0], U[1], U[2], U[3] = 2.0, 0.5, -0.25, 4.0
+        U[0][::2], U[3][:, ::4] = 8.0, 16.0
+    return U
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 7), (15, 32), (16, 33), (31, 65), (47, 70)])
+@pytest.mark.parametrize("kind", ["zeros", "roundoff", "tiny", "dense", "thin", "edge", "binary"])
+def test_rhs_and_steps_equal_the_oracle_at_every_range(nx, ny, kind):
+    for tc in (orc.RIEMANN_SEEDED, orc.SMOOTH):
+        for scheme in (orc.WENOJS, orc.WENOZ, orc.WENOZP):
+            p = orc.Problem(tc, nx, ny, scheme, 2, 0.3, seed=2)
+            U = _state(p, kind)
+            p.set_interior(U)
+            with wenofd.Solver({"TESTCASE": tc, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.3,
+                                "SCHEME": scheme, "SEED": 2}) as s:
+                s.set_state(U)
+                rhs = s.get_flux()
+                s.set_state(U)
+                dt = s.calc_dt()
+                s.rk_step(dt)
+                got = s.get_state()
+            want = p.assemble_rhs()
+            p.set_interior(U)
+            assert dt == p.calc_dt()
+            p.rk_step(dt)
+            if scheme == orc.WENOZP:  # pow(x, 2) of the C library: to rounding
+                assert np.max(np.abs(rhs - want)) <= 1e-12 * np.max(np.abs(want))
+                continue
+            assert_same(rhs, want, f"rhs {kind} tc {tc} scheme {scheme}")
+            assert_same(got, p.interior(), f"state {kind} tc {tc} scheme {scheme}")
+
+
+def test_nan_and_infinity_spread_as_in_the_oracle():
+    nx, ny = 40, 45
+    for bad in (np.nan, np.inf):
+        p = orc.Problem(orc.SMOOTH, nx, ny, orc.WENOZ, 2, 0.3, seed=2)
+        U = p.interior()
+        U[3, 20, 21] = bad
+        p.set_interior(U)
+        with wenofd.Solver({"TESTCASE": orc.SMOOTH, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.3,
+                            "SCHEME": orc.WENOZ}) as s:
+            s.set_state(U)
+            assert_same(s.get_flux(), p.assemble_rhs(), f"rhs with {bad}")
