@@ -53,6 +53,7 @@ struct wenofd_batch {
   int *h_flags = nullptr;
   BatchMemberStatus *h_gather = nullptr;
   // configuration
+  wenofd::Fp64Split split{15, 0};  // rows of the stage tiles (FP64 default configuration: fp64_split; else tile_i)
   int tile_i = 15, blocks_per_sm = 0, steps_setting = 0, steps_per_launch = 1, grid = 0;
   // learned form: (indicator, interval steps) pairs per graph replay, and the
   // members' indicator settings the work plan was made with
@@ -97,6 +98,8 @@ BatchArgs make_args(const wenofd_batch *b, int nsteps) {
   a.work.ind_prefix = b->d_prefix + 3 * (b->n + 1);
   a.n = b->n;
   a.nsteps = nsteps;
+  a.rows = b->split.rows;
+  a.pair = b->split.pair;
   a.rk = b->rk;
   a.counters = b->d_counters;
   a.barrier = b->d_barrier;
@@ -183,10 +186,10 @@ void drop_graph(wenofd_batch *b) {
   b->graph_tried = false;
 }
 
-// Work plan for a tile height: per-member tile counts and the three prefix
-// sums, uploaded with the member table.
-int plan(wenofd_batch *b, int tile_i) {
-  const int TI = tile_i == 0 ? 15 : tile_i;
+// Work plan for the configured tile rows: per-member tile counts and the three
+// prefix sums, uploaded with the member table.
+int plan(wenofd_batch *b) {
+  const int TI = b->split.rows;
   std::vector<BatchMember> host(b->n);
   std::vector<int> prefix(4 * size_t(b->n + 1), 0);
   int *tp = prefix.data(), *bp = tp + (b->n + 1), *pp = bp + (b->n + 1), *ip = pp + (b->n + 1);
@@ -240,6 +243,17 @@ int configure(wenofd_batch *b, int tile_i, int blocks_per_sm, int steps_per_laun
     return fail(WENOFD_BAD_ARG, "blocks_per_sm must be >= 0 and steps_per_launch in [0, 4096]");
   drop_graph(b);
   b->tile_i = tile_i == 0 ? 15 : tile_i;
+  b->split = wenofd::Fp64Split{b->tile_i, 0};
+  if (b->precision == WENOFD_FP64 && tile_i == 0) {
+    std::vector<int> nx, ny;
+    for (const wenofd_solver *s : b->members) {
+      nx.push_back(s->nx);
+      ny.push_back(s->ny);
+    }
+    int sms = 0;
+    BATCH_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+    b->split = wenofd::fp64_split(nx.data(), ny.data(), b->n, sms, b->tile_i);
+  }
   b->blocks_per_sm = blocks_per_sm;
   b->steps_setting = steps_per_launch;
   // Steps per launch: enough that launch and host-check latency are
@@ -250,7 +264,7 @@ int configure(wenofd_batch *b, int tile_i, int blocks_per_sm, int steps_per_laun
   // learned form: a graph replay runs whole (indicator, interval steps) pairs
   b->chunks = b->learned ? std::max(1, (b->steps_per_launch + b->interval - 1) / b->interval) : 1;
   if (b->learned) b->steps_per_launch = b->chunks * b->interval;
-  if (int rc = plan(b, b->tile_i)) return rc;
+  if (int rc = plan(b)) return rc;
   if (int rc = ensure_counters(b, b->learned ? b->interval : b->steps_per_launch)) return rc;
   BatchArgs q{};
   b->grid = 0;
@@ -428,7 +442,7 @@ int wenofd_batch_advance(wenofd_batch *b, long long max_steps, long long *steps_
   BATCH_TRY(cudaSetDevice(b->device));
   if (int rc = sync_members(b)) return rc;
   if (indicator_plan_stale(b))
-    if (int rc = plan(b, b->tile_i)) return rc;
+    if (int rc = plan(b)) return rc;
   if (int rc = ensure_graph(b)) return rc;
   BATCH_TRY(cudaMemsetAsync(b->d_flags, 0, 4 * sizeof(int), b->stream));
   BATCH_TRY(wenofd::launch_batch_setup(b->d_members, b->n, max_steps, b->stream));
@@ -509,7 +523,7 @@ int wenofd_batch_autotune(wenofd_batch *b, int steps, double *ms_per_step) {
   BATCH_TRY(cudaSetDevice(b->device));
   if (int rc = sync_members(b)) return rc;
   if (indicator_plan_stale(b))
-    if (int rc = plan(b, b->tile_i)) return rc;
+    if (int rc = plan(b)) return rc;
   const int keep_steps = b->steps_setting;
   // snapshot of every member's U^n (with ghosts) and control block
   size_t total = 0;

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? 3 : 1) : 2) 
       });
       barrier(Nothing());
       for_member_items(b, cnt + 3 + 2 * st, b.work.tile_prefix, sM, [&](int local, const BatchMember &M) {
-        const int ti = WENOFD_IX(M.g.guard, local / M.tiles_j, (M.g.nx + TI - 1) / TI),
+        const int ti = WENOFD_IX(M.g.guard, local / M.tiles_j, F32 ? (M.g.nx + TI - 1) / TI : M.g.nx),
                   tj = local - (local / M.tiles_j) * M.tiles_j;
         StageArgs a;
         a.uin = st == 0 ? M.S : (st == 1 ? M.A : M.B);
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? 3 : 1) : 2) 
         }
         if constexpr (F32)
           stage_tile_f32<SCHEME, TI, TJ, NT, ROUTE, true, !(NT <= 256)>(M.g, a, ti * TI, tj * TJ, smem_raw, local);
-        else stage_tile_f64<SCHEME, TI, TJ, NT, true>(M.g, a, ti * TI, tj * TJ, smem_raw);
+        else stage_tile_f64<SCHEME, TI, TJ, NT, true>(M.g, a, ti * b.rows, tj * TJ, b.rows, b.pair != 0, smem_raw);
       });
       if (st < nst - 1 || b.rk == 0) barrier(Nothing());
       else barrier(step_end);

@@ -519,18 +519,20 @@ __device__ __forceinline__ bool flux_split_f64(int dir, double gamma, const doub
 // `out` is not set.  One body for both directions: the normal and tangential
 // components change places, and the reference's row 1 of L and column 1 of R
 // change sign together in y, which changes no result.
+// pair: two adjacent lanes share the face (the even lane takes the + side, the
+// odd one the - side; all 32 lanes of the warp call it); both return it whole.
 template <int SCHEME>
-__device__ __forceinline__ bool face_flux_f64(int dir, double gamma, double zp_lambda, const double um[4],
+__device__ __forceinline__ bool face_flux_f64(int dir, bool pair, double gamma, double zp_lambda, const double um[4],
                                               const double u0[4], const double *fp, const double *fm, int ss, int cs,
                                               double out[4]) {
   const double rho = int_half(um[0] + u0[0]), E = int_half(um[3] + u0[3]);
   const double mu = int_half(um[1] + u0[1]), mv = int_half(um[2] + u0[2]);
-  if (!state_in_range(rho, mu, mv, E)) return false;
+  bool ok = state_in_range(rho, mu, mv, E);
   const IntDivisor by_rho(rho);
   const double u = by_rho.quotient(mu), v = by_rho.quotient(mv);
   const double K = int_mul(u, u) + int_mul(v, v);
   const double p = int_mul(gamma - 1.0, fma(-0.5, int_mul(rho, K), E));
-  if (!positive_in_range<-60, 60>(p)) return false;
+  ok = ok && positive_in_range<-60, 60>(p);
   const double c = int_sqrt(by_rho.quotient(int_mul(gamma, p)));
   const double H = by_rho.quotient(E + p);
   const double un = dir == 0 ? u : v, ut = dir == 0 ? v : u;  // normal and tangential velocity
@@ -545,8 +547,9 @@ __device__ __forceinline__ bool face_flux_f64(int dir, double gamma, double zp_l
   const int cn = dir == 0 ? cs : 2 * cs, ct = dir == 0 ? 2 * cs : cs;
 
   double vh[4] = {0.0, 0.0, 0.0, 0.0};
+  const int lane_side = int(threadIdx.x) & 1;
 #pragma unroll 1
-  for (int side = 0; side < 2; ++side) {
+  for (int side = pair ? lane_side : 0; ok && side < (pair ? lane_side + 1 : 2); ++side) {
     // the - side is mirrored: from its last node down
     const double *f = side == 0 ? fp : fm + 4 * ss;
     const int step = side == 0 ? ss : -ss;
@@ -575,9 +578,12 @@ __device__ __forceinline__ bool face_flux_f64(int dir, double gamma, double zp_l
         vh[k] += weno_plain<SCHEME>(x[k][0], x[k][1], x[k][2], x[k][3], x[k][4], zp_lambda);
     }
   }
-  if (!(in_range<-400, 200>(vh[0]) && in_range<-400, 200>(vh[1]) && in_range<-400, 200>(vh[2]) &&
-        in_range<-400, 200>(vh[3])))
-    return false;
+  if (pair) {  // warp-uniform
+#pragma unroll
+    for (int k = 0; k < 4; ++k) vh[k] += __shfl_xor_sync(0xffffffffu, vh[k], 1);
+  }
+  ok = ok && in_range<-400, 200>(vh[0]) && in_range<-400, 200>(vh[1]) && in_range<-400, 200>(vh[2]) &&
+       in_range<-400, 200>(vh[3]);
 
   // R * vh, rows in the reference's order (utils/equations.hpp:239-299)
   const double q2 = int_half(K), cun = int_mul(c, un);
@@ -587,7 +593,7 @@ __device__ __forceinline__ bool face_flux_f64(int dir, double gamma, double zp_l
   out[1] = dir == 0 ? on : ot;
   out[2] = dir == 0 ? ot : on;
   out[3] = int_mul(H - cun, vh[0]) - int_mul(ut, vh[1]) + int_mul(q2, vh[2]) + int_mul(H + cun, vh[3]);
-  return true;
+  return ok;
 }
 
 // face_flux_st out of line, for faces outside the integer forms' domain.

@@ -59,10 +59,12 @@ struct StageSmem {
 // non-coherent read-only path.  TMA (the per-solve kernel): the halo box
 // arrives by TMA through the map in `tma` (one thread issues it; a bounded
 // wait, on give-up the block records the error in a.wait_error and leaves
-// the tile); otherwise every thread loads nodes.
+// the tile); otherwise every thread loads nodes.  rows: nodes of the tile in
+// x, at most TI; pair: two lanes per face (Fp64Split).
 template <int SCHEME, int TI, int TJ, int NT, bool COH = false, bool TMA = false>
 __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a, const int i0, const int j0,
-                                               unsigned char *smem_raw, const StageTma *tma = nullptr) {
+                                               const int rows, const bool pair, unsigned char *smem_raw,
+                                               const StageTma *tma = nullptr) {
   using T = double;
   using S = StageSmem<TI, TJ>;
   constexpr int HI = S::HI, HJ = S::HJ;
@@ -110,7 +112,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
       const int rem = t - r * (HI * HJ);
       const int hi = rem / HJ, hj = rem - hi * HJ;
       const int ei = 1 + i0 + hi, ej = 1 + j0 + hj;
-      const bool ok = t < 4 * HI * HJ && ei < g.nxt && ej < g.nyt;
+      const bool ok = t < 4 * HI * HJ && hi < rows + 6 && ei < g.nxt && ej < g.nyt;
       if constexpr (COH) v[k] = ok ? __ldcg(&a.uin[WENOFD_STATE(g, r * g.plane + WENOFD_GNODE(g, ei, ej))]) : 0.0;
       else v[k] = ok ? __ldg(&a.uin[WENOFD_STATE(g, r * g.plane + WENOFD_GNODE(g, ei, ej))]) : 0.0;
     }
@@ -145,9 +147,9 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
 #pragma unroll 1
   for (int dir = 0; dir < 2; ++dir) {
     const bool xdir = dir == 0;
-    // split fluxes: x, halo rows 0..HI-1 of the tile's columns; y, halo
+    // split fluxes: x, halo rows 0..rows+5 of the tile's columns; y, halo
     // columns 0..HJ-1 of the tile's rows
-    const int sw = xdir ? TJ : HJ, scount = xdir ? HI * TJ : TI * HJ;
+    const int sw = xdir ? TJ : HJ, scount = xdir ? (rows + 6) * TJ : rows * HJ;
     bool outside = false;  // a split flux outside the integer forms' range
     for (int t = threadIdx.x; t < scount; t += NT) {
       const int row = t / sw, col = t - row * sw;
@@ -164,14 +166,22 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
       }
     }
     const bool plain = __syncthreads_or(outside);
-    // faces: x, f = 0..TI between tile nodes f-1 and f (halo rows f+2, f+3);
+    // faces: x, f = 0..rows between tile nodes f-1 and f (halo rows f+2, f+3);
     // y, f = 0..TJ of row i
-    const int fw = xdir ? TJ : TJ + 1, fcount = xdir ? (TI + 1) * TJ : TI * (TJ + 1);
+    const int fw = xdir ? TJ : TJ + 1, fcount = xdir ? (rows + 1) * TJ : rows * (TJ + 1);
     const int ss = xdir ? TJ : 1;  // stencil nodes apart; components scount apart
-    for (int t = threadIdx.x; t < fcount; t += NT) {
-      const int row = t / fw, col = t - row * fw;
+    // pair: two lanes a face, whole warps (a lane without a face repeats the
+    // tile's first and stores nothing)
+    const int lanes = pair ? 2 : 1, work = pair ? (2 * fcount + 31) & ~31 : fcount;
+    for (int w = threadIdx.x; w < work; w += NT) {
+      int t = w / lanes;
+      int row = t / fw, col = t - row * fw;
       // x: i0 + row is the face, j0 + col the node; y: the other way round
-      if (i0 + row >= g.nx + (xdir ? 1 : 0) || j0 + col >= g.ny + (xdir ? 0 : 1)) continue;
+      const bool inside = t < fcount && i0 + row < g.nx + (xdir ? 1 : 0) && j0 + col < g.ny + (xdir ? 0 : 1);
+      if (!inside) {
+        if (!pair) continue;
+        t = row = col = 0;
+      }
       const int hi = xdir ? row + 2 : row + 3, hj = xdir ? col + 3 : col + 2;
       T um[4], u0[4], out[4];
 #pragma unroll
@@ -182,7 +192,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
       const int s0 = row * sw + col;
       const T *fp = Fp + WENOFD_SPAN(g.guard, s0, s0 + 4 * ss + 3 * scount, S::kSplit);
       const T *fm = Fm + WENOFD_SPAN(g.guard, s0 + ss, s0 + 5 * ss + 3 * scount, S::kSplit);
-      if (plain || !face_flux_f64<SCHEME>(dir, gamma, zpl, um, u0, fp, fm, ss, scount, out)) {
+      if (plain || !face_flux_f64<SCHEME>(dir, pair, gamma, zpl, um, u0, fp, fm, ss, scount, out)) {
         const Flux4 o = xdir ? face_flux_plain<0, SCHEME>(gamma, zpl, um[0], um[1], um[2], um[3], u0[0], u0[1], u0[2],
                                                           u0[3], fp, fm, ss, scount)
                              : face_flux_plain<1, SCHEME>(gamma, zpl, um[0], um[1], um[2], um[3], u0[0], u0[1], u0[2],
@@ -190,8 +200,10 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
 #pragma unroll
         for (int r = 0; r < 4; ++r) out[r] = o.v[r];
       }
+      if (inside && w % lanes == 0) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) Hf[WENOFD_IX(g.guard, r * fcount + t, S::kFace)] = out[r];
+        for (int r = 0; r < 4; ++r) Hf[WENOFD_IX(g.guard, r * fcount + t, S::kFace)] = out[r];
+      }
     }
     __syncthreads();
     // rhs = 0 + x term, then + y term (rhs zeroed in assembleRHS, += in the sweeps)
@@ -202,7 +214,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
     for (int k = 0; k < PPT; ++k) {
       const int t = threadIdx.x + k * NT;
       const int i = t / TJ, j = t - (t / TJ) * TJ;
-      if (t < TI * TJ) {
+      if (t < rows * TJ) {
         const int left = i * fw + j, right = xdir ? left + TJ : left + 1;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -221,7 +233,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
     const int t = threadIdx.x + k * NT;
-    if (t >= TI * TJ) continue;
+    if (t >= rows * TJ) continue;
     const int i = t / TJ, j = t - i * TJ;
     if (i0 + i >= g.nx || j0 + j >= g.ny) continue;
     T rr[4];
@@ -276,8 +288,8 @@ __global__ void __launch_bounds__(NT, stage_blocks_per_sm<T, ROUTE, NT>())
         g, a, int(blockIdx.y) * TI, int(blockIdx.x) * TJ, smem_raw, int(blockIdx.y * gridDim.x + blockIdx.x),
         &tma);
   else
-    stage_tile_f64<SCHEME, TI, TJ, NT, false, true>(g, a, int(blockIdx.y) * TI, int(blockIdx.x) * TJ, smem_raw,
-                                                    &tma);
+    stage_tile_f64<SCHEME, TI, TJ, NT, false, true>(g, a, int(blockIdx.y) * a.rows, int(blockIdx.x) * TJ, a.rows,
+                                                    a.pair != 0, smem_raw, &tma);
 }
 
 // Dynamic shared memory of one stage tile.
@@ -290,10 +302,14 @@ constexpr size_t stage_smem_bytes() {
 // Host-side launcher for one precision: picks the kernel instance for the
 // scheme and tile height, sets its shared-memory size, launches it.
 template <typename T, int TI, int NT, bool ROUTE = false>
-cudaError_t launch_stage_tile(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, cudaStream_t s) {
+cudaError_t launch_stage_tile(const Geom &g, const StageArgs &args, const StageTma &tma, int scheme, cudaStream_t s,
+                              int rows = TI, int pair = 0) {
   constexpr int TJ = 32;
   constexpr size_t smem = stage_smem_bytes<T, TI, TJ, ROUTE, NT>();
-  const dim3 grid((g.ny + TJ - 1) / TJ, (g.nx + TI - 1) / TI);
+  StageArgs a = args;
+  a.rows = rows;
+  a.pair = pair;
+  const dim3 grid((g.ny + TJ - 1) / TJ, (g.nx + rows - 1) / rows);
   void (*fn)(Geom, StageArgs, StageTma) = nullptr;
   switch (scheme) {
     case kWenoJS: fn = k_stage<T, kWenoJS, TI, TJ, NT, ROUTE>; break;

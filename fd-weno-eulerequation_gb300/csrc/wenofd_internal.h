@@ -81,6 +81,8 @@ struct StageArgs {
   // on this integer instead of comparing the FP64 coefficients on the
   // device, where every FP64 compare issues on the 1/64-rate FP64 pipe.
   int form = 0;
+  // FP64 per-solve kernel: how its tiles are split (Fp64Split, set by the launcher)
+  int rows = 0, pair = 0;
   // FP32 per-solve tiles: set to 1 if a tile's TMA load wait gave up
   // (the host reports WENOFD_TIMEOUT).
   int *wait_error = nullptr;
@@ -126,6 +128,14 @@ cudaError_t launch_guard_selftest(unsigned long long *rec, int *buf, unsigned lo
 // maps in `tma` (make_stage_tma for the same tile height)
 cudaError_t launch_stage_fp64(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i,
                               cudaStream_t s);
+// How the FP64 stage tiles are split: their rows, and whether two lanes share
+// a face.
+struct Fp64Split {
+  int rows, pair;
+};
+// The split (tiles of 1 to `most` rows) that should finish a stage over the
+// given grids soonest on `sms` SMs.
+Fp64Split fp64_split(const int *nx, const int *ny, int n, int sms, int most);
 // The FP32 tiles load their halo by TMA: `tma` holds the maps of a.uin (and
 // of a.flags) for tiles of tile_i rows.
 cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i,
@@ -187,6 +197,7 @@ struct BatchArgs {
   // its ghosts, as the single solve's indicator does.  Uses the counters of
   // step nsteps (the counter array then holds nsteps + 1 steps).
   int fill_end = 0;
+  int rows = 0, pair = 0;  // FP64 members: Fp64Split (rows: the kernel's tile height or fewer)
   // FP32 forms: set by the block that releases a barrier when every member
   // that can step holds valid tile bounds of its U^n (Ctrl::bounds_valid):
   // the next time-step reduction then skips its screen and node passes and

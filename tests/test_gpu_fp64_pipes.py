@@ -73,3 +73,23 @@ def test_nan_and_infinity_spread_as_in_the_oracle():
                             "SCHEME": orc.WENOZ}) as s:
             s.set_state(U)
             assert_same(s.get_flux(), p.assemble_rhs(), f"rhs with {bad}")
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 6), (17, 40), (100, 100), (121, 481), (300, 33), (40, 900)])
+@pytest.mark.parametrize("batched", [False, True])
+def test_split_of_small_grids_changes_no_bit(nx, ny, batched):
+    """TILE_I = 0 picks the FP64 tiles' rows, and whether two lanes share a
+    face, from the grid and the number of SMs; 15 and 7 are fixed."""
+    got = []
+    for tile in (15, 7, 0):
+        cfg = {"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.5, "SCHEME": 1, "SEED": 4}
+        with wenofd.Solver(cfg if batched else dict(cfg, TILE_I=tile)) as s:
+            s.initialize()
+            if batched:
+                with wenofd.Batch([s]) as b:
+                    b.configure(tile_i=tile)
+                    assert b.advance(3) == 3
+            else:
+                assert s.advance(max_steps=3) == 3
+            got.append(s.get_state())
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
