@@ -224,60 +224,71 @@ __device__ __forceinline__ T weno(T a, T b, T c, T d, T e, T zp_lambda) {
   return weno_zpi(a, b, c, d, e);
 }
 
-// WENO-JS / WENO-Z on two stencils at once (betas, wenoz_weights or the
-// WENO-JS weights, and combine of physics.cuh, in the same order), used for
-// the + and - sides of one characteristic field: the arithmetic runs on packed
-// pairs, the reciprocals and the caps per element.
-__device__ __forceinline__ void betas2(float2 a, float2 b, float2 c, float2 d, float2 e, float2 &bm, float2 &b0,
-                                       float2 &bp) {
-  const float2 c1312 = splat2(float(13.0 / 12.0)), c14 = splat2(0.25f), m2 = splat2(-2.0f), m4 = splat2(-4.0f),
-               p3 = splat2(3.0f);
-  float2 t1 = __fadd2_rn(__ffma2_rn(m2, b, a), c);
-  float2 t2 = __ffma2_rn(p3, c, __ffma2_rn(m4, b, a));
-  bm = __ffma2_rn(__fmul2_rn(c1312, t1), t1, __fmul2_rn(__fmul2_rn(c14, t2), t2));
-  t1 = __fadd2_rn(__ffma2_rn(m2, c, b), d);
-  t2 = sub2(b, d);
-  b0 = __ffma2_rn(__fmul2_rn(c1312, t1), t1, __fmul2_rn(__fmul2_rn(c14, t2), t2));
-  t1 = __fadd2_rn(__ffma2_rn(m2, d, c), e);
-  t2 = __fadd2_rn(__ffma2_rn(m4, d, __fmul2_rn(p3, c)), e);
-  bp = __ffma2_rn(__fmul2_rn(c1312, t1), t1, __fmul2_rn(__fmul2_rn(c14, t2), t2));
+// FP32 WENO-JS / WENO-Z on two stencils at once, used for the + and - sides of
+// one characteristic field: the arithmetic runs on packed pairs (38 of them),
+// the reciprocals and the caps per element.  Written for the FMA pipe, which
+// bounds the FP32 form, on the stencil's differences d1..d4:
+//   4 beta_k + 4 eps = B_k = 13/3 s_k^2 + (t_k^2 + 4 eps), s the second
+//   differences and t = (d1 - 3 d2, d2 + d3, d4 - 3 d3);
+//   ratios tau/beta from tau = B_0 - B_2 (squared, so unsigned), capped at 1e15
+//   before squaring (a larger weight already makes its stencil's normalised
+//   weight 1 to FP32 precision, and products with it stay finite);
+//   the result c + sum alpha_k P_k / (6 sum alpha_k) with the candidates' 6 (p_k
+//   - c) = (5 d2 - 2 d1, d2 + 2 d3, 4 d3 - d4), which also cancels less than the
+//   candidates themselves.
+// Explicitly rounded operations: every unit computes the same bits.
+// The reciprocals, and the roots of the face's eigenvectors, are the bare
+// hardware approximations (about 1 ulp; a zero divisor is out of reach of B_k,
+// and subnormal ones count as zero): with the division intrinsic's handling of
+// subnormals one reconstruction takes 104 instructions instead of 65.
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
-
-__device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(__fdividef(1.0f, x.x), __fdividef(1.0f, x.y)); }
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_ftz(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_ftz(x.x), rcp_ftz(x.y)); }
 
 template <int SCHEME>
 __device__ __forceinline__ float2 weno2(float2 a, float2 b, float2 c, float2 d, float2 e) {
   static_assert(SCHEME == kWenoJS || SCHEME == kWenoZ, "packed WENO-JS and WENO-Z only");
-  float2 bm, b0, bp, w0, w1, w2;
-  betas2(a, b, c, d, e, bm, b0, bp);
+  const float2 d1 = sub2(b, a), d2 = sub2(c, b), d3 = sub2(d, c), d4 = sub2(e, d);
+  const float2 s0 = sub2(d2, d1), s1 = sub2(d3, d2), s2 = sub2(d4, d3);
+  const float2 m3 = splat2(-3.0f);
+  const float2 t0 = __ffma2_rn(m3, d2, d1), t1 = __fadd2_rn(d2, d3), t2 = __ffma2_rn(m3, d3, d4);
+  const float2 eps = splat2(SCHEME == kWenoZ ? 4.0e-20f : 4.0e-6f), c133 = splat2(float(13.0 / 3.0));
+  const float2 B0 = __ffma2_rn(c133, __fmul2_rn(s0, s0), __ffma2_rn(t0, t0, eps));
+  const float2 B1 = __ffma2_rn(c133, __fmul2_rn(s1, s1), __ffma2_rn(t1, t1, eps));
+  const float2 B2 = __ffma2_rn(c133, __fmul2_rn(s2, s2), __ffma2_rn(t2, t2, eps));
+  float2 r0 = rcp2(B0), r1 = rcp2(B1), r2 = rcp2(B2);
+  float2 w0, w1, w2;  // alpha_0, -alpha_1, alpha_2, times 10
   if constexpr (SCHEME == kWenoZ) {
-    const float2 eps = splat2(1.0e-20f), one = splat2(1.0f);
-    const float2 ibm = rcp2(__fadd2_rn(bm, eps)), ib0 = rcp2(__fadd2_rn(b0, eps)), ibp = rcp2(__fadd2_rn(bp, eps));
-    const float2 tau = make_float2(fabsf(bm.x - bp.x), fabsf(bm.y - bp.y));
-    float2 rm = __fmul2_rn(tau, ibm), r0 = __fmul2_rn(tau, ib0), rp = __fmul2_rn(tau, ibp);
-    rm = make_float2(fminf(rm.x, 1.0e18f), fminf(rm.y, 1.0e18f));
-    r0 = make_float2(fminf(r0.x, 1.0e18f), fminf(r0.y, 1.0e18f));
-    rp = make_float2(fminf(rp.x, 1.0e18f), fminf(rp.y, 1.0e18f));
-    w0 = __fmul2_rn(splat2(0.1f), __ffma2_rn(rm, rm, one));
-    w1 = __fmul2_rn(splat2(0.6f), __ffma2_rn(r0, r0, one));
-    w2 = __fmul2_rn(splat2(0.3f), __ffma2_rn(rp, rp, one));
+    const float2 tau = sub2(B0, B2);
+    auto cap = [](float2 x) { return make_float2(fminf(fabsf(x.x), 1.0e15f), fminf(fabsf(x.y), 1.0e15f)); };
+    r0 = cap(__fmul2_rn(tau, r0));
+    r1 = cap(__fmul2_rn(tau, r1));
+    r2 = cap(__fmul2_rn(tau, r2));
+    w0 = __ffma2_rn(r0, r0, splat2(1.0f));
+    w1 = __ffma2_rn(__fmul2_rn(splat2(-6.0f), r1), r1, splat2(-6.0f));
+    w2 = __ffma2_rn(__fmul2_rn(splat2(3.0f), r2), r2, splat2(3.0f));
   } else {
-    const float2 eps = splat2(1.0e-6f);
-    const float2 sm = __fadd2_rn(eps, bm), s0 = __fadd2_rn(eps, b0), sp = __fadd2_rn(eps, bp);
-    w0 = __fmul2_rn(splat2(0.1f), rcp2(__fmul2_rn(sm, sm)));
-    w1 = __fmul2_rn(splat2(0.6f), rcp2(__fmul2_rn(s0, s0)));
-    w2 = __fmul2_rn(splat2(0.3f), rcp2(__fmul2_rn(sp, sp)));
+    w0 = __fmul2_rn(r0, r0);
+    w1 = __fmul2_rn(__fmul2_rn(splat2(-6.0f), r1), r1);
+    w2 = __fmul2_rn(__fmul2_rn(splat2(3.0f), r2), r2);
   }
-  const float2 iws = rcp2(__fadd2_rn(__fadd2_rn(w0, w1), w2));
-  w0 = __fmul2_rn(w0, iws);
-  w1 = __fmul2_rn(w1, iws);
-  w2 = __fmul2_rn(w2, iws);
-  const float2 c13 = splat2(float(1.0 / 3.0)), c56 = splat2(float(5.0 / 6.0)), c116 = splat2(float(11.0 / 6.0));
-  const float2 mc76 = splat2(-float(7.0 / 6.0)), mc16 = splat2(-float(1.0 / 6.0));
-  const float2 q0 = __ffma2_rn(c116, c, __ffma2_rn(mc76, b, __fmul2_rn(c13, a)));
-  const float2 q1 = __ffma2_rn(c13, d, __ffma2_rn(c56, c, __fmul2_rn(mc16, b)));
-  const float2 q2 = __ffma2_rn(mc16, e, __ffma2_rn(c56, d, __fmul2_rn(c13, c)));
-  return __ffma2_rn(w2, q2, __ffma2_rn(w1, q1, __fmul2_rn(w0, q0)));
+  const float2 isum = rcp2(sub2(__fadd2_rn(w0, w2), w1));
+  const float2 q0 = __ffma2_rn(splat2(2.0f), t0, d2), q1 = __ffma2_rn(splat2(2.0f), d3, d2), q2 = sub2(t2, d3);
+  const float2 num = __ffma2_rn(w1, q1, __ffma2_rn(w2, q2, __fmul2_rn(w0, q0)));
+  return __ffma2_rn(__fmul2_rn(num, isum), splat2(float(-1.0 / 6.0)), c);
 }
 
 // The two sides of one characteristic field at a face: the + side on F+
@@ -315,15 +326,6 @@ struct StridedStencil {  // SoA: nodes `ss` elements apart, components `cs` apar
   int ss, cs;
   __device__ __forceinline__ T operator()(int s, int r) const { return p[s * ss + r * cs]; }
 };
-struct Float4Stencil {  // AoS: one float4 per node, nodes `ss` float4s apart
-  const float4 *p;
-  int ss;
-  __device__ __forceinline__ float operator()(int s, int r) const {
-    const float4 v = p[s * ss];
-    return r == 0 ? v.x : (r == 1 ? v.y : (r == 2 ? v.z : v.w));
-  }
-};
-
 template <typename T, int DIR, int SCHEME, typename St>
 __device__ __forceinline__ void face_flux_st(T gamma, T zp_lambda, const T um[4], const T u0[4], const St &fp,
                                              const St &fm, T out[4]) {
@@ -395,6 +397,96 @@ __device__ __forceinline__ void face_flux_st(T gamma, T zp_lambda, const T um[4]
     f += R[r][3] * vh[3];
     out[r] = f;
   }
+}
+
+// ------------------------------------------------- FP32 face and split
+//
+// The FP32 forms' face flux and split, in as few FMA-pipe operations as the
+// scheme needs (the FMA pipe and issue bound the FP32 form) and with explicitly
+// rounded operations, so that the per-solve and batched kernels agree bit for
+// bit.
+
+// Quantities of the x- (DIR 0) or y-Jacobian at a face's average state: normal
+// and tangential velocity, (u^2 + v^2)/2, sound speed and its inverse, enthalpy,
+// (gamma - 1)/(2 c^2).
+struct Eigen32 {
+  float un, ut, k2, c, ic, H, b;
+};
+template <int DIR>
+__device__ __forceinline__ Eigen32 eigen32(float gamma, const float4 um, const float4 u0) {
+  const float g1 = __fadd_rn(gamma, -1.0f);
+  const float ir = rcp_ftz(__fadd_rn(um.x, u0.x));  // halves of the sums cancel in quotients
+  const float u = __fmul_rn(__fadd_rn(um.y, u0.y), ir), v = __fmul_rn(__fadd_rn(um.z, u0.z), ir);
+  const float e = __fmul_rn(__fadd_rn(um.w, u0.w), ir);  // E / rho
+  Eigen32 q;
+  q.k2 = __fmul_rn(0.5f, __fmaf_rn(u, u, __fmul_rn(v, v)));
+  const float h = __fmul_rn(g1, __fadd_rn(e, -q.k2));  // p / rho
+  const float c2 = __fmul_rn(gamma, h);
+  // one Newton step on the hardware's 1/c: L and R are inverses to rounding
+  const float y = rsqrt_ftz(c2);
+  q.ic = __fmaf_rn(__fmul_rn(0.5f, y), __fmaf_rn(__fmul_rn(-c2, y), y, 1.0f), y);
+  q.c = __fmul_rn(c2, q.ic);
+  q.H = __fadd_rn(e, h);
+  q.b = __fmul_rn(__fmul_rn(0.5f, g1), __fmul_rn(q.ic, q.ic));
+  q.un = DIR == 0 ? u : v;
+  q.ut = DIR == 0 ? v : u;
+  return q;
+}
+
+// Characteristic flux at a face (face_flux_st) from float4 nodes P, M (F+ at
+// face-3.., F- at face-2.., `ss` apart).  Rows 0 and 3 of L are Q + D and Q - D
+// with Q = (B1/2)((u^2+v^2)/2 f0 - u f1 - v f2 + f3) and D = (un f0 - fn)/(2c),
+// row 2 is f0 - 2 Q: 10 operations a node instead of 16.  In y row 1 of L and
+// column 1 of R change sign together.
+template <int DIR, int SCHEME>
+__device__ __forceinline__ float4 face_flux_f32(float gamma, float zpl, const float4 um, const float4 u0,
+                                                const float4 *P, const float4 *M, int ss) {
+  const Eigen32 g = eigen32<DIR>(gamma, um, u0);
+  const float q0 = __fmul_rn(g.b, g.k2), qn = -__fmul_rn(g.b, g.un), qt = -__fmul_rn(g.b, g.ut);
+  const float dn = __fmul_rn(-0.5f, g.ic), d0 = -__fmul_rn(dn, g.un);
+  float vp[4][5], vm[4][5];
+  auto project = [&](const float4 f, float &x0, float &x1, float &x2, float &x3) {
+    const float fn = DIR == 0 ? f.y : f.z, ft = DIR == 0 ? f.z : f.y;
+    const float Q = __fmaf_rn(g.b, f.w, __fmaf_rn(qt, ft, __fmaf_rn(qn, fn, __fmul_rn(q0, f.x))));
+    const float D = __fmaf_rn(dn, fn, __fmul_rn(d0, f.x));
+    x0 = __fadd_rn(Q, D);
+    x1 = __fmaf_rn(g.ut, f.x, -ft);
+    x2 = __fmaf_rn(-2.0f, Q, f.x);
+    x3 = __fadd_rn(Q, -D);
+  };
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    project(P[s * ss], vp[0][s], vp[1][s], vp[2][s], vp[3][s]);
+    project(M[s * ss], vm[0][s], vm[1][s], vm[2][s], vm[3][s]);
+  }
+  float h[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) h[k] = weno_sides<float, SCHEME>(vp[k], vm[k], zpl);
+  const float S = __fadd_rn(h[0], h[3]), cD = __fmul_rn(g.c, __fadd_rn(h[3], -h[0]));
+  const float o0 = __fadd_rn(S, h[2]);
+  const float on = __fmaf_rn(g.un, o0, cD), ot = __fmaf_rn(g.ut, o0, -h[1]);
+  const float o3 =
+      __fmaf_rn(g.k2, h[2], __fmaf_rn(-g.ut, h[1], __fmaf_rn(g.un, cD, __fmul_rn(g.H, S))));
+  return DIR == 0 ? make_float4(o0, on, ot, o3) : make_float4(o0, ot, on, o3);
+}
+
+// Pointwise Lax-Friedrichs split of one node in direction DIR: halves of the
+// physical flux -+ half the wave speed times U.
+template <int DIR>
+__device__ __forceinline__ void split4(float gamma, const float4 q, float4 &fm, float4 &fp) {
+  const float ir = rcp_ftz(q.x);
+  const float u = __fmul_rn(q.y, ir), v = __fmul_rn(q.z, ir);
+  const float g1 = __fadd_rn(gamma, -1.0f);
+  const float p = __fmul_rn(g1, __fmaf_rn(-0.5f, __fmaf_rn(q.y, u, __fmul_rn(q.z, v)), q.w));
+  const float mn = DIR == 0 ? q.y : q.z, mt = DIR == 0 ? q.z : q.y, un = DIR == 0 ? u : v;
+  const float c = sqrt_ftz(__fmul_rn(__fmul_rn(gamma, p), ir));
+  const float hu = __fmul_rn(0.5f, un), hw = __fmul_rn(0.5f, __fadd_rn(fabsf(un), c));
+  const float f0 = __fmul_rn(0.5f, mn), fn = __fmaf_rn(mn, hu, __fmul_rn(0.5f, p)), ft = __fmul_rn(mt, hu);
+  const float f3 = __fmul_rn(__fadd_rn(q.w, p), hu);
+  const float2 F01 = make_float2(f0, DIR == 0 ? fn : ft), F23 = make_float2(DIR == 0 ? ft : fn, f3);
+  const float2 mws = splat2(-hw), pws = splat2(hw);
+  fm = join2(__ffma2_rn(mws, lo2(q), F01), __ffma2_rn(mws, hi2(q), F23));
+  fp = join2(__ffma2_rn(pws, lo2(q), F01), __ffma2_rn(pws, hi2(q), F23));
 }
 
 // ------------------------------------ FP64 on the FP64 and integer pipes

@@ -14,6 +14,12 @@
 //   Un64 double [4][TI][TJ] the tile's FP64 U^n (stages 2-3, cp.async)
 // The TMA form lands the tile's FP64 halo box, [4][HI][40] doubles, at the
 // base, over Fp/Fm/Hf, which the sweeps write only after it is converted.
+//
+// Bound of the FP32 form: issue and the FMA pipe.  With the reconstruction on
+// the stencil's differences, eigenvector rows sharing Q and D and bare hardware
+// reciprocals (physics.cuh) a node takes 1,364 thread instructions a stage
+// instead of 2,725; stage 1 at 2048^2 (WENO-Z) 283 -> 212 us, FMA pipe 56 %,
+// issue 69 %.
 #pragma once
 
 #include "aux_device.cuh"
@@ -46,36 +52,6 @@ struct StageSmem32 {
   static constexpr size_t bytes =
       128 + sizeof(float4) * (size_t(kU) + 2 * kSplit + kFace) + sizeof(double) * kKeep;
 };
-
-__device__ __forceinline__ float4 f4_split_store(float a, float b, float c, float d) { return make_float4(a, b, c, d); }
-
-// Pointwise Lax-Friedrichs split of one node (flux_split in physics.cuh; the
-// same operations, F -+ ws U and the halving on packed pairs).
-template <int DIR>
-__device__ __forceinline__ void split4(float gamma, const float4 q, float4 &fm, float4 &fp) {
-  const float U[4] = {q.x, q.y, q.z, q.w};
-  float u, v, p;
-  primitives(gamma, U, u, v, p);
-  const float rho = q.x, E = q.w;
-  float F[4];
-  if (DIR == 0) {
-    F[0] = rho * u;
-    F[1] = rho * u * u + p;
-    F[2] = rho * u * v;
-    F[3] = (E + p) * u;
-  } else {
-    F[0] = rho * v;
-    F[1] = rho * u * v;
-    F[2] = rho * v * v + p;
-    F[3] = (E + p) * v;
-  }
-  const float c = tsqrt(tdiv(gamma * p, rho));
-  const float ws = (DIR == 0 ? tabs(u) : tabs(v)) + c;
-  const float2 h = splat2(0.5f), mws = splat2(-ws), pws = splat2(ws);
-  const float2 F01 = make_float2(F[0], F[1]), F23 = make_float2(F[2], F[3]);
-  fm = join2(__fmul2_rn(h, __ffma2_rn(mws, lo2(q), F01)), __fmul2_rn(h, __ffma2_rn(mws, hi2(q), F23)));
-  fp = join2(__fmul2_rn(h, __ffma2_rn(pws, lo2(q), F01)), __fmul2_rn(h, __ffma2_rn(pws, hi2(q), F23)));
-}
 
 // Linear fifth-order upwind flux of one component: WENO with its weights
 // frozen at (0.1, 0.6, 0.3), on F+ at nodes face-3..face+1 (p0..p4) and on F-
@@ -115,93 +91,41 @@ __device__ __forceinline__ float4 linear_face4(const float4 *P, const float4 *M,
                lin5x2(hi2(p0), hi2(p1), hi2(p2), hi2(p3), hi2(p4), hi2(m0), hi2(m1), hi2(m2), hi2(m3), hi2(m4)));
 }
 
-// Characteristic WENO face from float4 stencils (face_flux_st).
-template <int DIR, int SCHEME>
-__device__ __forceinline__ float4 weno_face4(float gamma, float zpl, const float4 um4, const float4 u04,
-                                             const float4 *P, const float4 *M, int ss) {
-  const float um[4] = {um4.x, um4.y, um4.z, um4.w}, u0[4] = {u04.x, u04.y, u04.z, u04.w};
-  float out[4];
-  face_flux_st<float, DIR, SCHEME>(gamma, zpl, um, u0, Float4Stencil{P, ss}, Float4Stencil{M, ss}, out);
-  return make_float4(out[0], out[1], out[2], out[3]);
-}
-
 // One characteristic field of a WENO face, for the routed form where the
 // faces that need WENO are few and would otherwise keep a handful of threads
 // busy while the block waits: four consecutive lanes take one face, lane k
 // projects the ten stencil fluxes on left eigenvector k and reconstructs
-// characteristic field k (face_flux_st's per-field work, same operation
-// order), the four fields are exchanged by shuffles, and lane k returns
-// component k of R * vh.  All 32 lanes of the warp must call it.
+// characteristic field k, the four fields are exchanged by shuffles, and lane k
+// returns component k of R * vh.  All 32 lanes of the warp must call it.
 template <int DIR, int SCHEME>
 __device__ __forceinline__ float weno_face_lane(float gamma, float zpl, const float4 um4, const float4 u04,
                                                 const float4 *P, const float4 *M, int ss, int k) {
-  const float um[4] = {um4.x, um4.y, um4.z, um4.w}, u0[4] = {u04.x, u04.y, u04.z, u04.w};
-  float ave[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) ave[r] = 0.5f * (um[r] + u0[r]);
-  float u, v, p;
-  primitives(gamma, ave, u, v, p);
-  const float rho = ave[0], E = ave[3];
-  const float c = tsqrt(tdiv(gamma * p, rho));
-  const float B1 = tdiv((gamma - 1.0f), (c * c));
-  const float B2 = B1 * (u * u + v * v) * 0.5f;
-  const float H = tdiv((E + p), rho);
-  const float ic = tdiv(1.0f, c);
-  const float nc = tdiv(DIR == 0 ? u : v, c);
-  const float B1u = B1 * u, B1v = B1 * v;
-  // row k of the left eigenvector matrix (face_flux_st)
-  float l0, l1, l2, l3;
-  if (DIR == 0) {
-    l0 = k == 0 ? (B2 + nc) * 0.5f : (k == 1 ? v : (k == 2 ? (1.0f - B2) : (B2 - nc) * 0.5f));
-    l1 = k == 0 ? -(B1u + ic) * 0.5f : (k == 1 ? 0.0f : (k == 2 ? B1u : -(B1u - ic) * 0.5f));
-    l2 = k == 0 ? -(B1v) * 0.5f : (k == 1 ? -1.0f : (k == 2 ? B1v : -B1v * 0.5f));
-    l3 = k == 0 ? B1 * 0.5f : (k == 1 ? 0.0f : (k == 2 ? -B1 : B1 * 0.5f));
-  } else {
-    l0 = k == 0 ? (B2 + nc) * 0.5f : (k == 1 ? -u : (k == 2 ? 1.0f - B2 : (B2 - nc) * 0.5f));
-    l1 = k == 0 ? -(B1u) * 0.5f : (k == 1 ? 1.0f : (k == 2 ? B1u : -(B1u) * 0.5f));
-    l2 = k == 0 ? -(B1v + ic) * 0.5f : (k == 1 ? 0.0f : (k == 2 ? B1v : -(B1v - ic) * 0.5f));
-    l3 = k == 0 ? B1 * 0.5f : (k == 1 ? 0.0f : (k == 2 ? -B1 : B1 * 0.5f));
-  }
+  const Eigen32 g = eigen32<DIR>(gamma, um4, u04);
+  // row k of L on (f0, fn, ft, f3): rows 0 and 3 are Q +- D, row 2 is f0 - 2 Q
+  // (face_flux_f32)
+  const float dn = k == 0 ? -0.5f * g.ic : (k == 3 ? 0.5f * g.ic : 0.0f);
+  const float b = k == 1 ? 0.0f : (k == 2 ? -2.0f * g.b : g.b);
+  const float l0 = k == 1 ? g.ut : __fmaf_rn(b, g.k2, __fmaf_rn(-dn, g.un, k == 2 ? 1.0f : 0.0f));
+  const float ln = __fmaf_rn(-b, g.un, dn), lt = k == 1 ? -1.0f : __fmul_rn(-b, g.ut);
   float vp[5], vm[5];
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
-    const float4 a = P[s * ss], b = M[s * ss];
-    float x = l0 * a.x;
-    x += l1 * a.y;
-    x += l2 * a.z;
-    x += l3 * a.w;
-    vp[s] = x;
-    float y = l0 * b.x;
-    y += l1 * b.y;
-    y += l2 * b.z;
-    y += l3 * b.w;
-    vm[s] = y;
+    const float4 x = P[s * ss], y = M[s * ss];
+    vp[s] = __fmaf_rn(b, x.w, __fmaf_rn(lt, DIR == 0 ? x.z : x.y, __fmaf_rn(ln, DIR == 0 ? x.y : x.z, __fmul_rn(l0, x.x))));
+    vm[s] = __fmaf_rn(b, y.w, __fmaf_rn(lt, DIR == 0 ? y.z : y.y, __fmaf_rn(ln, DIR == 0 ? y.y : y.z, __fmul_rn(l0, y.x))));
   }
   const float vhk = weno_sides<float, SCHEME>(vp, vm, zpl);
   const int base = (threadIdx.x & 31) & ~3;
-  const float vh0 = __shfl_sync(0xffffffffu, vhk, base + 0);
-  const float vh1 = __shfl_sync(0xffffffffu, vhk, base + 1);
-  const float vh2 = __shfl_sync(0xffffffffu, vhk, base + 2);
-  const float vh3 = __shfl_sync(0xffffffffu, vhk, base + 3);
-  // row k of R (face_flux_st, utils/equations.hpp:239-299)
-  const float q2 = (u * u + v * v) * 0.5f;
-  float r0, r1, r2, r3;
-  if (DIR == 0) {
-    r1 = k == 0 ? 0.0f : (k == 1 ? 0.0f : (k == 2 ? -1.0f : -v));
-    r2 = k == 0 ? 1.0f : (k == 1 ? u : (k == 2 ? v : q2));
-    r3 = k == 0 ? 1.0f : (k == 1 ? u + c : (k == 2 ? v : H + c * u));
-    r0 = k == 0 ? 1.0f : (k == 1 ? u - c : (k == 2 ? v : H - c * u));
-  } else {
-    r1 = k == 0 ? 0.0f : (k == 1 ? 1.0f : (k == 2 ? 0.0f : u));
-    r2 = k == 0 ? 1.0f : (k == 1 ? u : (k == 2 ? v : q2));
-    r3 = k == 0 ? 1.0f : (k == 1 ? u : (k == 2 ? v + c : H + c * v));
-    r0 = k == 0 ? 1.0f : (k == 1 ? u : (k == 2 ? v - c : H - c * v));
-  }
-  float f = r0 * vh0;
-  f += r1 * vh1;
-  f += r2 * vh2;
-  f += r3 * vh3;
-  return f;
+  const float h0 = __shfl_sync(0xffffffffu, vhk, base + 0);
+  const float h1 = __shfl_sync(0xffffffffu, vhk, base + 1);
+  const float h2 = __shfl_sync(0xffffffffu, vhk, base + 2);
+  const float h3 = __shfl_sync(0xffffffffu, vhk, base + 3);
+  // component k of R * vh
+  const float S = __fadd_rn(h0, h3), cD = __fmul_rn(g.c, __fadd_rn(h3, -h0)), o0 = __fadd_rn(S, h2);
+  const int normal = DIR == 0 ? 1 : 2;
+  const float o3 = __fmaf_rn(g.k2, h2, __fmaf_rn(-g.ut, h1, __fmaf_rn(g.un, cD, __fmul_rn(g.H, S))));
+  const float on = __fmaf_rn(g.un, o0, cD), ot = __fmaf_rn(g.ut, o0, -h1);
+  return k == 0 ? o0 : (k == 3 ? o3 : (k == normal ? on : ot));
 }
 
 __device__ __forceinline__ void cp_async8_f32(void *smem, const void *gmem) {
@@ -451,7 +375,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
       const unsigned char *fl = sflag + WENOFD_SPAN(g.guard, f * FS + (j + 2 + FO), (f + 3) * FS + (j + 2 + FO), FI * FS);
       if (fl[0] | fl[FS] | fl[2 * FS] | fl[3 * FS]) slist[WENOFD_IX(g.guard, atomicAdd(&scount_x, 1), kMaxFaces)] = short(t);
     } else {
-      Hf[WENOFD_IX(g.guard, t, S::kFace)] = weno_face4<0, SCHEME>(
+      Hf[WENOFD_IX(g.guard, t, S::kFace)] = face_flux_f32<0, SCHEME>(
           gamma, zpl, Us[WENOFD_IX(g.guard, (f + 2) * HJ + j + 3, S::kU)], Us[WENOFD_IX(g.guard, (f + 3) * HJ + j + 3, S::kU)],
           Fp + WENOFD_SPAN(g.guard, t, t + 4 * TJ, S::kSplit), Fm + WENOFD_SPAN(g.guard, t + TJ, t + 5 * TJ, S::kSplit), TJ);
     }
@@ -512,7 +436,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
       const unsigned char *fl = sflag + WENOFD_SPAN(g.guard, (i + 2) * FS + f + FO, (i + 2) * FS + f + FO + 3, FI * FS);
       if (fl[0] | fl[1] | fl[2] | fl[3]) slist[WENOFD_IX(g.guard, atomicAdd(&scount_y, 1), kMaxFaces)] = short(t);
     } else {
-      Hf[WENOFD_IX(g.guard, t, S::kFace)] = weno_face4<1, SCHEME>(
+      Hf[WENOFD_IX(g.guard, t, S::kFace)] = face_flux_f32<1, SCHEME>(
           gamma, zpl, Us[WENOFD_IX(g.guard, (i + 3) * HJ + f + 2, S::kU)], Us[WENOFD_IX(g.guard, (i + 3) * HJ + f + 3, S::kU)],
           Fp + WENOFD_SPAN(g.guard, s, s + 4, S::kSplit), Fm + WENOFD_SPAN(g.guard, s + 1, s + 5, S::kSplit), 1);
     }

@@ -167,3 +167,29 @@ def test_tma_tiles_on_small_and_ragged_grids(nx, ny, tile_i):
         if U64 is not None:
             assert np.max(np.abs(U32 - U64)) <= 1e-3 * scale, (tc, nx, ny)
         assert np.max(np.abs(Ul - U32)) <= 1e-3 * scale, (tc, nx, ny)
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 9), (15, 32), (16, 33), (31, 64), (46, 97)])
+@pytest.mark.parametrize("scheme", [orc.WENOJS, orc.WENOZ])
+@pytest.mark.parametrize("tile_i", [0, 31])
+def test_fp32_rhs_of_a_smooth_flow_is_fp64_to_rounding(nx, ny, scheme, tile_i):
+    """Where the reconstruction's weights are well conditioned (the smooth
+    wave; a stencil that is flat up to roundoff has weights of 0/0) the FP32 RHS
+    differs from FP64's by rounding alone: a face flux is a few dozen operations
+    on values of at most max(|F| + (|u| + c) |U|), so 32 roundings of 2^-24 each
+    of that on two faces per direction bound it."""
+    rhs = {}
+    for prec in (wenofd.FP64, wenofd.FP32):
+        cfg = {"TESTCASE": orc.SMOOTH, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.5, "SCHEME": scheme,
+               "PRECISION": prec, "TILE_I": tile_i if prec == wenofd.FP32 else 0}
+        with wenofd.Solver(cfg) as s:
+            s.initialize()
+            U, info = s.get_state(), s.info()
+            rhs[prec] = s.get_flux()
+    u, v = U[1] / U[0], U[2] / U[0]
+    p = (info.gamma - 1) * (U[3] - 0.5 * U[0] * (u * u + v * v))
+    c = np.sqrt(info.gamma * p / U[0])
+    speed = np.max(np.abs(u)) + np.max(np.abs(v)) + np.max(c)
+    largest = speed * max(np.max(np.abs(U)), np.max(U[3] + p)) * 2
+    bound = 32 * 2.0 ** -24 * largest * (2 / info.dx + 2 / info.dy)
+    assert np.max(np.abs(rhs[wenofd.FP32] - rhs[wenofd.FP64])) <= bound
