@@ -3,6 +3,7 @@
 // ghost entry and a node's wave-speed sum for the time step.
 #pragma once
 
+#include "approx.cuh"
 #include "convert.cuh"
 #include "guard.cuh"
 #include "wenofd_internal.h"
@@ -149,40 +150,38 @@ __device__ __forceinline__ double exact_speed(const Geom &g, double rho, double 
 }
 
 // FP32 estimate s32 of a node's s and a bound e with |s32 - s| <= e.  Error
-// budget (eps = 2^-23): inputs truncated to FP32 (eps each), u and v from
-// __fdividef (3 eps), kinetic energy ke (< 9.5 eps relative), so
-// p = (gamma-1)(E - ke) carries at most 12 eps (|E| + ke) / (E - ke)
-// relative error (the cancellation term); c = sqrt(gamma p / rho) half of
-// that plus 2 eps; the final bound takes 4x the propagated sum.  Nodes with
-// a non-positive or non-finite FP32 pressure get e = inf.
+// budget (eps = 2^-23, each operation and the hardware's reciprocal and root at
+// most eps): inputs truncated to FP32 (eps each), u and v 4 eps, kinetic energy
+// ke 7 eps, so p = (gamma-1)(E - ke) carries at most rp = 12 eps (|E| + ke) /
+// (E - ke) relative error (the cancellation term); c^2 that plus 5 eps, c half
+// of it plus eps; s = (|u| + c)/dx + (|v| + c)/dy then 7 eps of itself plus rp/2
+// of c/dx + c/dy.  The bound takes 4x that.  Nodes with a non-positive or
+// non-finite FP32 pressure or sound speed get e = inf.  (About 30 instructions:
+// the last stage of every step runs it on every node; IEEE divisions and root
+// here took some 100.)
 __device__ __forceinline__ void screen_speed(const Geom &g, double rho_d, double mu_d, double mv_d, double E_d,
                                              float &s, float &e) {
   // Explicit round-to-nearest operations: no multiply-add contraction, so
   // every translation unit (the stage kernels' fused screen, the reduction
   // kernels, the batched kernel) computes the same s and e.
   const float eps = 1.1920929e-07f;
-  const float r = f64_to_f32(rho_d), mu = f64_to_f32(mu_d), mv = f64_to_f32(mv_d), E = f64_to_f32(E_d);
-  const float u = __fdividef(mu, r), v = __fdividef(mv, r);
-  const float ke = __fmul_rn(__fmul_rn(0.5f, r), __fadd_rn(__fmul_rn(u, u), __fmul_rn(v, v)));
-  const float pp = __fsub_rn(E, ke);
-  const float c2 = __fdividef(__fmul_rn(g.gamma32, __fmul_rn(__fsub_rn(g.gamma32, 1.0f), pp)), r);
-  if (!(pp > 0.0f) || !(c2 > 0.0f) || !(c2 < 3.0e38f) || !(fabsf(u) < 3.0e38f) || !(fabsf(v) < 3.0e38f)) {
+  const float4 q = f64x4_to_f32(rho_d, mu_d, mv_d, E_d);
+  const float ir = rcp_ftz(q.x), u = __fmul_rn(q.y, ir), v = __fmul_rn(q.z, ir);
+  const float ke = __fmul_rn(0.5f, __fmaf_rn(q.y, u, __fmul_rn(q.z, v)));
+  const float pp = __fadd_rn(q.w, -ke);
+  const float c2 = __fmul_rn(__fmul_rn(__fmul_rn(g.gamma32, __fadd_rn(g.gamma32, -1.0f)), pp), ir);
+  if (!(pp > 0.0f) || !(c2 > 0.0f) || !(c2 < 3.0e38f)) {
     s = 0.0f;
     e = __int_as_float(0x7f800000);
     return;
   }
-  const float c = __fsqrt_rn(c2);
-  const float au = fabsf(u), av = fabsf(v);
-  s = __fadd_rn(__fmul_rn(__fadd_rn(au, c), g.inv_dx32), __fmul_rn(__fadd_rn(av, c), g.inv_dy32));
-  const float rp = __fdiv_rn(__fmul_rn(__fmul_rn(12.0f, eps), __fadd_rn(fabsf(E), ke)), pp);
-  const float rc = __fadd_rn(__fmul_rn(0.5f, rp), __fmul_rn(2.0f, eps));
-  const float ex = __fadd_rn(__fmul_rn(__fmul_rn(au, 3.0f), eps), __fmul_rn(c, rc));
-  const float ey = __fadd_rn(__fmul_rn(__fmul_rn(av, 3.0f), eps), __fmul_rn(c, rc));
-  e = __fadd_rn(__fmul_rn(4.0f, __fadd_rn(__fadd_rn(__fmul_rn(ex, g.inv_dx32), __fmul_rn(ey, g.inv_dy32)),
-                                          __fmul_rn(__fmul_rn(s, 4.0f), eps))),
-                __fmul_rn(1e-12f, s));
+  const float c = sqrt_ftz(c2);
+  const float cs = __fmaf_rn(c, g.inv_dx32, __fmul_rn(c, g.inv_dy32));
+  s = __fmaf_rn(fabsf(u), g.inv_dx32, __fmaf_rn(fabsf(v), g.inv_dy32, cs));
+  // 4 (7 eps s + (rp / 2) cs)
+  const float rp = __fmul_rn(__fadd_rn(fabsf(q.w), ke), rcp_ftz(pp));
+  e = __fmul_rn(eps, __fmaf_rn(28.0f, s, __fmul_rn(24.0f, __fmul_rn(rp, cs))));
 }
-
 
 }  // namespace dev
 }  // namespace wenofd

@@ -9,6 +9,7 @@
 // infinity-07/FD-WENO-EulerEquation.
 #pragma once
 
+#include "approx.cuh"
 #include "int_f64.cuh"
 #include "wenofd_internal.h"
 
@@ -238,24 +239,9 @@ __device__ __forceinline__ T weno(T a, T b, T c, T d, T e, T zp_lambda) {
 //   candidates themselves.
 // Explicitly rounded operations: every unit computes the same bits.
 // The reciprocals, and the roots of the face's eigenvectors, are the bare
-// hardware approximations (about 1 ulp; a zero divisor is out of reach of B_k,
-// and subnormal ones count as zero): with the division intrinsic's handling of
-// subnormals one reconstruction takes 104 instructions instead of 65.
-__device__ __forceinline__ float rcp_ftz(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float sqrt_ftz(float x) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
+// hardware approximations (approx.cuh; B_k is never zero): with the division
+// intrinsic's handling of subnormals one reconstruction takes 104 instructions
+// instead of 65.
 __device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_ftz(x.x), rcp_ftz(x.y)); }
 
 template <int SCHEME>

@@ -53,42 +53,30 @@ struct StageSmem32 {
       128 + sizeof(float4) * (size_t(kU) + 2 * kSplit + kFace) + sizeof(double) * kKeep;
 };
 
-// Linear fifth-order upwind flux of one component: WENO with its weights
-// frozen at (0.1, 0.6, 0.3), on F+ at nodes face-3..face+1 (p0..p4) and on F-
-// mirrored (nodes face+2..face-2, m4..m0): (2a - 13b + 47c + 27d - 3e) / 60
-// each.
-__device__ __forceinline__ float lin5(float p0, float p1, float p2, float p3, float p4, float m0, float m1, float m2,
-                                      float m3, float m4) {
-  const float c0 = float(2.0 / 60.0), c1 = float(-13.0 / 60.0), c2 = float(47.0 / 60.0), c3 = float(27.0 / 60.0),
-              c4 = float(-3.0 / 60.0);
-  const float plus = c0 * p0 + c1 * p1 + c2 * p2 + c3 * p3 + c4 * p4;
-  const float minus = c0 * m4 + c1 * m3 + c2 * m2 + c3 * m1 + c4 * m0;
-  return plus + minus;
-}
-
-// lin5 on two components at once (the same operation order).
-__device__ __forceinline__ float2 lin5x2(float2 p0, float2 p1, float2 p2, float2 p3, float2 p4, float2 m0, float2 m1,
-                                         float2 m2, float2 m3, float2 m4) {
-  const float2 c0 = splat2(float(2.0 / 60.0)), c1 = splat2(float(-13.0 / 60.0)), c2 = splat2(float(47.0 / 60.0)),
-               c3 = splat2(float(27.0 / 60.0)), c4 = splat2(float(-3.0 / 60.0));
-  float2 plus = __fmul2_rn(c0, p0);
-  plus = __ffma2_rn(c1, p1, plus);
-  plus = __ffma2_rn(c2, p2, plus);
-  plus = __ffma2_rn(c3, p3, plus);
-  plus = __ffma2_rn(c4, p4, plus);
-  float2 minus = __fmul2_rn(c0, m4);
-  minus = __ffma2_rn(c1, m3, minus);
-  minus = __ffma2_rn(c2, m2, minus);
-  minus = __ffma2_rn(c3, m1, minus);
-  minus = __ffma2_rn(c4, m0, minus);
-  return __fadd2_rn(plus, minus);
+// Linear fifth-order upwind flux at a face: WENO with its weights frozen at
+// (0.1, 0.6, 0.3), (2a - 13b + 47c + 27d - 3e) / 60 of F+ at nodes face-3..
+// face+1 (P) and the mirror image of F- at nodes face+2..face-2 (M, from its
+// first node), summed node by node: every kernel adds in this order.
+__host__ __device__ constexpr float lin_coef(int s) {
+  return s == 0 ? float(2.0 / 60.0)
+                : (s == 1 ? float(-13.0 / 60.0) : (s == 2 ? float(47.0 / 60.0) : (s == 3 ? float(27.0 / 60.0) : float(-3.0 / 60.0))));
 }
 
 __device__ __forceinline__ float4 linear_face4(const float4 *P, const float4 *M, int ss) {
-  const float4 p0 = P[0], p1 = P[ss], p2 = P[2 * ss], p3 = P[3 * ss], p4 = P[4 * ss];
-  const float4 m0 = M[0], m1 = M[ss], m2 = M[2 * ss], m3 = M[3 * ss], m4 = M[4 * ss];
-  return join2(lin5x2(lo2(p0), lo2(p1), lo2(p2), lo2(p3), lo2(p4), lo2(m0), lo2(m1), lo2(m2), lo2(m3), lo2(m4)),
-               lin5x2(hi2(p0), hi2(p1), hi2(p2), hi2(p3), hi2(p4), hi2(m0), hi2(m1), hi2(m2), hi2(m3), hi2(m4)));
+  const float4 first = P[0];
+  float2 lo = __fmul2_rn(splat2(lin_coef(0)), lo2(first)), hi = __fmul2_rn(splat2(lin_coef(0)), hi2(first));
+#pragma unroll
+  for (int s = 1; s < 6; ++s) {
+    if (s < 5) {
+      const float4 p = P[s * ss];
+      lo = __ffma2_rn(splat2(lin_coef(s)), lo2(p), lo);
+      hi = __ffma2_rn(splat2(lin_coef(s)), hi2(p), hi);
+    }
+    const float4 m = M[(s - 1) * ss];
+    lo = __ffma2_rn(splat2(lin_coef(5 - s)), lo2(m), lo);
+    hi = __ffma2_rn(splat2(lin_coef(5 - s)), hi2(m), hi);
+  }
+  return join2(lo, hi);
 }
 
 // One characteristic field of a WENO face, for the routed form where the
@@ -137,6 +125,58 @@ __device__ __forceinline__ void cp_async_wait_all_f32() { asm volatile("cp.async
 // Asks L2 for the 128-byte line holding p (a hint: no data moves to the
 // thread, and nothing waits for it).
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.L2 [%0];" ::"l"(p)); }
+
+// The RK combination of one node in FP64 (kModeRHS: the RHS itself).  FP64
+// runs at 1/64 of the FP32 rate here, and the RK combination is most of a
+// routed stage's FP64 work: the middle stages with c = b = 2^-k take c * (dt *
+// rhs + (a / c) * U^n + U), two FP64 operations per component instead of three,
+// the power-of-two scale on the integer ALU.  The form comes from the host
+// (StageArgs::form), so no FP64 compare runs here.
+__device__ __forceinline__ void rk_combine(const StageArgs &a, const double dt, const float rr[4], const double ui[4],
+                                           const double un[4], double w[4]) {
+  double rd[4];
+  f32x4_to_f64(rr, rd);
+  if (a.mode == kModeRHS) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = rd[r];
+  } else if (a.form == kFormStage1) {  // (1, 0, 1): c * dt = dt
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = fma(dt, rd[r], ui[r]);
+  } else if (a.form == kFormRK3Mid) {  // (3/4, 1/4, 1/4)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = fma(dt, rd[r], fma(3.0, un[r], ui[r]));
+    scale4_pow2_down<2>(w);
+  } else if (a.form == kFormRK2Mid) {  // (1/2, 1/2, 1/2)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = fma(dt, rd[r], un[r] + ui[r]);
+    scale4_pow2_down<1>(w);
+  } else {
+    const double cdt = a.c * dt;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = fma(cdt, rd[r], fma(a.b, ui[r], a.a * un[r]));
+  }
+}
+
+// A tile's screen bounds from its threads' (all NT threads of the block).
+template <int NT>
+__device__ __forceinline__ void store_tile_bounds(const Geom &g, const StageArgs &a, float lo, float hi, int tile) {
+  __shared__ float2 sred[NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = make_float2(lo, hi);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float2 b = sred[0];
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w) b = make_float2(fmaxf(b.x, sred[w].x), fmaxf(b.y, sred[w].y));
+    // (allocated for tiles of 15 rows, the most tiles)
+    a.bounds[WENOFD_IX(g.guard, tile, ((g.nx + 14) / 15) * ((g.ny + 31) / 32))] = b;
+    atomicMax(a.screen, __float_as_uint(b.x));
+  }
+}
 
 // One tile (TI x TJ interior nodes from i0, j0) of one RK stage, all NT
 // threads of the block.  ROUTE: faces take the linear upwind flux unless a
@@ -258,7 +298,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
 #pragma unroll
         for (int r = 0; r < 4; ++r) x[r] = h ? v[r].y : v[r].x;
         Us[WENOFD_IX(g.guard, hi * HJ + hj, S::kU)] =
-            make_float4(f64_to_f32(x[0]), f64_to_f32(x[1]), f64_to_f32(x[2]), f64_to_f32(x[3]));
+            f64x4_to_f32(x[0], x[1], x[2], x[3]);
         if constexpr (KEEP) {
           if (hi >= 3 && hi < 3 + TI && hj >= 3 && hj < 3 + TJ) {
             const int q = (hi - 3) * TJ + hj - 3;
@@ -326,7 +366,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
 #pragma unroll
           for (int r = 0; r < 4; ++r) x[r] = h ? v[k][r].y : v[k][r].x;
           Us[WENOFD_IX(g.guard, hi * HJ + hj, S::kU)] =
-              make_float4(f64_to_f32(x[0]), f64_to_f32(x[1]), f64_to_f32(x[2]), f64_to_f32(x[3]));
+              f64x4_to_f32(x[0], x[1], x[2], x[3]);
           if constexpr (KEEP) {
             if (hi >= 3 && hi < 3 + TI && hj >= 3 && hj < 3 + TJ) {
               const int q = (hi - 3) * TJ + hj - 3;
@@ -461,12 +501,6 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
 
   // --- y term, source, RK combination in FP64, store
   const double dt = COH ? __ldcg(a.dt) : *a.dt;
-  // FP64 runs at 1/64 of the FP32 rate here, and the RK combination is most
-  // of a routed stage's FP64 work: the middle stages with c = b = 2^-k take
-  // c * (dt * rhs + (a / c) * U^n + U), two FP64 operations per component
-  // instead of three, the power-of-two scale on the integer ALU.  The form
-  // comes from the host (StageArgs::form), so no FP64 compare runs here.
-  const int form = a.form;
   if constexpr (!COH && KEEP) {
     cp_async_wait_all_f32();
     __syncthreads();
@@ -507,17 +541,9 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
       }
     }
     double w[4];
+    rk_combine(a, dt, rr, ui, un, w);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const long long ix = r * g.plane + gidx;
-      const double rd = f32_to_f64(rr[r]);
-      if (a.mode == kModeRHS) w[r] = rd;
-      else if (form == kFormStage1) w[r] = fma(dt, rd, ui[r]);  // (1, 0, 1): c * dt = dt
-      else if (form == kFormRK3Mid) w[r] = scale_pow2_down<2>(fma(dt, rd, fma(3.0, un[r], ui[r])));  // (3/4, 1/4, 1/4)
-      else if (form == kFormRK2Mid) w[r] = scale_pow2_down<1>(fma(dt, rd, un[r] + ui[r]));          // (1/2, 1/2, 1/2)
-      else w[r] = fma(a.c * dt, rd, fma(a.b, ui[r], a.a * un[r]));
-      a.uout[ix] = w[r];
-    }
+    for (int r = 0; r < 4; ++r) a.uout[r * g.plane + gidx] = w[r];
     if (a.bounds) {
       float s32, e;
       screen_speed(g, w[0], w[1], w[2], w[3], s32, e);
@@ -525,24 +551,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
       hi = fmaxf(hi, s32 + e);
     }
   }
-  if (a.bounds) {  // block-uniform
-    __shared__ float2 sred[NT / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = make_float2(lo, hi);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float2 b = sred[0];
-#pragma unroll
-      for (int w = 1; w < NT / 32; ++w) b = make_float2(fmaxf(b.x, sred[w].x), fmaxf(b.y, sred[w].y));
-      // (allocated for tiles of 15 rows, the most tiles)
-      a.bounds[WENOFD_IX(g.guard, tile, ((g.nx + 14) / 15) * ((g.ny + 31) / 32))] = b;
-      atomicMax(a.screen, __float_as_uint(b.x));
-    }
-  }
+  if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, tile);  // block-uniform
 }
 
 }  // namespace dev
