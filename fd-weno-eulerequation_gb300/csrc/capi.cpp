@@ -151,7 +151,8 @@ int launch_stage(wenofd_solver *s, const double *in, const double *un, double *o
   }
   args.wait_error = s->wait_error;
   if (s->precision != WENOFD_FP64) {
-    CUDA_TRY(wenofd::launch_stage_fp32(s->g, args, s->tma[stage_buffer(s, in)], s->scheme, s->tile_i, s->stream));
+    CUDA_TRY(wenofd::launch_stage_fp32(s->g, args, s->tma[stage_buffer(s, in)], s->scheme, s->tile_i, s->stage_rows,
+                                       s->stream));
   } else {
     CUDA_TRY(wenofd::launch_stage_fp64(s->g, args, s->tma[stage_buffer(s, in)], s->scheme, s->tile_i, s->stream));
   }
@@ -189,7 +190,7 @@ int enqueue_dt_reduce(wenofd_solver *s) {
     CUDA_TRY(wenofd::launch_dt_reduce(s->g, s->S, s->ctrl, s->stream));
     s->launches += 1;
   } else {
-    CUDA_TRY(wenofd::launch_dt_reduce_two_pass(s->g, s->S, s->ctrl, s->tile_bounds, s->tile_i, s->stream));
+    CUDA_TRY(wenofd::launch_dt_reduce_two_pass(s->g, s->S, s->ctrl, s->tile_bounds, s->stage_rows, s->stream));
     s->launches += 2;
   }
   return WENOFD_OK;
@@ -368,7 +369,7 @@ int create_from_map(const std::map<std::string, std::string> &opt, wenofd_solver
             cudaMalloc(&s->ctrl, sizeof(Ctrl)) == cudaSuccess &&
             cudaMallocHost(&s->ctrl_host, sizeof(Ctrl)) == cudaSuccess &&
             cudaMallocHost(&s->red_host, 4 * sizeof(double)) == cudaSuccess;
-  if (ok && precision != WENOFD_FP64) {  // stage tiles of 15 (or 31) x 32 nodes
+  if (ok && precision != WENOFD_FP64) {  // stage tiles of 15 (or 16, or 31) x 32 nodes
     const size_t tiles = size_t((nx + 14) / 15) * size_t((ny + 31) / 32);
     ok = cudaMalloc(&s->tile_bounds, tiles * sizeof(float2)) == cudaSuccess;
   }
@@ -387,8 +388,9 @@ int create_from_map(const std::map<std::string, std::string> &opt, wenofd_solver
   }
   {  // TMA maps of the three stage inputs
     double *bufs[3] = {s->S, s->A, s->B};
+    s->stage_rows = wenofd::stage_rows(s->g, precision, tile_i);
     for (int k = 0; k < 3; ++k)
-      if ((e = wenofd::make_stage_tma(s->g, bufs[k], s->flags, tile_i, &s->tma[k])) != cudaSuccess)
+      if ((e = wenofd::make_stage_tma(s->g, bufs[k], s->flags, s->stage_rows, &s->tma[k])) != cudaSuccess)
         return bail(fail(WENOFD_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the stage tiles' TMA maps"));
   }
   ok = cudaMemsetAsync(s->S, 0, s->state_bytes, s->stream) == cudaSuccess &&
@@ -425,7 +427,7 @@ namespace {
 void guard_fill_report(const unsigned long long h[wenofd::kGuardWords], long long report[4], char *where,
                        int where_len) {
   static const char *const kFiles[] = {"aux_device.cuh", "aux_kernels.cu",   "batch_kernel.cuh", "learned.cu",
-                                       "learned_data.cu", "noalloc.cu",      "stage_f32.cuh",    "stage_kernel.cuh",
+                                       "learned_data.cu", "noalloc.cu",      "stage_f32.cuh",    "stage_kernel.cuh", "stage_routed.cuh",
                                        "guard.cuh",       "physics.cuh",     "tma.cuh"};
   report[0] = (long long)h[wenofd::kGuardCount];
   report[1] = h[wenofd::kGuardCount] ? (long long)(h[wenofd::kGuardSite] & 0xffffffffull) : 0;
@@ -787,7 +789,7 @@ int wenofd_time_stages(wenofd_solver *s, int reps, double *ms_per_launch) {
       a.wait_error = s->wait_error;
       cudaError_t e = s->precision != WENOFD_FP64
                           ? wenofd::launch_stage_fp32(s->g, a, s->tma[stage_buffer(s, x.in)], s->scheme, s->tile_i,
-                                                      s->stream)
+                                                      s->stage_rows, s->stream)
                           : wenofd::launch_stage_fp64(s->g, a, s->tma[stage_buffer(s, x.in)], s->scheme, s->tile_i,
                                                       s->stream);
       CUDA_TRY(e);

@@ -7,13 +7,58 @@
 #include <mutex>
 
 #include "stage_kernel.cuh"
+#include "stage_routed.cuh"
 
 namespace wenofd {
 
+namespace {
+
+template <int SCHEME>
+cudaError_t launch_routed(const Geom &g, const StageArgs &a, const StageTma &tma, cudaStream_t s) {
+  using T = dev::RoutedTile;
+  static unsigned long long configured = 0;  // one bit per device (launch_stage_tile)
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (device & 63);
+  if (!(configured & bit)) {
+    e = cudaFuncSetAttribute(dev::k_stage_routed<SCHEME>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(T::bytes));
+    if (e != cudaSuccess) return e;
+    configured |= bit;
+  }
+  const dim3 grid((g.ny + T::TJ - 1) / T::TJ, (g.nx + T::TI - 1) / T::TI);
+  dev::k_stage_routed<SCHEME><<<grid, T::NT, T::bytes, s>>>(g, a, tma);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+// The learned form's default tile: k_stage_routed's where its tiles fill the
+// resident blocks (four on each of 152 SMs) one and a half times, else 15 x 32,
+// whose block is done sooner.  Measured, 8 steps (k_stage_routed / 15 x 32): 512^2
+// 920 / 911 us, 700^2 1,133 / 1,145, 1024^2 1,694 / 1,764, 2048^2 4,538 / 4,801.
+int stage_rows(const Geom &g, int precision, int tile_i) {
+  using T = dev::RoutedTile;
+  if (precision == 2 && tile_i == 0) {
+    const long long tiles = (long long)((g.nx + T::TI - 1) / T::TI) * ((g.ny + T::TJ - 1) / T::TJ);
+    if (tiles > 3LL * T::kBlocks * 152 / 2) return T::TI;
+  }
+  return tile_i > 0 ? tile_i : 15;
+}
+
 // With a.flags set the kernel routes each face: linear upwind flux unless a
 // node around it is flagged, characteristic WENO otherwise.
-cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i,
+cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i, int rows,
                               cudaStream_t s) {
+  if (a.flags && rows == dev::RoutedTile::TI && tile_i == 0) {
+    switch (scheme) {
+      case kWenoJS: return launch_routed<kWenoJS>(g, a, tma, s);
+      case kWenoZ: return launch_routed<kWenoZ>(g, a, tma, s);
+      case kWenoZP: return launch_routed<kWenoZP>(g, a, tma, s);
+      case kWenoZPI: return launch_routed<kWenoZPI>(g, a, tma, s);
+    }
+    return cudaErrorInvalidValue;
+  }
   if (a.flags) {
     switch (tile_i) {
       case 0:
@@ -50,11 +95,11 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 }  // namespace
 
-cudaError_t make_stage_tma(const Geom &g, const double *state, const unsigned char *flags, int tile_i,
+cudaError_t make_stage_tma(const Geom &g, const double *state, const unsigned char *flags, int rows,
                            StageTma *out) {
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode || !out || !state) return cudaErrorInvalidValue;
-  const int ti = (tile_i == 31 || tile_i == 7) ? tile_i : 15;
+  const int ti = (rows == 31 || rows == 7 || rows == dev::RoutedTile::TI) ? rows : 15;
   *out = StageTma{};
   {
     using S = dev::StageSmem32<15, 32>;

@@ -98,9 +98,11 @@ struct StageTma {
   CUtensorMap flags;
 };
 // Encodes the maps of one state array (and of the flag array, if not null)
-// for stage tiles of tile_i rows (FP32 tiles 15 or 31, FP64 tiles 15 or 7).
-cudaError_t make_stage_tma(const Geom &g, const double *state, const unsigned char *flags, int tile_i,
-                           StageTma *out);
+// for stage tiles of up to `rows` rows (FP32 tiles 15 or 31, the learned form's
+// 16, FP64 tiles 15 or 7; stage_rows).
+cudaError_t make_stage_tma(const Geom &g, const double *state, const unsigned char *flags, int rows, StageTma *out);
+// Rows of the per-solve stage tiles of a precision form with TILE_I = tile_i.
+int stage_rows(const Geom &g, int precision, int tile_i);
 enum { kModeRK = 0, kModeRHS = 1 };
 // RK stage forms: a = 1, b = 0 on U^n itself (stage 1); SSP-RK3's middle
 // stage (3/4, 1/4, 1/4); RK2's second stage (1/2, 1/2, 1/2); any other.
@@ -137,8 +139,8 @@ struct Fp64Split {
 // given grids soonest on `sms` SMs.
 Fp64Split fp64_split(const int *nx, const int *ny, int n, int sms, int most);
 // The FP32 tiles load their halo by TMA: `tma` holds the maps of a.uin (and
-// of a.flags) for tiles of tile_i rows.
-cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i,
+// of a.flags) for tiles of `rows` rows (stage_rows).
+cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma &tma, int scheme, int tile_i, int rows,
                               cudaStream_t s);
 
 // batch_fp64.cu / batch_fp32.cu: the persistent batched kernel

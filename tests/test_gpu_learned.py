@@ -356,3 +356,26 @@ def test_indicator_guard_keeps_strong_jumps_physical():
         U64 = s.get_state()
     assert np.all(np.isfinite(U)) and np.all(U[0] > 0)
     assert np.mean(np.abs(U[0] - U64[0])) <= 0.05 * np.mean(np.abs(U64[0]))
+
+
+@pytest.mark.parametrize("nx,ny", [(17, 14700), (14620, 33), (701, 707)])
+@pytest.mark.parametrize("testcase", [orc.SHEAR, orc.RIEMANN_SEEDED, orc.RTI])
+@pytest.mark.parametrize("rk", [1, 2])
+def test_routed_tile_of_large_grids_equals_the_small_tile(nx, ny, testcase, rk):
+    """Grids of many tiles take a 16 x 32 tile by default, others (and TILE_I =
+    15) the 15 x 32 one.  Both do the same operations in the same order, so the
+    states are the same bits: on one tile and a remainder in each direction, with
+    no, some and every node flagged, periodic, mirrored, wall and fixed ghosts."""
+    few = mlp_oracle.init_params(5)
+    few[2720] -= 1.0
+    for params in (_constant_net(-50.0), few, _constant_net(50.0)):
+        got = []
+        for tile in (0, 15):
+            with wenofd.Solver({"TESTCASE": testcase, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": rk, "CFL": 0.4,
+                                "SCHEME": 1, "SEED": 5, "PRECISION": wenofd.LEARNED, "TILE_I": tile,
+                                "INDICATOR_GUARD": 0.5}) as s:
+                s.initialize()
+                s.set_indicator(params, 0.5)
+                assert s.advance(max_steps=2) == 2
+                got.append(s.get_state())
+        assert np.array_equal(got[0], got[1])
