@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -49,114 +50,180 @@ __global__ void k_mlp_forward(const float *P, const float *X, long long n, float
   }
 }
 
-// One block = kBB samples of the batch.  Per sample: forward, dL/dlogit of
-// the mean binary cross-entropy (scaled by inv_n), back-propagation to dz1,
-// dz2.  Then the block sums the weight gradients over its samples and adds
-// them (and its loss share) to grad / loss with one atomic per entry, or,
+// The backward pass of the mean binary cross-entropy (scaled by inv_n).  A
+// block of 256 threads takes groups of kGroup = 32 samples: lane = sample, warp =
+// four hidden units in the forward pass and in the back-propagation (a unit's
+// weights are one broadcast 128-bit load for four inputs, the activations lie
+// [unit][sample]), then lane = output unit, warp = a range of inputs for the
+// weight gradients, whose sums stay in registers over the block's groups.  At
+// the end the block adds its sums to grad / loss with one atomic per entry or,
 // given `part`, writes them to its own row there for an ordered sum.
-constexpr int kBB = 128;
+// What bounds it: the latency of one group's chain of small products; a
+// mini-batch of 4,096 samples is 128 blocks.  (128 samples a block, a thread a
+// sample: 32 blocks on 152 SMs, 97 us a mini-batch.)
+constexpr int kGroup = 32, kBackThreads = 256, kBackBlocks = 4 * 152;
+constexpr int kSS = kGroup + 4;   // row stride of [unit][sample] arrays (128-bit aligned, no bank conflicts)
+constexpr int kWS = 52;           // row stride of W1 in shared memory
+
+struct BackSmem {
+  // read as float4: 16-byte aligned arrays and rows
+  float w1[kHid * kWS], w2[kHid * kHid];
+  float x[kIn * kSS], h1[kHid * kSS], h2[kHid * kSS], dz1[kHid * kSS], dz2[kHid * kSS];
+  float d[kGroup], loss[kGroup];
+  float sum[8 * kGroup], b1[kHid], b2[kHid], w3[kHid], b3;
+};
+static_assert(kSS % 4 == 0 && kWS % 4 == 0, "16-byte aligned rows");
+static_assert(offsetof(BackSmem, w2) % 16 == 0 && offsetof(BackSmem, x) % 16 == 0 && offsetof(BackSmem, h1) % 16 == 0 &&
+                  offsetof(BackSmem, h2) % 16 == 0 && offsetof(BackSmem, dz1) % 16 == 0 &&
+                  offsetof(BackSmem, dz2) % 16 == 0 && offsetof(BackSmem, d) % 16 == 0 &&
+                  offsetof(BackSmem, loss) % 16 == 0,
+              "16-byte aligned arrays");
+
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float dot4(const float4 a, const float4 b, float c) {
+  c = fmaf(a.x, b.x, c);
+  c = fmaf(a.y, b.y, c);
+  c = fmaf(a.z, b.z, c);
+  return fmaf(a.w, b.w, c);
+}
 
 // rows: with idx set, sample s of the mini-batch is row idx[s] of X and Y
 // (rows of them in all).
-__global__ void __launch_bounds__(kBB) k_mlp_backward(const float *P, const float *X, const float *Y, long long n,
-                                                      float inv_n, float *grad, float *loss, float *part,
-                                                      const long long *idx, long long rows,
-                                                      unsigned long long *guard) {
-  extern __shared__ float sm[];
-  float *sp = sm;                  // kParams
-  float *sx = sp + kParams;        // kBB * kIn
-  float *sdz1 = sx + kBB * kIn;    // kBB * kHid
-  float *sh1 = sdz1 + kBB * kHid;  // kBB * kHid
-  float *sdz2 = sh1 + kBB * kHid;  // kBB * kHid
-  float *sh2 = sdz2 + kBB * kHid;  // kBB * kHid
-  float *sd = sh2 + kBB * kHid;    // kBB
-  float *sl = sd + kBB;            // kBB
-  for (int k = threadIdx.x; k < kParams; k += kBB) sp[k] = P[k];
-  const long long s0 = (long long)blockIdx.x * kBB;
-  for (int k = threadIdx.x; k < kBB * kIn; k += kBB) {
-    const long long s = s0 + k / kIn;
-    if (s >= n) sx[k] = 0.0f;
-    else if (idx) sx[k] = X[WENOFD_IX(guard, idx[s], rows) * kIn + (k - (k / kIn) * kIn)];
-    else sx[k] = X[s0 * kIn + k];
+__global__ void __launch_bounds__(kBackThreads)
+    k_mlp_backward(const float *P, const float *X, const float *Y, long long n, float inv_n, float *grad, float *loss,
+                   float *part, const unsigned *idx, long long rows, unsigned long long *guard) {
+  extern __shared__ __align__(16) unsigned char back_raw[];
+  BackSmem &S = *reinterpret_cast<BackSmem *>(back_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < kHid * kIn; e += kBackThreads) S.w1[(e / kIn) * kWS + e % kIn] = P[oW1 + e];
+  for (int e = tid; e < kHid * (kWS - kIn); e += kBackThreads) S.w1[(e / 2) * kWS + kIn + (e & 1)] = 0.0f;
+  for (int e = tid; e < kHid * kHid; e += kBackThreads) S.w2[e] = P[oW2 + e];
+  if (tid < kHid) {
+    S.b1[tid] = P[oB1 + tid];
+    S.b2[tid] = P[oB2 + tid];
+    S.w3[tid] = P[oW3 + tid];
   }
-  __syncthreads();
-  const int t = threadIdx.x;
-  const bool valid = s0 + t < n;
-  float z1[kHid];
-  const float *x = sx + t * kIn;
-  for (int o = 0; o < kHid; ++o) {
-    float z = sp[oB1 + o];
-    for (int k = 0; k < kIn; ++k) z += sp[oW1 + o * kIn + k] * x[k];
-    z1[o] = z;
-    sh1[t * kHid + o] = gelu(z);
-  }
-  float z2[kHid];
-  float logit = sp[oB3];
-  for (int o = 0; o < kHid; ++o) {
-    float z = sp[oB2 + o];
-    for (int k = 0; k < kHid; ++k) z += sp[oW2 + o * kHid + k] * sh1[t * kHid + k];
-    z2[o] = z;
-    const float h = gelu(z);
-    sh2[t * kHid + o] = h;
-    logit += sp[oW3 + o] * h;
-  }
-  const float y = valid ? Y[WENOFD_IX(guard, idx ? idx[s0 + t] : s0 + t, rows)] : 0.0f;
-  const float pr = 1.0f / (1.0f + expf(-logit));
-  const float d = valid ? (pr - y) * inv_n : 0.0f;
-  sd[t] = d;
-  sl[t] = valid ? (fmaxf(logit, 0.0f) - logit * y + log1pf(expf(-fabsf(logit)))) * inv_n : 0.0f;
-  for (int o = 0; o < kHid; ++o) sdz2[t * kHid + o] = d * sp[oW3 + o] * gelu_grad(z2[o]);
-  for (int k = 0; k < kHid; ++k) {
-    float dh = 0.0f;
-    for (int o = 0; o < kHid; ++o) dh += sp[oW2 + o * kHid + k] * sdz2[t * kHid + o];
-    sdz1[t * kHid + k] = dh * gelu_grad(z1[k]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kParams; e += kBB) {
-    float acc = 0.0f;
-    if (e < oB1) {
-      const int o = e / kIn, k = e - (e / kIn) * kIn;
-      for (int s = 0; s < kBB; ++s) acc += sdz1[s * kHid + o] * sx[s * kIn + k];
-    } else if (e < oW2) {
-      for (int s = 0; s < kBB; ++s) acc += sdz1[s * kHid + (e - oB1)];
-    } else if (e < oB2) {
-      const int o = (e - oW2) / kHid, k = (e - oW2) - o * kHid;
-      for (int s = 0; s < kBB; ++s) acc += sdz2[s * kHid + o] * sh1[s * kHid + k];
-    } else if (e < oW3) {
-      for (int s = 0; s < kBB; ++s) acc += sdz2[s * kHid + (e - oB2)];
-    } else if (e < oB3) {
-      for (int s = 0; s < kBB; ++s) acc += sd[s] * sh2[s * kHid + (e - oW3)];
-    } else {
-      for (int s = 0; s < kBB; ++s) acc += sd[s];
+  if (tid == 0) S.b3 = P[oB3];
+  // weight gradients of output unit `lane`: inputs 7 warp .. 7 warp + 6 of
+  // layer 1 (warp 7: input 49), inputs 4 warp .. 4 warp + 3 of layer 2; warp 7
+  // also the biases, the output layer and the loss
+  float g1[7] = {0, 0, 0, 0, 0, 0, 0}, g2[4] = {0, 0, 0, 0}, gb1 = 0, gb2 = 0, g3 = 0, gs = 0;
+  const int k0 = 7 * warp, kn = warp < 7 ? 7 : 1;
+  const long long groups = (n + kGroup - 1) / kGroup;
+  for (long long grp = blockIdx.x; grp < groups; grp += gridDim.x) {
+    const long long s0 = grp * kGroup;
+    __syncthreads();  // the last group's sums are done (and the weights are in)
+    for (int e = tid; e < kGroup * kIn; e += kBackThreads) {
+      const int s = e / kIn, k = e - s * kIn;
+      float v = 0.0f;
+      if (s0 + s < n) {
+        const long long row = idx ? (long long)WENOFD_IX(guard, idx[s0 + s], rows) : s0 + s;
+        v = X[row * kIn + k];
+      }
+      S.x[k * kSS + s] = v;
     }
-    if (part) part[(long long)blockIdx.x * (kParams + 1) + e] = acc;
-    else atomicAdd(&grad[e], acc);
+    __syncthreads();
+    const bool valid = s0 + lane < n;
+    const int u0 = 4 * warp;  // this thread's hidden units u0 .. u0 + 3 of sample `lane`
+    float z1[4], z2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) z1[j] = S.b1[u0 + j];
+#pragma unroll
+    for (int k = 0; k < kIn; k += 4) {
+      const float4 x = make_float4(S.x[k * kSS + lane], S.x[(k + 1) * kSS + lane],
+                                   k + 2 < kIn ? S.x[(k + 2) * kSS + lane] : 0.0f,
+                                   k + 3 < kIn ? S.x[(k + 3) * kSS + lane] : 0.0f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z1[j] = dot4(ld4(&S.w1[(u0 + j) * kWS + k]), x, z1[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) S.h1[(u0 + j) * kSS + lane] = gelu(z1[j]);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) z2[j] = S.b2[u0 + j];
+#pragma unroll
+    for (int k = 0; k < kHid; k += 4) {
+      const float4 h = make_float4(S.h1[k * kSS + lane], S.h1[(k + 1) * kSS + lane], S.h1[(k + 2) * kSS + lane],
+                                   S.h1[(k + 3) * kSS + lane]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z2[j] = dot4(ld4(&S.w2[(u0 + j) * kHid + k]), h, z2[j]);
+    }
+    float out = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float h = gelu(z2[j]);
+      S.h2[(u0 + j) * kSS + lane] = h;
+      out = fmaf(S.w3[u0 + j], h, out);
+    }
+    S.sum[warp * kGroup + lane] = out;
+    __syncthreads();
+    float logit = S.b3;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) logit += S.sum[w * kGroup + lane];
+    float y = 0.0f;
+    if (valid) y = Y[idx ? (long long)WENOFD_IX(guard, idx[s0 + lane], rows) : s0 + lane];
+    const float pr = 1.0f / (1.0f + expf(-logit));
+    const float d = valid ? (pr - y) * inv_n : 0.0f;
+    if (warp == 0) {
+      S.d[lane] = d;
+      S.loss[lane] = valid ? (fmaxf(logit, 0.0f) - logit * y + log1pf(expf(-fabsf(logit)))) * inv_n : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) S.dz2[(u0 + j) * kSS + lane] = d * S.w3[u0 + j] * gelu_grad(z2[j]);
+    __syncthreads();
+    float4 dh = make_float4(0, 0, 0, 0);  // dL/dh1 of the units u0 .. u0 + 3
+#pragma unroll 8
+    for (int o = 0; o < kHid; ++o) {
+      const float4 w = ld4(&S.w2[o * kHid + u0]);
+      const float dz = S.dz2[o * kSS + lane];
+      dh.x = fmaf(w.x, dz, dh.x);
+      dh.y = fmaf(w.y, dz, dh.y);
+      dh.z = fmaf(w.z, dz, dh.z);
+      dh.w = fmaf(w.w, dz, dh.w);
+    }
+    S.dz1[(u0 + 0) * kSS + lane] = dh.x * gelu_grad(z1[0]);
+    S.dz1[(u0 + 1) * kSS + lane] = dh.y * gelu_grad(z1[1]);
+    S.dz1[(u0 + 2) * kSS + lane] = dh.z * gelu_grad(z1[2]);
+    S.dz1[(u0 + 3) * kSS + lane] = dh.w * gelu_grad(z1[3]);
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kGroup; s += 4) {
+      const float4 a = ld4(&S.dz1[lane * kSS + s]), c = ld4(&S.dz2[lane * kSS + s]);
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+        if (j < kn) g1[j] = dot4(a, ld4(&S.x[(k0 + j) * kSS + s]), g1[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) g2[j] = dot4(c, ld4(&S.h1[(u0 + j) * kSS + s]), g2[j]);
+      if (warp == 7) {
+        const float4 one = make_float4(1, 1, 1, 1), dd = ld4(&S.d[s]);
+        gb1 = dot4(a, one, gb1);
+        gb2 = dot4(c, one, gb2);
+        g3 = dot4(dd, ld4(&S.h2[lane * kSS + s]), g3);
+        if (lane < 2) gs = dot4(lane == 0 ? dd : ld4(&S.loss[s]), one, gs);
+      }
+    }
   }
-  if (threadIdx.x == 0) {
-    float l = 0.0f;
-    for (int s = 0; s < kBB; ++s) l += sl[s];
-    if (part) part[(long long)blockIdx.x * (kParams + 1) + kParams] = l;
-    else atomicAdd(loss, l);
+  float *row = part ? part + (long long)blockIdx.x * (kParams + 1) : nullptr;
+  auto emit = [&](int e, float v) {
+    if (row) row[e] = v;
+    else atomicAdd(e < kParams ? &grad[e] : loss, v);
+  };
+#pragma unroll
+  for (int j = 0; j < 7; ++j)
+    if (j < kn) emit(oW1 + lane * kIn + k0 + j, g1[j]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) emit(oW2 + lane * kHid + 4 * warp + j, g2[j]);
+  if (warp == 7) {
+    emit(oB1 + lane, gb1);
+    emit(oB2 + lane, gb2);
+    emit(oW3 + lane, g3);
+    if (lane == 0) emit(oB3, gs);
+    if (lane == 1) emit(kParams, gs);
   }
 }
 
-// The blocks' partial gradients (and loss shares) summed in block order:
-// the training loop's gradient does not depend on the order in which the
-// blocks finished, so a training run is repeatable bit for bit.
-__global__ void k_grad_reduce(const float *part, int blocks, float *grad, float *loss) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > kParams) return;
-  float acc = 0.0f;
-  for (int b = 0; b < blocks; ++b) acc += part[(long long)b * (kParams + 1) + e];
-  if (e < kParams) grad[e] = acc;
-  else *loss = acc;
-}
-
-__global__ void k_adam(float *P, const float *G, float *M, float *V, int step, float lr) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kParams) return;
+__device__ __forceinline__ void adam_update(float *P, float g, float *M, float *V, int k, int step, float lr) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float g = G[k];
   const float m = b1 * M[k] + (1.0f - b1) * g;
   const float v = b2 * V[k] + (1.0f - b2) * g * g;
   M[k] = m;
@@ -164,6 +231,34 @@ __global__ void k_adam(float *P, const float *G, float *M, float *V, int step, f
   const float mh = m / (1.0f - powf(b1, float(step)));
   const float vh = v / (1.0f - powf(b2, float(step)));
   P[k] -= lr * mh / (sqrtf(vh) + eps);
+}
+
+__global__ void k_adam(float *P, const float *G, float *M, float *V, int step, float lr) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < kParams) adam_update(P, G[k], M, V, k, step, lr);
+}
+
+// The training loop's step: the blocks' partial gradients (and loss shares)
+// summed in a fixed order -- four quarters of the rows, each in row order --
+// and Adam on the sums.  The gradient does not depend on the order in which the
+// blocks finished, so a training run is repeatable bit for bit.
+constexpr int kStepParams = 64;  // parameters per block, four threads each
+__global__ void __launch_bounds__(4 * kStepParams)
+    k_train_step(const float *part, int blocks, float *P, float *M, float *V, int step, float lr, float *loss) {
+  __shared__ float quarter[4][kStepParams];
+  const int c = threadIdx.x % kStepParams, q = threadIdx.x / kStepParams, e = blockIdx.x * kStepParams + c;
+  const int first = int((long long)blocks * q / 4), last = int((long long)blocks * (q + 1) / 4);
+  float acc = 0.0f;
+  if (e <= kParams) {
+#pragma unroll 8
+    for (int b = first; b < last; ++b) acc += part[(long long)b * (kParams + 1) + e];
+  }
+  quarter[q][c] = acc;
+  __syncthreads();
+  if (q != 0 || e > kParams) return;
+  const float g = (quarter[0][c] + quarter[1][c]) + (quarter[2][c] + quarter[3][c]);
+  if (e < kParams) adam_update(P, g, M, V, e, step, lr);
+  else *loss = g;
 }
 
 // ------------------------------------------- tensor-core inference (tcgen05)
@@ -806,15 +901,20 @@ extern "C" int wenofd_mlp_forward(const float *dev_params, const float *dev_x, l
 
 namespace {
 
+// Blocks of a backward pass over n samples.
+int back_blocks(long long n) {
+  using namespace wenofd::lrn;
+  return int(std::min<long long>((n + kGroup - 1) / kGroup, kBackBlocks));
+}
+
 // One backward pass over n samples: with part null the blocks add their
 // gradients into grad / loss with atomics (after zeroing them); with part
-// (room for one row of kParams + 1 floats per block) they write partials and
-// k_grad_reduce sums them in block order.
+// (room for one row of kParams + 1 floats per block) they write partials.
 // (rows: the rows of x and y that idx indexes)
 int launch_backward(const float *params, const float *x, const float *y, long long n, float *grad, float *loss,
-                    float *part, cudaStream_t s, const long long *idx = nullptr, long long rows = 0) {
+                    float *part, cudaStream_t s, const unsigned *idx = nullptr, long long rows = 0) {
   using namespace wenofd::lrn;
-  const size_t smem = sizeof(float) * (kParams + kBB * kIn + 4 * kBB * kHid + 2 * kBB);
+  const size_t smem = sizeof(BackSmem);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return WENOFD_CUDA_ERROR;
   static unsigned long long configured = 0;  // one bit per device
@@ -824,13 +924,11 @@ int launch_backward(const float *params, const float *x, const float *y, long lo
       return WENOFD_CUDA_ERROR;
     configured |= bit;
   }
-  const long long blocks = (n + kBB - 1) / kBB;
   if (!part && (cudaMemsetAsync(grad, 0, kParams * sizeof(float), s) != cudaSuccess ||
                 cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess))
     return WENOFD_CUDA_ERROR;
-  k_mlp_backward<<<int(blocks), kBB, smem, s>>>(params, x, y, n, 1.0f / float(n), grad, loss, part, idx,
-                                                idx ? rows : n, wenofd::guard_record());
-  if (part) k_grad_reduce<<<(kParams + 1 + 255) / 256, 256, 0, s>>>(part, int(blocks), grad, loss);
+  k_mlp_backward<<<back_blocks(n), kBackThreads, smem, s>>>(params, x, y, n, 1.0f / float(n), grad, loss, part, idx,
+                                                            idx ? rows : n, wenofd::guard_record());
   return cudaGetLastError() == cudaSuccess ? WENOFD_OK : WENOFD_CUDA_ERROR;
 }
 
@@ -852,33 +950,33 @@ extern "C" int wenofd_mlp_adam(float *dev_params, const float *dev_grad, float *
 
 // Training loop: per epoch a seeded permutation of the samples (so the data
 // may come in any order, e.g. grouped by snapshot and node), cut into
-// mini-batches, and per mini-batch one backward pass and one Adam step.  The
-// epoch's mean loss is estimated from every 16th mini-batch's loss.  Each
-// mini-batch's gradient is summed in block order (k_grad_reduce), so the same
-// data and seed give the same parameters bit for bit.
+// mini-batches, and per mini-batch one backward pass and one launch that sums
+// its gradient in block order and takes the Adam step (k_train_step), so the
+// same data and seed give the same parameters bit for bit.  The epoch's mean
+// loss is estimated from every 16th mini-batch's loss (and the last).
+// 131,072 samples in mini-batches of 4,096, one epoch: 4.06 ms with 32 blocks a
+// mini-batch, a reduction, an Adam launch and a loss read-back each.
+// Now 1.67 ms, the larger part of it the shuffle on the host.
 extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const float *dev_y, long long n, int epochs,
                                 int batch, float lr, unsigned long long seed, float *host_epoch_loss, void *stream) {
   WENOFD_TRACE("wenofd_mlp_train");
   using namespace wenofd::lrn;
   if (!dev_params || !dev_x || !dev_y || n <= 0 || epochs < 1 || batch < 1) return WENOFD_BAD_ARG;
+  if (n > 0xffffffffLL) return WENOFD_BAD_ARG;  // 32-bit row indices (as many rows take 860 GB)
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // grad | m | v | loss | epoch loss | the backward blocks' partial rows
-  const long long part_rows = (std::min<long long>(batch, n) + kBB - 1) / kBB;
+  const long long nb = (n + batch - 1) / batch;
+  // m | v | the mini-batches' losses | the backward blocks' partial rows | permutation
+  const size_t part_floats = size_t(back_blocks(std::min<long long>(batch, n))) * (kParams + 1);
   float *buf = nullptr;
-  long long *perm_dev = nullptr;
-  if (cudaMalloc(&buf, sizeof(float) * (3 * kParams + 2 + part_rows * (kParams + 1))) != cudaSuccess)
+  if (cudaMalloc(&buf, sizeof(float) * (2 * kParams + size_t(nb) + part_floats + size_t(n))) != cudaSuccess)
     return WENOFD_CUDA_ERROR;
-  if (cudaMalloc(&perm_dev, sizeof(long long) * size_t(n)) != cudaSuccess) {
-    cudaFree(buf);
-    return WENOFD_CUDA_ERROR;
-  }
-  float *grad = buf, *m = buf + kParams, *v = buf + 2 * kParams, *loss = buf + 3 * kParams;
-  float *part = buf + 3 * kParams + 2;
+  float *m = buf, *v = m + kParams, *losses = v + kParams, *part = losses + nb;
+  unsigned *perm_dev = reinterpret_cast<unsigned *>(part + part_floats);
   int rc = WENOFD_OK;
   if (cudaMemsetAsync(m, 0, sizeof(float) * 2 * kParams, s) != cudaSuccess) rc = WENOFD_CUDA_ERROR;
-  const long long nb = (n + batch - 1) / batch;
-  std::vector<long long> perm(n);
-  for (long long r = 0; r < n; ++r) perm[r] = r;
+  std::vector<unsigned> perm(static_cast<size_t>(n));
+  std::vector<float> host_losses(host_epoch_loss ? size_t(nb) : 0);
+  for (long long r = 0; r < n; ++r) perm[r] = unsigned(r);
   unsigned long long st = seed ? seed : 0x9E3779B97F4A7C15ULL;
   int step = 0;
   for (int e = 0; e < epochs && rc == WENOFD_OK; ++e) {
@@ -892,30 +990,36 @@ extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const flo
     // the previous epoch's mini-batches read the permutation buffer: copy
     // after they ran (same stream; the copy from pageable memory returns
     // once the host buffer is staged)
-    if (cudaMemcpyAsync(perm_dev, perm.data(), sizeof(long long) * size_t(n), cudaMemcpyHostToDevice, s) !=
+    if (cudaMemcpyAsync(perm_dev, perm.data(), sizeof(unsigned) * size_t(n), cudaMemcpyHostToDevice, s) !=
         cudaSuccess)
       rc = WENOFD_CUDA_ERROR;
-    // the loss of every 16th mini-batch (and the last) estimates the epoch's mean
-    double epoch_loss = 0.0;
-    int sampled = 0;
     for (long long k = 0; k < nb && rc == WENOFD_OK; ++k) {
       const long long off = k * batch;
       const long long cnt = off + batch <= n ? batch : n - off;
-      rc = launch_backward(dev_params, dev_x, dev_y, cnt, grad, loss, part, s, perm_dev + off, n);
-      if (rc == WENOFD_OK) rc = wenofd_mlp_adam(dev_params, grad, m, v, ++step, lr, stream);
-      if (rc == WENOFD_OK && host_epoch_loss && (k == nb - 1 || k % 16 == 0)) {
-        float l = 0.0f;
-        if (cudaMemcpyAsync(&l, loss, sizeof(float), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-          rc = WENOFD_CUDA_ERROR;
-        epoch_loss += l;
-        ++sampled;
-      }
+      rc = launch_backward(dev_params, dev_x, dev_y, cnt, nullptr, nullptr, part, s, perm_dev + off, n);
+      if (rc != WENOFD_OK) break;
+      k_train_step<<<(kParams + kStepParams) / kStepParams, 4 * kStepParams, 0, s>>>(part, back_blocks(cnt), dev_params, m, v,
+                                                                                    ++step, lr, losses + k);
+      if (cudaGetLastError() != cudaSuccess) rc = WENOFD_CUDA_ERROR;
     }
-    if (host_epoch_loss && sampled) host_epoch_loss[e] = float(epoch_loss / sampled);
+    if (rc == WENOFD_OK && host_epoch_loss) {
+      if (cudaMemcpyAsync(host_losses.data(), losses, sizeof(float) * size_t(nb), cudaMemcpyDeviceToHost, s) !=
+              cudaSuccess ||
+          cudaStreamSynchronize(s) != cudaSuccess) {
+        rc = WENOFD_CUDA_ERROR;
+        break;
+      }
+      double epoch_loss = 0.0;
+      int sampled = 0;
+      for (long long k = 0; k < nb; ++k)
+        if (k == nb - 1 || k % 16 == 0) {
+          epoch_loss += host_losses[k];
+          ++sampled;
+        }
+      host_epoch_loss[e] = float(epoch_loss / sampled);
+    }
   }
   if (cudaStreamSynchronize(s) != cudaSuccess) rc = WENOFD_CUDA_ERROR;
   cudaFree(buf);
-  cudaFree(perm_dev);
   return rc;
 }
