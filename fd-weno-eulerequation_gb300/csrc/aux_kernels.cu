@@ -101,7 +101,11 @@ __global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
 // Pass 2: the exact FP64 s of every node with s32 + e >= L (the node holding
 // the maximum is one of them), max-reduced as in k_dt_reduce.  With valid
 // per-tile bounds (the last stage of the previous step screened the nodes it
-// wrote) a warp per tile skips the tiles whose upper bound stays below L.
+// wrote) a block takes the tiles blockIdx, blockIdx + gridDim, ..., reads their
+// bounds together, skips those whose upper bound stays below L and spreads the
+// others' nodes over its threads: in a Riemann problem's uniform quadrants most
+// tiles remain, and a warp per tile (15 nodes a lane, one FP64 evaluation after
+// the other) took 37 us at 257 x 193 where this takes 7.
 __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *bounds, int tile_i) {
   if (!c->active) return;
   const float L = __uint_as_float(c->screen_bits);
@@ -121,15 +125,23 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
   };
   if (bounds && c->bounds_valid) {
     const int tiles_j = (g.ny + 31) / 32, ntiles = ((g.nx + tile_i - 1) / tile_i) * tiles_j;
-    const int lane = threadIdx.x & 31;
-    const int warps = int(gridDim.x * blockDim.x) >> 5;
-    for (int t = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps) {
+    __shared__ int kept[256], nkept;
+    for (int first = blockIdx.x; first < ntiles; first += int(gridDim.x) * int(blockDim.x)) {
+      if (threadIdx.x == 0) nkept = 0;
+      __syncthreads();
+      const long long t = first + (long long)threadIdx.x * gridDim.x;
       // (bounds are allocated for tiles of 15 rows, the most tiles)
-      if (bounds[WENOFD_IX(g.guard, t, ((g.nx + 14) / 15) * tiles_j)].y < L) continue;  // warp-uniform
-      const int i0 = (t / tiles_j) * tile_i, j = (t - (t / tiles_j) * tiles_j) * 32 + lane;
-      const int i1 = i0 + tile_i < g.nx ? i0 + tile_i : g.nx;
-      if (j < g.ny)
-        for (int i = i0; i < i1; ++i) visit(i, j);
+      if (t < ntiles && !(bounds[WENOFD_IX(g.guard, t, ((g.nx + 14) / 15) * tiles_j)].y < L))
+        kept[WENOFD_IX(g.guard, atomicAdd(&nkept, 1), 256)] = int(t);
+      __syncthreads();
+      const int count = nkept;
+      for (int k = 0; k < count; ++k) {
+        const int i0 = (kept[k] / tiles_j) * tile_i, j = (kept[k] % tiles_j) * 32 + int(threadIdx.x & 31);
+        const int i1 = i0 + tile_i < g.nx ? i0 + tile_i : g.nx;
+        if (j < g.ny)
+          for (int i = i0 + int(threadIdx.x >> 5); i < i1; i += int(blockDim.x >> 5)) visit(i, j);
+      }
+      __syncthreads();
     }
   } else {
     const long long n = (long long)g.nx * g.ny;
