@@ -89,10 +89,13 @@ struct Nothing {
   __device__ void operator()() const {}
 };
 
-// Hand out the items [0, prefix[n]) of one phase to the blocks.  Thread 0
-// claims an item from the phase's counter, finds its member and reads the
-// member's `active` flag; the claim of the next item is issued before the
-// current item runs, so its latency overlaps the work.  f(local item, member)
+// Hand out the items [0, prefix[n]) of one phase to the blocks.  A block's
+// first item is its own number; the others thread 0 claims from the phase's
+// counter, finds their member and reads the member's `active` flag; the claim
+// of the next item is issued before the current item runs, so its latency
+// overlaps the work.  (With the first items claimed too, the blocks that left
+// the barrier first took two each: a phase of 281 tiles on 304 blocks ran two
+// tiles one after the other.)  f(local item, member)
 // runs with the whole block for items of active members, with the member's
 // record staged in shared memory (sM).
 template <typename F>
@@ -108,7 +111,8 @@ __device__ __forceinline__ void for_member_items(const BatchArgs &b, unsigned *c
       s_on[slot] = __ldcg(&b.members[m].ctrl->active);
     }
   };
-  if (threadIdx.x == 0) resolve(0, int(atomicAdd(counter, 1u)));
+  const int blocks = int(gridDim.x);
+  if (threadIdx.x == 0) resolve(0, int(blockIdx.x));
   __syncthreads();
   int cur = -1;
   for (int it = 0;; ++it) {
@@ -118,7 +122,7 @@ __device__ __forceinline__ void for_member_items(const BatchArgs &b, unsigned *c
     const int m = s_m[slot];
     const bool on = s_on[slot] != 0;
     int next = 0;
-    if (threadIdx.x == 0) next = int(atomicAdd(counter, 1u));
+    if (threadIdx.x == 0) next = blocks + int(atomicAdd(counter, 1u));
     if (on) {
       if (m != cur) {  // block-uniform: stage the member record
         const unsigned *src = reinterpret_cast<const unsigned *>(&b.members[m]);
@@ -138,11 +142,13 @@ __device__ __forceinline__ int runnable(const Ctrl *c) {
   return (!__ldcg(&c->done) && !__ldcg(&c->error) && __ldcg(&c->steps) < __ldcg(&c->max_steps)) ? 1 : 0;
 }
 
+// Resident blocks: FP64 two (stage_blocks_per_sm), FP32 three, the learned form
+// four (80 bytes of spills; 1.44 -> 1.40 ms per step of 32 shear layers).
 // ROUTE (FP32 only): the learned form; each member's stage tiles route
 // their faces with the member's flags (BatchMember::flags), which the
 // batched indicator launch between two launches of this kernel writes.
 template <typename T, int SCHEME, int TI, int NT, bool WITHHOLD = false, bool ROUTE = false>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? 3 : 1) : 2) k_batch(BatchArgs b) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 : 3) : (ROUTE ? 2 : 1)) : 2) k_batch(BatchArgs b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BatchMember sM;
   constexpr int TJ = 32;
