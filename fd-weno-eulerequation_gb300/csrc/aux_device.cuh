@@ -115,6 +115,90 @@ __device__ __forceinline__ void bc_fill_entry(const Geom &g, double *U, const do
   }
 }
 
+// The ghost nodes whose value interior node (i, j) determines (bc_fill_entry's
+// rules the other way round: its images across x, across y and in the corners).
+// SPECIAL ghosts are constants and stay as filled.
+__device__ __forceinline__ void store_images(const Geom &g, double *U, int i, int j) {
+  auto ghost = [](int k) { return unsigned(k - 1) < unsigned(kGhost); };
+  // image across the low (side 0) and the high edge: the node's distance k from
+  // the edge that the rule reads, ghost node k of that side
+  const int xl = g.bc_left == kPeriod ? g.nx - 1 - i : i, xr = g.bc_right == kPeriod ? i : g.nx - 1 - i;
+  const int yl = g.bc_y == kPeriod ? g.ny - 1 - j : j, yr = g.bc_y == kPeriod ? j : g.ny - 1 - j;
+  const bool hx[2] = {g.bc_left != kSpecial && ghost(xl), g.bc_right != kSpecial && ghost(xr)};
+  const bool hy[2] = {g.bc_y != kSpecial && ghost(yl), g.bc_y != kSpecial && ghost(yr)};
+  if (!(hx[0] || hx[1] || hy[0] || hy[1])) return;
+  const int ei[2] = {kGhost - xl, kGhost + g.nx - 1 + xr}, ej[2] = {kGhost - yl, kGhost + g.ny - 1 + yr};
+  const bool sx[2] = {g.bc_left == kSlip, g.bc_right == kSlip}, sy = g.bc_y == kSlip;
+  double w[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) w[r] = __ldcg(&U[at(g, r, kGhost + i, kGhost + j)]);
+  auto put = [&](int di, int dj, bool x, bool y) {
+    U[at(g, 0, di, dj)] = w[0];
+    U[at(g, 1, di, dj)] = x ? -w[1] : w[1];
+    U[at(g, 2, di, dj)] = y ? -w[2] : w[2];
+    U[at(g, 3, di, dj)] = w[3];
+  };
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    if (hx[a]) put(ei[a], kGhost + j, sx[a], false);
+    if (hy[a]) put(kGhost + i, ej[a], false, sy);
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      if (hx[a] && hy[b]) put(ei[a], ej[b], sx[a], sy);
+}
+
+// End of a stage tile in the time loop (all NT threads): the ghosts that the
+// tile's nodes determine, so that the loop needs no boundary launch per stage.
+// Read back from the nodes just stored, in the tiles at the grid's edge only:
+// done at each node's store it cost the grids of many tiles 4 to 12 % (a call and
+// the grid's description on the stack of every thread).
+template <int TI, int TJ, int NT>
+__device__ __forceinline__ void store_tile_ghosts(const Geom &g, const StageArgs &a, int i0, int j0) {
+  if (!a.ghosts || (i0 > kGhost && j0 > kGhost && i0 + TI + kGhost < g.nx && j0 + TJ + kGhost < g.ny)) return;
+  __syncthreads();  // the tile's nodes are stored
+  for (int t = threadIdx.x; t < TI * TJ; t += NT) {
+    const int i = i0 + t / TJ, j = j0 + t % TJ;
+    if (i < g.nx && j < g.ny) store_images(g, a.uout, i, j);
+  }
+}
+
+// Whether the next graph-driven step runs: while |now - t_end| > 1e-9 (the loop
+// condition of src/WENOFD.cpp:213), no error, and under the step cap.
+__device__ __forceinline__ void gate_step(Ctrl *c) {
+  c->active = (!c->done && !c->error && c->steps < c->max_steps) ? 1 : 0;
+}
+
+// m_now += dt; count++ (src/WENOFD.cpp:238-239), then the loop condition.
+// fused: the step's last stage wrote the screen bounds of the new U^n.
+__device__ __forceinline__ void end_step(Ctrl *c, int fused) {
+  c->now += c->dt;
+  c->steps += 1;
+  c->done = !(fabs(c->now - c->t_end) > 1e-9);
+  c->bounds_valid = fused;
+}
+
+// True in the thread whose arrival is the launch's last; one thread of each
+// block calls it.
+__device__ __forceinline__ bool arrive_last(Ctrl *c) {
+  if (atomicAdd(&c->arrivals, 1u) != gridDim.x * gridDim.y - 1u) return false;
+  c->arrivals = 0u;
+  return true;
+}
+
+// In the last stage of a step: the last block to come here ends the step.  Of
+// what that writes a stage reads only the gate, so one thread of each block calls
+// it once its block has passed the gate (a barrier after it), beside the wait for
+// the tile's copy; the stage itself need not have ended.
+__device__ __forceinline__ void finish_step(const StageArgs &a) {
+  if (a.end && arrive_last(a.end)) {
+    end_step(a.end, 1);
+    gate_step(a.end);
+  }
+}
+
 // A node's s depends only on its four state values.  In uniform regions
 // (the quadrants of a Riemann problem) every node ties for the maximum and
 // the FP64 evaluation (five divisions and a square root on a pipe at 1/73 of

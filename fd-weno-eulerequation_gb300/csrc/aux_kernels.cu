@@ -22,6 +22,34 @@ __global__ void k_bc_fill(Geom g, double *U, const double *special, const int *a
     dev::bc_fill_entry(g, U, special, t);
 }
 
+// dt = min(1.0, cfl / max s), then clipped to t_end - now
+// (src/WENOFD.cpp:401, 426-435).  NaN -> error NAN_DT (the reference aborts,
+// lines 437-442).  One thread, after every block's atomics.
+__device__ __forceinline__ void dt_finalize(Ctrl *c) {
+  const double ms = __longlong_as_double((long long)__ldcg(&c->max_s_bits));
+  c->max_s_bits = 0ull;
+  c->screen_bits = 0u;
+  if (__ldcg(&c->nan_flag)) {
+    c->nan_flag = 0;
+    c->error = 3;  // WENOFD_NAN_DT
+    c->active = 0;
+    return;
+  }
+  const double cand = c->cfl / ms;
+  double timestep = 1.0;
+  if (!(cand > timestep)) timestep = cand;
+  if (c->t_end - c->now < timestep) timestep = c->t_end - c->now;
+  if (timestep != timestep) {
+    c->error = 3;
+    c->active = 0;
+    return;
+  }
+  c->dt = timestep;
+}
+__global__ void k_dt_finalize(Ctrl *c) {
+  if (c->active) dt_finalize(c);
+}
+
 // calculateDeltaT (src/WENOFD.cpp:398-452).  Per node the reference forms
 // tmp = cfl / (lx/dx + ly/dy) with lx = |u*1 + v*0| + c, ly = |u*0 + v*1| + c
 // (getMaxEigenValue(U, 1, 0) and (U, 0, 1), utils/equations.hpp:137-147) and
@@ -99,7 +127,8 @@ __global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
 }
 
 // Pass 2: the exact FP64 s of every node with s32 + e >= L (the node holding
-// the maximum is one of them), max-reduced as in k_dt_reduce.  With valid
+// the maximum is one of them), max-reduced as in k_dt_reduce; the last block to
+// finish forms dt.  With valid
 // per-tile bounds (the last stage of the previous step screened the nodes it
 // wrote) a block takes the tiles blockIdx, blockIdx + gridDim, ..., reads their
 // bounds together, skips those whose upper bound stays below L and spreads the
@@ -171,6 +200,11 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
     }
     atomicMax(&c->max_s_bits, (unsigned long long)__double_as_longlong(m));
     if (nn) atomicOr(&c->nan_flag, 1);
+    __threadfence();
+    if (dev::arrive_last(c)) {
+      __threadfence();
+      dt_finalize(c);
+    }
   }
 }
 
@@ -182,47 +216,16 @@ __global__ void k_ctrl_open(Ctrl *c) {
   c->screen_bits = 0u;
   c->nan_flag = 0;
   c->error = 0;
+  c->arrivals = 0u;
 }
 
-// Start of a graph-driven step: run while |now - t_end| > 1e-9 (the loop
-// condition of src/WENOFD.cpp:213), no error, and under the step cap.
-__global__ void k_step_begin(Ctrl *c) {
-  c->active = (!c->done && !c->error && c->steps < c->max_steps) ? 1 : 0;
-}
+// Start of a graph-driven step whose predecessor's last stage did not end it
+// (end_step).
+__global__ void k_step_begin(Ctrl *c) { dev::gate_step(c); }
 
-// dt = min(1.0, cfl / max s), then clipped to t_end - now
-// (src/WENOFD.cpp:401, 426-435).  NaN -> error NAN_DT (the reference aborts,
-// lines 437-442).
-__global__ void k_dt_finalize(Ctrl *c) {
-  if (!c->active) return;
-  const double ms = __longlong_as_double((long long)c->max_s_bits);
-  c->max_s_bits = 0ull;
-  c->screen_bits = 0u;
-  if (c->nan_flag) {
-    c->nan_flag = 0;
-    c->error = 3;  // WENOFD_NAN_DT
-    c->active = 0;
-    return;
-  }
-  const double cand = c->cfl / ms;
-  double timestep = 1.0;
-  if (!(cand > timestep)) timestep = cand;
-  if (c->t_end - c->now < timestep) timestep = c->t_end - c->now;
-  if (timestep != timestep) {
-    c->error = 3;
-    c->active = 0;
-    return;
-  }
-  c->dt = timestep;
-}
-
-// m_now += dt; count++ (src/WENOFD.cpp:238-239), then the loop condition.
-__global__ void k_step_end(Ctrl *c, int fused) {
-  if (!c->active) return;
-  c->now += c->dt;
-  c->steps += 1;
-  c->done = !(fabs(c->now - c->t_end) > 1e-9);
-  c->bounds_valid = fused;
+// The time update by itself: RK1, the FP64 form and the host-driven step.
+__global__ void k_step_end(Ctrl *c) {
+  if (c->active) dev::end_step(c, 0);
 }
 
 __global__ void k_set_dt(Ctrl *c, double dt) {
@@ -245,6 +248,8 @@ __global__ void k_advance_setup(Ctrl *c, long long max_steps) {
   c->nan_flag = 0;
   c->bounds_valid = 0;
   c->ind_base = c->steps;
+  c->arrivals = 0u;
+  dev::gate_step(c);
 }
 
 __global__ void k_copy_interior(Geom g, const double *src, double *dst, const int *active) {
@@ -426,11 +431,13 @@ cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream
   return cudaGetLastError();
 }
 
-cudaError_t launch_dt_reduce_two_pass(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i,
-                                      cudaStream_t s) {
-  const int grid = grid_for((long long)g.nx * g.ny, 256);
-  k_dt_screen<<<grid, 256, 0, s>>>(g, U, c);
-  k_dt_refine<<<grid, 256, 0, s>>>(g, U, c, bounds, tile_i > 0 ? tile_i : 15);
+cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream_t s) {
+  k_dt_screen<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, s>>>(g, U, c);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i, cudaStream_t s) {
+  k_dt_refine<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, s>>>(g, U, c, bounds, tile_i > 0 ? tile_i : 15);
   return cudaGetLastError();
 }
 
@@ -446,8 +453,8 @@ cudaError_t launch_dt_finalize(Ctrl *c, cudaStream_t s) {
   k_dt_finalize<<<1, 1, 0, s>>>(c);
   return cudaGetLastError();
 }
-cudaError_t launch_step_end(Ctrl *c, int fused, cudaStream_t s) {
-  k_step_end<<<1, 1, 0, s>>>(c, fused);
+cudaError_t launch_step_end(Ctrl *c, cudaStream_t s) {
+  k_step_end<<<1, 1, 0, s>>>(c);
   return cudaGetLastError();
 }
 cudaError_t launch_set_dt(Ctrl *c, double dt, cudaStream_t s) {

@@ -117,11 +117,15 @@ int sync(wenofd_solver *s) {
   return WENOFD_OK;
 }
 
-// bounds: this stage writes U^{n+1} at the end of a graph-driven step; its
-// epilogue also screens the next time step (FP32 forms).
-// timeloop: launched by the graph-driven step of wenofd_advance.
+// Whether the graph-driven steps of wenofd_advance run on the stages' own
+// epilogues (prepare_loop): the FP32 forms with SSP-RK2 or RK3.  RK1's stage does
+// not write U^n itself.  The FP64 form keeps a launch for each part of a step.
+bool fused_loop(const wenofd_solver *s) { return s->precision != WENOFD_FP64 && s->rk != 0; }
+
+// loop: launched by the graph-driven step of wenofd_advance; last: the step's
+// last stage, which in a fused loop screens the next time step and ends the step.
 int launch_stage(wenofd_solver *s, const double *in, const double *un, double *out, double a, double b,
-                 double c, int mode, bool bounds = false, bool timeloop = false) {
+                 double c, int mode, bool loop = false, bool last = false) {
   StageArgs args;
   args.uin = in;
   args.un = un;
@@ -134,18 +138,24 @@ int launch_stage(wenofd_solver *s, const double *in, const double *un, double *o
   args.mode = mode;
   args.form = wenofd::rk_form(a, b, c, in, un);
   args.flags = s->precision == WENOFD_LEARNED ? s->flags : nullptr;
-  if (bounds && s->tile_bounds) {
+  const bool fills = loop && fused_loop(s);
+  args.ghosts = fills ? 1 : 0;
+  if (fills && last) {
     args.bounds = s->tile_bounds;
     args.screen = &s->ctrl->screen_bits;
+    args.end = s->ctrl;
   }
-  CUDA_TRY(wenofd::launch_bc_fill(s->g, const_cast<double *>(in), s->special, &s->ctrl->active, s->stream));
-  s->launches += 2;
+  if (!fills) {
+    CUDA_TRY(wenofd::launch_bc_fill(s->g, const_cast<double *>(in), s->special, &s->ctrl->active, s->stream));
+    s->launches += 1;
+  }
+  s->launches += 1;
   // The learned form classifies the nodes once per step, on the stage-1
   // input (ghosts just filled); all stages of the step route with those flags.
   if (s->precision == WENOFD_LEARNED && in == s->S && un == s->S && s->ind_ready) {
     CUDA_TRY(wenofd::launch_indicator(s->g, in, s->ind_weights, s->ind_logit_threshold, s->ind_guard, s->flags,
                                       s->wait_error,
-                                      &s->ctrl->active, timeloop ? s->ctrl : nullptr, s->ind_interval,
+                                      &s->ctrl->active, loop ? s->ctrl : nullptr, s->ind_interval,
                                       s->stream));
     s->launches += 1;
   }
@@ -162,50 +172,74 @@ int launch_stage(wenofd_solver *s, const double *in, const double *un, double *o
 // RunRK1/2/3 (src/WENOFD.cpp:301-396), dt from the control block.  Stage k
 // reads its input with a halo and writes a different buffer; the last stage
 // writes U^{n+1} over U^n, which it reads only at the node itself.
-// fused: the last stage also screens the next time step (RK2, RK3).
-int enqueue_rk(wenofd_solver *s, bool fused = false, bool timeloop = false) {
+// loop: launch_stage's.
+int enqueue_rk(wenofd_solver *s, bool loop = false) {
   int rc;
   double *S = s->S, *A = s->A, *B = s->B;
   switch (s->rk) {
     case 0:  // U += dt * rhs, as (1*U + 0*U) + (1*dt)*rhs (same rounding)
-      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, false, timeloop))) return rc;
+      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, loop))) return rc;
       CUDA_TRY(wenofd::launch_copy_interior(s->g, A, S, &s->ctrl->active, s->stream));
       s->launches += 1;
       return WENOFD_OK;
     case 1:
-      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, false, timeloop))) return rc;
-      return launch_stage(s, A, S, S, 0.5, 0.5, 0.5, wenofd::kModeRK, fused);
+      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, loop))) return rc;
+      return launch_stage(s, A, S, S, 0.5, 0.5, 0.5, wenofd::kModeRK, loop, true);
     case 2:
-      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, false, timeloop))) return rc;
-      if ((rc = launch_stage(s, A, S, B, 3.0 / 4.0, 1.0 / 4.0, 1.0 / 4.0, wenofd::kModeRK))) return rc;
-      return launch_stage(s, B, S, S, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, wenofd::kModeRK, fused);
+      if ((rc = launch_stage(s, S, S, A, 1.0, 0.0, 1.0, wenofd::kModeRK, loop))) return rc;
+      if ((rc = launch_stage(s, A, S, B, 3.0 / 4.0, 1.0 / 4.0, 1.0 / 4.0, wenofd::kModeRK, loop))) return rc;
+      return launch_stage(s, B, S, S, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, wenofd::kModeRK, loop, true);
   }
   return fail(WENOFD_BAD_CONFIG, "Error: Invalid Runge-Kutta method");
 }
 
-// The time-step reduction: FP64 form one FP64 pass; FP32 forms the two-pass
-// reduction (same result bit for bit, FP32 screen + FP64 refine).
-int enqueue_dt_reduce(wenofd_solver *s) {
+// The time-step reduction and dt: FP64 form one FP64 pass; FP32 forms the
+// two-pass reduction (same result bit for bit, FP32 screen + FP64 refine).
+// screened: the pass over every node has run (prepare_loop, or the last stage of
+// the step before).
+int enqueue_dt(wenofd_solver *s, bool screened = false) {
   if (s->precision == WENOFD_FP64) {
     CUDA_TRY(wenofd::launch_dt_reduce(s->g, s->S, s->ctrl, s->stream));
-    s->launches += 1;
-  } else {
-    CUDA_TRY(wenofd::launch_dt_reduce_two_pass(s->g, s->S, s->ctrl, s->tile_bounds, s->stage_rows, s->stream));
+    CUDA_TRY(wenofd::launch_dt_finalize(s->ctrl, s->stream));
     s->launches += 2;
+    return WENOFD_OK;
   }
+  if (!screened) {
+    CUDA_TRY(wenofd::launch_dt_screen(s->g, s->S, s->ctrl, s->stream));
+    s->launches += 1;
+  }
+  CUDA_TRY(wenofd::launch_dt_refine(s->g, s->S, s->ctrl, s->tile_bounds, s->stage_rows, s->stream));
+  s->launches += 1;
   return WENOFD_OK;
 }
 
-// One graph-driven step: gate, dt reduction, dt, stages, time update.
+// Before the steps of a fused loop: the ghosts of U^n, the SPECIAL ghosts of the
+// stage buffers (constants that no stage writes) and the screen of U^n.  From
+// here on the stages' epilogues keep both up: a step is the refinement (which
+// forms dt), its stages and, in the learned form, the indicator: 4 or 5 launches
+// where a gate, a screen, a dt, an end and a ghost fill per stage made 11 or 12.
+int prepare_loop(wenofd_solver *s) {
+  if (!fused_loop(s)) return WENOFD_OK;
+  for (double *buf : {s->S, s->A, s->B})
+    CUDA_TRY(wenofd::launch_bc_fill(s->g, buf, s->special, &s->ctrl->active, s->stream));
+  CUDA_TRY(wenofd::launch_dt_screen(s->g, s->S, s->ctrl, s->stream));
+  s->launches += 4;
+  return WENOFD_OK;
+}
+
+// One graph-driven step: gate, dt, stages, time update.
 int enqueue_step(wenofd_solver *s) {
-  CUDA_TRY(wenofd::launch_step_begin(s->ctrl, s->stream));
-  if (int rc = enqueue_dt_reduce(s)) return rc;
-  CUDA_TRY(wenofd::launch_dt_finalize(s->ctrl, s->stream));
-  const bool fused = s->tile_bounds && s->rk != 0;
-  int rc = enqueue_rk(s, fused, true);
-  if (rc) return rc;
-  CUDA_TRY(wenofd::launch_step_end(s->ctrl, fused ? 1 : 0, s->stream));
-  s->launches += 3;
+  const bool fused = fused_loop(s);
+  if (!fused) {
+    CUDA_TRY(wenofd::launch_step_begin(s->ctrl, s->stream));
+    s->launches += 1;
+  }
+  if (int rc = enqueue_dt(s, fused)) return rc;
+  if (int rc = enqueue_rk(s, true)) return rc;
+  if (!fused) {
+    CUDA_TRY(wenofd::launch_step_end(s->ctrl, s->stream));
+    s->launches += 1;
+  }
   return WENOFD_OK;
 }
 
@@ -617,9 +651,8 @@ int wenofd_calc_dt(wenofd_solver *s, double *dt) {
   if (!dt) return fail(WENOFD_BAD_ARG, "null dt");
   CUDA_TRY(cudaSetDevice(s->device));
   CUDA_TRY(wenofd::launch_ctrl_open(s->ctrl, s->stream));
-  if (int rc = enqueue_dt_reduce(s)) return rc;
-  CUDA_TRY(wenofd::launch_dt_finalize(s->ctrl, s->stream));
-  s->launches += 2;
+  if (int rc = enqueue_dt(s)) return rc;
+  s->launches += 1;
   if (int rc = read_ctrl(s)) return rc;
   if (s->ctrl_host->error) return fail(WENOFD_NAN_DT, "Error: Timestep is not a number...");
   *dt = s->ctrl_host->dt;
@@ -641,11 +674,10 @@ int wenofd_step(wenofd_solver *s, double *dt_out) {
   if (int rc = check_handle(s)) return rc;
   CUDA_TRY(cudaSetDevice(s->device));
   CUDA_TRY(wenofd::launch_ctrl_open(s->ctrl, s->stream));
-  if (int rc = enqueue_dt_reduce(s)) return rc;
-  CUDA_TRY(wenofd::launch_dt_finalize(s->ctrl, s->stream));
+  if (int rc = enqueue_dt(s)) return rc;
   if (int rc = enqueue_rk(s)) return rc;
-  CUDA_TRY(wenofd::launch_step_end(s->ctrl, 0, s->stream));
-  s->launches += 3;
+  CUDA_TRY(wenofd::launch_step_end(s->ctrl, s->stream));
+  s->launches += 2;
   if (int rc = read_ctrl(s)) return rc;
   if (int rc = check_wait(s)) return rc;
   if (s->ctrl_host->error) return fail(WENOFD_NAN_DT, "Error: Timestep is not a number...");
@@ -715,6 +747,7 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
   }
   CUDA_TRY(wenofd::launch_advance_setup(s->ctrl, max_steps, s->stream));
   s->launches += 1;
+  if (int rc = prepare_loop(s)) return rc;
   // Steps this call may still take (-1: no cap).  A chunk past the cap runs
   // gated-off launches that return at once; when fewer steps than a chunk
   // remain, one-step graphs are replayed instead.

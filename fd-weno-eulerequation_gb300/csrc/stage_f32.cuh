@@ -228,6 +228,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
       if constexpr (ROUTE)
         if (WENOFD_REQUIRE(g.guard, (j0 & 15) == 0, j0, 16))
           tma_load_2d(tma_smem_addr(sflag), &tma->flags, j0, 2 + i0, bar);
+      finish_step(a);
     }
   }
 
@@ -552,6 +553,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
     }
   }
   if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, tile);  // block-uniform
+  if constexpr (TMA) store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
 }
 
 }  // namespace dev

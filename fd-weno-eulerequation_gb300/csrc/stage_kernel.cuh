@@ -283,13 +283,14 @@ __global__ void __launch_bounds__(NT, stage_blocks_per_sm<T, ROUTE, NT>())
   if (*a.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // first interior node of the tile (0-based)
-  if constexpr (sizeof(T) == 4)
+  if constexpr (sizeof(T) == 4) {
     stage_tile_f32<SCHEME, TI, TJ, NT, ROUTE, false, stage_keeps_inputs<T, ROUTE, NT>(), true>(
         g, a, int(blockIdx.y) * TI, int(blockIdx.x) * TJ, smem_raw, int(blockIdx.y * gridDim.x + blockIdx.x),
         &tma);
-  else
+  } else {
     stage_tile_f64<SCHEME, TI, TJ, NT, false, true>(g, a, int(blockIdx.y) * a.rows, int(blockIdx.x) * TJ, a.rows,
                                                     a.pair != 0, smem_raw, &tma);
+  }
 }
 
 // Dynamic shared memory of one stage tile.

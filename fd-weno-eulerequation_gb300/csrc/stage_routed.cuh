@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
     }
   }
   __syncthreads();  // the barrier is initialised
+  if (threadIdx.x == 0) finish_step(a);
   const bool landed = tma_bar_wait(tma_smem_addr(&tma_bar), 0, kTmaWaitLimit);
   if (__syncthreads_or(!landed)) {
     if (threadIdx.x == 0) {
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
     }
   }
   if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, int(blockIdx.y * gridDim.x + blockIdx.x));
+  store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
 }
 
 }  // namespace dev

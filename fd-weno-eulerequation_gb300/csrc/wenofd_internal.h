@@ -55,6 +55,10 @@ struct Ctrl {
   // Learned form: steps counted from here (set at the start of every
   // advance) decide which steps run the indicator (INDICATOR_INTERVAL).
   long long ind_base;
+  // Blocks of the running launch that have come to its arrival: the last one of
+  // a time-step refinement forms dt, the last one of a step's last stage ends
+  // the step.
+  unsigned arrivals;
 };
 
 // Arguments of one RK stage launch.  uin is read with a 3-node halo (its
@@ -81,6 +85,12 @@ struct StageArgs {
   // on this integer instead of comparing the FP64 coefficients on the
   // device, where every FP64 compare issues on the 1/64-rate FP64 pipe.
   int form = 0;
+  // FP32 per-solve kernels in the time loop: the tile also writes the ghost
+  // nodes whose values its nodes determine (store_tile_ghosts).
+  int ghosts = 0;
+  // Last stage of a step in the time loop: its last block to start ends the
+  // step (finish_step).
+  Ctrl *end = nullptr;
   // FP64 per-solve kernel: how its tiles are split (Fp64Split, set by the launcher)
   int rows = 0, pair = 0;
   // FP32 per-solve tiles: set to 1 if a tile's TMA load wait gave up
@@ -280,18 +290,17 @@ constexpr int kIndBandTiles = 16;
 cudaError_t launch_bc_fill(const Geom &g, double *U, const double *special, const int *active, cudaStream_t s);
 cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream_t s);
 // Same result, bit for bit, in two passes that keep the FP64 pipe nearly
-// idle: an FP32 screen with a rigorous error bound, then FP64 only where a
-// node can hold the maximum.
+// idle: an FP32 screen with a rigorous error bound (launch_dt_screen), then FP64
+// only where a node can hold the maximum, and dt (launch_dt_refine).
 // With bounds (per-tile screen bounds of stage tiles `tile_i` x 32) and
 // Ctrl::bounds_valid set, the screen pass is skipped and the refine pass
 // visits only the tiles whose upper bound reaches the maximum lower bound.
-cudaError_t launch_dt_reduce_two_pass(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i,
-                                      cudaStream_t s);
+cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream_t s);
+cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i, cudaStream_t s);
 cudaError_t launch_ctrl_open(Ctrl *c, cudaStream_t s);
 cudaError_t launch_step_begin(Ctrl *c, cudaStream_t s);
 cudaError_t launch_dt_finalize(Ctrl *c, cudaStream_t s);
-// fused: the step's last stage wrote screen bounds of the new U^n
-cudaError_t launch_step_end(Ctrl *c, int fused, cudaStream_t s);
+cudaError_t launch_step_end(Ctrl *c, cudaStream_t s);
 cudaError_t launch_set_dt(Ctrl *c, double dt, cudaStream_t s);
 cudaError_t launch_set_time(Ctrl *c, double now, cudaStream_t s);
 cudaError_t launch_advance_setup(Ctrl *c, long long max_steps, cudaStream_t s);

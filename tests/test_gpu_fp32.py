@@ -126,6 +126,44 @@ def test_fused_screen_steps_equal_separate_steps(precision, tile_i):
     assert np.array_equal(Ua, Ub)
 
 
+@pytest.mark.parametrize("bc", [(0, 0, 0), (1, 3, 1), (3, 1, 0), (0, 0, 3), (2, 1, 3), (3, 2, 1), (0, 0, 2), (2, 2, 2),
+                                (1, 1, 2)])
+@pytest.mark.parametrize("rk", [0, 1, 2])
+@pytest.mark.parametrize("precision", [wenofd.FP32, wenofd.LEARNED])
+def test_steps_of_the_time_loop_equal_host_driven_steps(bc, rk, precision):
+    """The time loop's stages write the ghosts of their results, the last block
+    of a step's last stage ends the step and the last block of the refinement
+    forms dt; host-driven steps launch a ghost fill per stage and a kernel for
+    each of the others.  Same bits, on every boundary kind, on grids whose edge
+    nodes image to both sides, on several tiles, and on the large grids' tile;
+    a second call starts from the ghosts of the first."""
+    import mlp_oracle
+
+    sizes = [(6, 6), (7, 9), (9, 40), (33, 65)] + ([(33, 9800)] if precision == wenofd.LEARNED and rk == 2 else [])
+    for nx, ny in sizes:
+        cfg = {"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": rk, "CFL": 0.4, "SCHEME": 1, "SEED": 6,
+               "PRECISION": precision, "BC_LEFT": bc[0], "BC_RIGHT": bc[1], "BC_BOTTOM": bc[2], "BC_TOP": bc[2]}
+
+        def make():
+            s = wenofd.Solver(cfg)
+            s.initialize()
+            if precision == wenofd.LEARNED:
+                s.set_indicator(mlp_oracle.init_params(3), 0.5)
+            return s
+
+        with make() as a:
+            assert a.advance(max_steps=2) == 2
+            assert a.advance(max_steps=3) == 3
+            Ua, ta = a.get_state(), a.info().now
+        with make() as b:
+            for _ in range(5):
+                b.step()
+            Ub, tb = b.get_state(), b.info().now
+        assert ta == tb, (nx, ny)
+        assert np.array_equal(Ua, Ub, equal_nan=True), (nx, ny)
+        assert np.all(np.isfinite(Ua)), (nx, ny)
+
+
 @pytest.mark.parametrize("nx,ny", [(6, 6), (7, 9), (16, 31), (33, 65), (100, 7)])
 @pytest.mark.parametrize("tile_i", [15, 31])
 def test_tma_tiles_on_small_and_ragged_grids(nx, ny, tile_i):
