@@ -601,7 +601,8 @@ __device__ __forceinline__ bool indicator_band(const Geom &g, const double *U, f
       const float Rp = window_store(w, sA1, tid, kColP, 0.0f, 0.0f, g.guard);
       guarded = guarded || (guard > 0.0f && Rp > guard * fabsf(w[12]));
     }
-    // 3. layer 1 (bias included)
+    // 3. layer 1 (bias included); the weights have landed
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (!layer([&] { mma_layer<kK1, kHid>(tc.tmem, sA1, sm.B1); })) return false;
     // 4. GELU -> A2
     {
@@ -634,12 +635,17 @@ __device__ __forceinline__ bool indicator_band(const Geom &g, const double *U, f
   return true;
 }
 
-// Copies the packed weights into the CTA's operand buffers (all threads).
-__device__ __forceinline__ void load_weights(const IndicatorWeights *W, __nv_bfloat16 *B1, __nv_bfloat16 *B2,
-                                             __nv_bfloat16 *B3) {
-  for (int k = threadIdx.x; k < kHid * kK1; k += kCells) B1[k] = W->w1[k];
-  for (int k = threadIdx.x; k < kHid * kK2; k += kCells) B2[k] = W->w2[k];
-  for (int k = threadIdx.x; k < kN3 * kK2; k += kCells) B3[k] = W->w3[k];
+// Starts the copy of the packed weights into the CTA's operand buffers (all
+// threads), 16 bytes at a time; indicator_band waits for it before the first
+// MMA, so it runs beside the set-up and the first tile's node loads.  (Element by
+// element through registers it stood in front of both and took most of the launch
+// on small grids: 512^2, 2 tiles a CTA, 49 us against 18 now.)
+__device__ __forceinline__ void load_weights(const IndicatorWeights *W, IndicatorWeights *sW) {
+  static_assert(sizeof(IndicatorWeights) % 16 == 0, "whole 16-byte copies");
+  const char *src = reinterpret_cast<const char *>(W);
+  const unsigned dst = smem_u32(sW);
+  for (int k = threadIdx.x; k < int(sizeof(IndicatorWeights) / 16); k += kCells)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * unsigned(k)), "l"(src + 16 * k) : "memory");
 }
 
 // CTA set-up: the completion mbarrier and 64 tensor-memory columns.
@@ -679,14 +685,12 @@ __global__ void __launch_bounds__(kCells, kResident) k_indicator_tc(Geom g, cons
   if (active && *active == 0) return;
   if (ctrl && interval > 1 && (ctrl->steps - ctrl->ind_base) % interval != 0) return;
   __shared__ __align__(128) __nv_bfloat16 sA[kCells * kK1];
-  __shared__ __align__(128) __nv_bfloat16 sB1[kHid * kK1];
-  __shared__ __align__(128) __nv_bfloat16 sB2[kHid * kK2];
-  __shared__ __align__(128) __nv_bfloat16 sB3[kN3 * kK2];
+  __shared__ __align__(128) IndicatorWeights sW;
   __shared__ float sRho[kPI * kPJ], sPre[kPI * kPJ];
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ unsigned tmem_base_sh;
 
-  load_weights(W, sB1, sB2, sB3);
+  load_weights(W, &sW);
   IndTc tc = indicator_open(&mbar, &tmem_base_sh);
   // CTA b walks one band of rows down one strip (a strip = 32 columns, tiles
   // of 4 rows each): strip b % tiles_j, band b / tiles_j of the grid's
@@ -698,7 +702,7 @@ __global__ void __launch_bounds__(kCells, kResident) k_indicator_tc(Geom g, cons
   const int bands = int(gridDim.x) / tiles_j;
   const int strip = int(blockIdx.x) % tiles_j, band = int(blockIdx.x) / tiles_j;
   const int first = int((long long)tiles_i * band / bands), last = int((long long)tiles_i * (band + 1) / bands);
-  const IndSmem sm{sA, sB1, sB2, sB3, sRho, sPre};
+  const IndSmem sm{sA, sW.w1, sW.w2, sW.w3, sRho, sPre};
   indicator_band(g, U, logit_threshold, guard, flags, flag_pitch, error, strip, first, last, sm, tc);
   indicator_close(tc);
 }
@@ -714,9 +718,7 @@ __global__ void __launch_bounds__(kCells, kResident)
     k_indicator_batch(const BatchMember *members, const int *prefix, int n, unsigned *counter, int *error,
                       unsigned long long *guard) {
   __shared__ __align__(128) __nv_bfloat16 sA[kCells * kK1];
-  __shared__ __align__(128) __nv_bfloat16 sB1[kHid * kK1];
-  __shared__ __align__(128) __nv_bfloat16 sB2[kHid * kK2];
-  __shared__ __align__(128) __nv_bfloat16 sB3[kN3 * kK2];
+  __shared__ __align__(128) IndicatorWeights sW;
   __shared__ float sRho[kPI * kPJ], sPre[kPI * kPJ];
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ unsigned tmem_base_sh;
@@ -724,10 +726,10 @@ __global__ void __launch_bounds__(kCells, kResident)
   __shared__ BatchMember sM;  // the record of the member whose items run
 
   IndTc tc = indicator_open(&mbar, &tmem_base_sh);
-  const IndSmem sm{sA, sB1, sB2, sB3, sRho, sPre};
+  const IndSmem sm{sA, sW.w1, sW.w2, sW.w3, sRho, sPre};
   const int total = __ldg(&prefix[n]);
   int cur = -1;                  // member staged in sM
-  const void *loaded = nullptr;  // weights now in sB1..sB3
+  const void *loaded = nullptr;  // weights now in sW
   for (;;) {
     __syncthreads();  // every thread has read the last claim and sM
     if (threadIdx.x == 0) {
@@ -753,7 +755,7 @@ __global__ void __launch_bounds__(kCells, kResident)
       cur = m;
       if (sM.ind_weights != loaded) {
         // every MMA that read the old weights has completed (each layer waits)
-        load_weights(static_cast<const IndicatorWeights *>(sM.ind_weights), sB1, sB2, sB3);
+        load_weights(static_cast<const IndicatorWeights *>(sM.ind_weights), &sW);
         loaded = sM.ind_weights;
       }
     }
@@ -837,6 +839,9 @@ cudaError_t launch_indicator(const Geom &g, const double *U, const void *weights
   if (sms == 0 && (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   int bands = (sms * lrn::kResident) / tiles_j;
   bands = bands < 1 ? 1 : (bands > tiles_i ? tiles_i : bands);
+  // no more bands than their longest needs: 512^2 (128 tile rows, 76 bands fit)
+  // runs 64 bands of 2 tiles, not 76 of which some have 2 and some 1
+  bands = (tiles_i + (tiles_i + bands - 1) / bands - 1) / ((tiles_i + bands - 1) / bands);
   const int grid = tiles_j * bands;
   lrn::k_indicator_tc<<<grid, lrn::kCells, 0, s>>>(g, U, static_cast<const lrn::IndicatorWeights *>(weights),
                                                    logit_threshold, guard, flags, g.pitch, error, active, ctrl,
