@@ -198,9 +198,10 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
       m = wmax[w] > m ? wmax[w] : m;
       nn |= wnan[w];
     }
-    atomicMax(&c->max_s_bits, (unsigned long long)__double_as_longlong(m));
+    // (most blocks have no candidate, and the maximum starts at 0)
+    if (m > 0.0) atomicMax(&c->max_s_bits, (unsigned long long)__double_as_longlong(m));
     if (nn) atomicOr(&c->nan_flag, 1);
-    __threadfence();
+    if (m > 0.0 || nn) __threadfence();
     if (dev::arrive_last(c)) {
       __threadfence();
       dt_finalize(c);
@@ -437,7 +438,11 @@ cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream
 }
 
 cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i, cudaStream_t s) {
-  k_dt_refine<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, s>>>(g, U, c, bounds, tile_i > 0 ? tile_i : 15);
+  // a block per tile, as many as are resident at once: each more is one more
+  // arrival on the same word
+  const int rows = tile_i > 0 ? tile_i : 15;
+  const long long tiles = (long long)((g.nx + rows - 1) / rows) * ((g.ny + 31) / 32);
+  k_dt_refine<<<int(tiles < 152 * 8 ? tiles : 152 * 8), 256, 0, s>>>(g, U, c, bounds, rows);
   return cudaGetLastError();
 }
 
