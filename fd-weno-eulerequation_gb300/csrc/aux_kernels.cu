@@ -13,6 +13,7 @@ namespace {
 
 constexpr int kReduceThreads = 256;
 constexpr int kReduceBlocks = 2 * 152;  // two CTAs per SM of a GB300
+constexpr int kDtBlocks = 4;            // blocks of k_dt_reduce per SM
 
 
 __global__ void k_bc_fill(Geom g, double *U, const double *special, const int *active) {
@@ -57,27 +58,24 @@ __global__ void k_dt_finalize(Ctrl *c) {
 // min(cfl/s) == cfl/max(s): the reduction keeps max(s), as IEEE bits (all s
 // are >= 0, where bit order is value order), and k_dt_finalize divides once.
 // A NaN s sets a flag instead of entering the maximum.
-__global__ void k_dt_reduce(Geom g, const double *U, Ctrl *c) {
+// All blocks are resident, so that their first passes run together and the
+// second ones meet a bound that is nearly the maximum.
+__global__ void __launch_bounds__(256, kDtBlocks) k_dt_reduce(Geom g, const double *U, Ctrl *c) {
   if (!c->active) return;
-  const long long n = (long long)g.nx * g.ny;
-  const double gamma = g.gamma;
   double smax = 0.0;
   int nan_seen = 0;
-  dev::SpeedMemo memo;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = int(t / g.ny), j = int(t - (t / g.ny) * g.ny);
-    const long long base = WENOFD_NODE(g, i, j);
-    const double rho = U[base], mu = U[g.plane + base], mv = U[2 * g.plane + base], E = U[3 * g.plane + base];
-    if (memo.repeat(rho, mu, mv, E)) continue;
-    const double u = mu / rho, v = mv / rho;
-    const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
-    const double cs = sqrt(gamma * p / rho);
-    const double lx = fabs(u * 1.0 + v * 0.0) + cs;
-    const double ly = fabs(u * 0.0 + v * 1.0) + cs;
-    const double s = lx / g.dx + ly / g.dy;
-    if (s != s) nan_seen = 1;
-    else if (s > smax) smax = s;
-  }
+  dev::screened_max(
+      g, &c->screen_bits, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)g.nx * g.ny,
+      (long long)gridDim.x * blockDim.x,
+      [&](long long t, double &rho, double &mu, double &mv, double &E) {
+        const int i = int(t / g.ny), j = int(t - (t / g.ny) * g.ny);
+        const long long b = WENOFD_NODE(g, i, j);
+        rho = U[b], mu = U[g.plane + b], mv = U[2 * g.plane + b], E = U[3 * g.plane + b];
+      },
+      [&](double s) {
+        if (s != s) nan_seen = 1;
+        else if (s > smax) smax = s;
+      });
   for (int o = 16; o > 0; o >>= 1) {
     const double other = __shfl_xor_sync(0xffffffffu, smax, o);
     smax = other > smax ? other : smax;
@@ -134,7 +132,7 @@ __global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
 // bounds together, skips those whose upper bound stays below L and spreads the
 // others' nodes over its threads: in a Riemann problem's uniform quadrants most
 // tiles remain, and a warp per tile (15 nodes a lane, one FP64 evaluation after
-// the other) took 37 us at 257 x 193 where this takes 7.
+// the other) took 37 us at 257 x 193 where this takes 9.
 __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *bounds, int tile_i) {
   if (!c->active) return;
   const float L = __uint_as_float(c->screen_bits);
@@ -147,7 +145,7 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
     float s32, e;
     dev::screen_speed(g, rho, mu, mv, E, s32, e);
     if (s32 + e >= L && !memo.repeat(rho, mu, mv, E)) {
-      const double s = dev::exact_speed(g, rho, mu, mv, E);
+      const double s = dev::exact_speed(g.gamma, g.dx, g.dy, rho, mu, mv, E);
       if (s != s) nan_seen = 1;
       else if (s > smax) smax = s;
     }
@@ -387,6 +385,7 @@ Geom make_geom(int nx, int ny, double dx, double dy, double gamma, double zp_lam
   g.gravity = gravity;
   g.gamma32 = float(gamma);
   g.zpl32 = float(zp_lambda);
+  g.gg32 = float(gamma * (gamma - 1.0));
   g.inv_dx32 = float(1.0 / dx);
   g.inv_dy32 = float(1.0 / dy);
   g.guard = guard_record();
@@ -428,7 +427,8 @@ cudaError_t launch_bc_fill(const Geom &g, double *U, const double *special, cons
 }
 
 cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream_t s) {
-  k_dt_reduce<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, s>>>(g, U, c);
+  const long long blocks = ((long long)g.nx * g.ny + 255) / 256;
+  k_dt_reduce<<<int(blocks < 152 * kDtBlocks ? blocks : 152 * kDtBlocks), 256, 0, s>>>(g, U, c);
   return cudaGetLastError();
 }
 

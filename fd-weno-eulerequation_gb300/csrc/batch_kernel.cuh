@@ -218,23 +218,28 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
     auto exact_pass = [&](int local, const BatchMember &M) {
       const long long first = (long long)local * kPtChunk;
       const long long npts = (long long)M.g.nx * M.g.ny;
-      float L = 0.0f;
-      if constexpr (F32) L = __uint_as_float(__ldcg(&M.ctrl->screen_bits));
+      const long long end = first + kPtChunk < npts ? first + kPtChunk : npts;
       double smax = 0.0;
       int nan_seen = 0;
-      SpeedMemo memo;
-      for (long long t = first + threadIdx.x; t < first + kPtChunk && t < npts; t += NT) {
-        double rho, mu, mv, E;
-        node(M, t, rho, mu, mv, E);
-        if constexpr (F32) {  // refine: only nodes that can hold the maximum
-          float s32, e;
-          screen_speed(M.g, rho, mu, mv, E, s32, e);
-          if (!(s32 + e >= L)) continue;
-        }
-        if (memo.repeat(rho, mu, mv, E)) continue;
-        const double s = exact_speed(M.g, rho, mu, mv, E);
+      auto offer = [&](double s) {
         if (s != s) nan_seen = 1;
         else if (s > smax) smax = s;
+      };
+      if constexpr (F32) {  // refine: only nodes that can hold the maximum
+        const float L = __uint_as_float(__ldcg(&M.ctrl->screen_bits));
+        SpeedMemo memo;
+        for (long long t = first + threadIdx.x; t < end; t += NT) {
+          double rho, mu, mv, E;
+          node(M, t, rho, mu, mv, E);
+          float s32, e;
+          screen_speed(M.g, rho, mu, mv, E, s32, e);
+          if (s32 + e >= L && !memo.repeat(rho, mu, mv, E))
+            offer(exact_speed(M.g.gamma, M.g.dx, M.g.dy, rho, mu, mv, E));
+        }
+      } else {
+        screened_max(
+            M.g, &M.ctrl->screen_bits, first + threadIdx.x, end, NT,
+            [&](long long t, double &rho, double &mu, double &mv, double &E) { node(M, t, rho, mu, mv, E); }, offer);
       }
       for (int o = 16; o > 0; o >>= 1) {
         const double other = __shfl_xor_sync(0xffffffffu, smax, o);
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
             float s32, e;
             screen_speed(M.g, rho, mu, mv, E, s32, e);
             if (s32 + e >= L && !memo.repeat(rho, mu, mv, E)) {
-              const double sp = exact_speed(M.g, rho, mu, mv, E);
+              const double sp = exact_speed(M.g.gamma, M.g.dx, M.g.dy, rho, mu, mv, E);
               if (sp != sp) nan_seen = 1;
               else if (sp > smax) smax = sp;
             }

@@ -30,7 +30,7 @@ struct Geom {
   int bc_left, bc_right, bc_y;  // y uses the bottom condition on both sides (src/WENOFD.cpp:1009)
   int gravity;                  // RTI source term (src/WENOFD.cpp:800-821)
   // FP32-form constants, rounded once on the host: gamma, zp_lambda, 1/dx, 1/dy
-  float gamma32, zpl32, inv_dx32, inv_dy32;
+  float gamma32, zpl32, inv_dx32, inv_dy32, gg32;
   // Bounds-checked build: the device guard record of this device
   // (guard.cuh); null in the release build.
   unsigned long long *guard;

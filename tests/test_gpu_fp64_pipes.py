@@ -93,3 +93,55 @@ def test_split_of_small_grids_changes_no_bit(nx, ny, batched):
                 assert s.advance(max_steps=3) == 3
             got.append(s.get_state())
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+def _speed_states(nx, ny):
+    """Conserved states whose time step goes through every branch: ties, one
+    maximum, values that FP32 or the integer forms do not hold, pressure left
+    over from a cancellation of 20 bits."""
+    rng = np.random.default_rng(nx * 1000 + ny)
+    rho = rng.uniform(0.5, 2.0, (nx, ny))
+    u, v, p = rng.uniform(-1, 1, (nx, ny)), rng.uniform(-1, 1, (nx, ny)), rng.uniform(0.5, 2.0, (nx, ny))
+
+    def state(rho, u, v, p):
+        return np.stack([rho, rho * u, rho * v, p / 0.4 + 0.5 * rho * (u * u + v * v)])
+
+    yield "random", state(rho, u, v, p)
+    half = np.where(np.arange(nx)[:, None] < nx // 2, 1.0, 0.125) * np.ones((nx, ny))
+    yield "ties", state(half, 0 * u, 0 * v, 1.6 * half)
+    yield "tiny", state(rho, u, v, p) * 2.0 ** -150
+    yield "huge", state(rho, u, v, p) * 2.0 ** 140
+    yield "cancelling", state(rho, 30 * u, 30 * v, 1e-3 * p)
+    mixed = state(rho, u, v, p)
+    mixed[:, nx // 2, ny // 3] *= 2.0 ** -90
+    mixed[1:3, nx // 3, ny // 2] *= 2.0 ** 35  # (kinetic energy below the energy: a positive pressure)
+    mixed[3, nx // 3, ny // 2] *= 2.0 ** 75
+    yield "mixed", mixed
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 6), (33, 65), (257, 193), (700, 411)])
+@pytest.mark.parametrize("precision", [wenofd.FP64, wenofd.FP32])
+def test_time_step_is_the_exact_maximum(nx, ny, precision):
+    """calc_dt, and the batched kernel's time step, against the formula in
+    float64 in the reference's operation order, bit for bit: the screen may
+    only drop nodes that do not hold the maximum and the integer forms round
+    as FP64 does."""
+    cfg = {"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.6, "SCHEME": 1, "SEED": 2,
+           "PRECISION": precision}
+    for name, U in _speed_states(nx, ny):
+        with wenofd.Solver(cfg) as s:
+            s.initialize()
+            inf = s.info()
+            with np.errstate(all="ignore"):
+                u, v = U[1] / U[0], U[2] / U[0]
+                p = (inf.gamma - 1.0) * (U[3] - 0.5 * U[0] * (u * u + v * v))
+                c = np.sqrt(inf.gamma * p / U[0])
+                dt = np.min(0.6 / ((np.abs(u) + c) / inf.dx + (np.abs(v) + c) / inf.dy))
+            assert np.isfinite(dt)
+            want = min(1.0, dt, inf.t_end)
+            s.set_state(U)
+            assert s.calc_dt() == want, name
+            if name in ("random", "ties", "cancelling"):
+                with wenofd.Batch([s]) as b:
+                    assert b.advance(1) == 1
+                assert s.info().now == want, name
