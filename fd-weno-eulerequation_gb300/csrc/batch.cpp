@@ -455,6 +455,11 @@ int wenofd_batch_advance(wenofd_batch *b, long long max_steps, long long *steps_
   std::vector<long long> before(b->n);
   for (int m = 0; m < b->n; ++m) before[m] = b->h_gather[m].steps;
   bool any_error = false;
+  // Launches between two looks at the status: a look leaves the GPU idle for
+  // some 20 us, which launches of one step (large batches) feel; up to 4 of
+  // those, never past the cap.  (One that finds no member able to step, or a
+  // wait that gave up in the one before, ends promptly.)
+  long long planned = 0;  // steps launched so far
   for (;;) {
     if (b->hold_block >= 0) {
       // armed by wenofd_batch_test_withhold: one direct launch of the test
@@ -471,8 +476,12 @@ int wenofd_batch_advance(wenofd_batch *b, long long max_steps, long long *steps_
       BATCH_TRY(cudaMemsetAsync(b->d_barrier, 0, sizeof(unsigned), b->stream));
       BATCH_TRY(wenofd::launch_batch_fp64_withhold(a, b->stream, &grid));
       b->launches += 1;
-    } else if (int rc = launch_step_block(b)) {
-      return rc;
+    } else {
+      for (int k = 0; k < (b->steps_per_launch <= 2 ? 4 : 1); ++k) {
+        if (k > 0 && max_steps >= 0 && planned >= max_steps) break;
+        if (int rc = launch_step_block(b)) return rc;
+        planned += b->steps_per_launch;
+      }
     }
     BATCH_TRY(cudaMemcpyAsync(b->h_flags, b->d_flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     BATCH_TRY(cudaStreamSynchronize(b->stream));

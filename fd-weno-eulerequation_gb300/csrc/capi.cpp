@@ -103,15 +103,6 @@ int check_handle(const wenofd_solver *s) {
 // Index of a state array in s->tma: 0 = S, 1 = A, 2 = B.
 int stage_buffer(const wenofd_solver *s, const double *in) { return in == s->A ? 1 : (in == s->B ? 2 : 0); }
 
-// After the stream has drained: TIMEOUT if a device wait gave up.
-int check_wait(wenofd_solver *s) {
-  if (!s->wait_error) return WENOFD_OK;
-  int err = 0;
-  CUDA_TRY(cudaMemcpy(&err, s->wait_error, sizeof(int), cudaMemcpyDeviceToHost));
-  if (err) return fail(WENOFD_TIMEOUT, "a bounded device wait gave up (stage TMA load or tensor-core completion)");
-  return WENOFD_OK;
-}
-
 int sync(wenofd_solver *s) {
   CUDA_TRY(cudaStreamSynchronize(s->stream));
   return WENOFD_OK;
@@ -154,12 +145,12 @@ int launch_stage(wenofd_solver *s, const double *in, const double *un, double *o
   // input (ghosts just filled); all stages of the step route with those flags.
   if (s->precision == WENOFD_LEARNED && in == s->S && un == s->S && s->ind_ready) {
     CUDA_TRY(wenofd::launch_indicator(s->g, in, s->ind_weights, s->ind_logit_threshold, s->ind_guard, s->flags,
-                                      s->wait_error,
+                                      &s->ctrl->wait_error,
                                       &s->ctrl->active, loop ? s->ctrl : nullptr, s->ind_interval,
                                       s->stream));
     s->launches += 1;
   }
-  args.wait_error = s->wait_error;
+  args.wait_error = &s->ctrl->wait_error;
   if (s->precision != WENOFD_FP64) {
     CUDA_TRY(wenofd::launch_stage_fp32(s->g, args, s->tma[stage_buffer(s, in)], s->scheme, s->tile_i, s->stage_rows,
                                        s->stream));
@@ -248,6 +239,13 @@ int read_ctrl(wenofd_solver *s) {
   return sync(s);
 }
 
+// On the control block just read: TIMEOUT if a device wait gave up.
+int check_wait(const wenofd_solver *s) {
+  if (s->ctrl_host->wait_error)
+    return fail(WENOFD_TIMEOUT, "a bounded device wait gave up (stage TMA load or tensor-core completion)");
+  return WENOFD_OK;
+}
+
 int copy_interior(wenofd_solver *s, double *dst_base, const double *src_base, size_t dst_pitch_b,
                   size_t src_pitch_b, bool to_device, cudaMemcpyKind kind) {
   const size_t plane_host = size_t(s->nx) * s->ny;
@@ -283,7 +281,6 @@ void release(wenofd_solver *s) {
   cudaFree(s->ctrl);
   cudaFree(s->flags);
   cudaFree(s->ind_weights);
-  cudaFree(s->wait_error);
   cudaFree(s->tile_bounds);
   cudaFreeHost(s->ctrl_host);
   cudaFreeHost(s->red_host);
@@ -407,9 +404,6 @@ int create_from_map(const std::map<std::string, std::string> &opt, wenofd_solver
     const size_t tiles = size_t((nx + 14) / 15) * size_t((ny + 31) / 32);
     ok = cudaMalloc(&s->tile_bounds, tiles * sizeof(float2)) == cudaSuccess;
   }
-  if (ok)  // the stage tiles' TMA waits (and the indicator's) report here
-    ok = cudaMalloc(&s->wait_error, sizeof(int)) == cudaSuccess &&
-         cudaMemsetAsync(s->wait_error, 0, sizeof(int), s->stream) == cudaSuccess;
   if (ok && precision == WENOFD_LEARNED) {
     const size_t fb = size_t(s->g.nxt) * s->g.pitch;
     ok = cudaMalloc(&s->flags, fb) == cudaSuccess &&
@@ -614,7 +608,13 @@ int wenofd_set_time(wenofd_solver *s, double now) {
   if (int rc = check_handle(s)) return rc;
   CUDA_TRY(cudaSetDevice(s->device));
   CUDA_TRY(wenofd::launch_set_time(s->ctrl, now, s->stream));
-  return sync(s);
+  // In stream order like wenofd_set_state_device: what follows on this stream,
+  // or in a batch (which waits for its members' streams), sees it.  A wait here
+  // cost each call about 20 us, 32 times per pass over a batch of 32.  A stream
+  // under capture is refused by the wait, as before.
+  cudaStreamCaptureStatus capture;
+  CUDA_TRY(cudaStreamIsCapturing(s->stream, &capture));
+  return capture == cudaStreamCaptureStatusNone ? WENOFD_OK : sync(s);
 }
 
 int wenofd_set_boundary_values(wenofd_solver *s, const double *host_table) {
@@ -641,7 +641,7 @@ int wenofd_get_flux(wenofd_solver *s, double *host_rhs) {
   if (int rc = launch_stage(s, s->S, s->S, s->A, 0.0, 0.0, 0.0, wenofd::kModeRHS)) return rc;
   if (host_rhs)
     if (int rc = download(s, s->A, host_rhs, cudaMemcpyDeviceToHost)) return rc;
-  if (int rc = sync(s)) return rc;
+  if (int rc = read_ctrl(s)) return rc;
   return check_wait(s);
 }
 
@@ -665,7 +665,7 @@ int wenofd_rk_step(wenofd_solver *s, double dt) {
   CUDA_TRY(cudaSetDevice(s->device));
   CUDA_TRY(wenofd::launch_set_dt(s->ctrl, dt, s->stream));
   if (int rc = enqueue_rk(s)) return rc;
-  if (int rc = sync(s)) return rc;
+  if (int rc = read_ctrl(s)) return rc;
   return check_wait(s);
 }
 
@@ -730,8 +730,6 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
   WENOFD_TRACE("wenofd_advance");
   if (int rc = check_handle(s)) return rc;
   CUDA_TRY(cudaSetDevice(s->device));
-  if (int rc = read_ctrl(s)) return rc;
-  const long long start = s->ctrl_host->steps;
   if (!s->graph) {
     // One gated-off pass outside capture configures the kernels' shared
     // memory limits on this device: the gate is closed (max_steps = steps),
@@ -752,6 +750,10 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
   // gated-off launches that return at once; when fewer steps than a chunk
   // remain, one-step graphs are replayed instead.
   long long left = max_steps < 0 ? -1 : max_steps;
+  // Graphs launched between two looks at the control block: one, until a step
+  // has shown how many are left; then as many as half of those fill, at most 8
+  // (a look leaves the GPU idle for some 20 us, which a one-step graph feels).
+  long long ahead = 1;
   for (;;) {
     if (left >= 0 && left < s->graph_steps) {
       if (!s->graph1) {
@@ -762,20 +764,25 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
         s->launches += s->graph1_kernels;
       }
     } else {
-      CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-      s->launches += s->graph_kernels;
+      for (long long k = 0; k < ahead; ++k) {
+        CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
+        s->launches += s->graph_kernels;
+      }
     }
     if (int rc = read_ctrl(s)) return rc;
     const Ctrl &c = *s->ctrl_host;
     if (int rc = check_wait(s)) return rc;
     if (c.error) {
-      if (steps_done) *steps_done = c.steps - start;
+      if (steps_done) *steps_done = c.steps - c.ind_base;
       return fail(WENOFD_NAN_DT, "Error: Timestep is not a number...");
     }
     if (c.done || c.steps >= c.max_steps) break;
     if (left >= 0) left = c.max_steps - c.steps;
+    const double rest = 0.5 * (c.t_end - c.now) / (c.dt * s->graph_steps);
+    ahead = rest >= 8.0 ? 8 : (rest >= 2.0 ? (long long)rest : 1);
+    if (left >= 0) ahead = std::max(1LL, std::min(ahead, left / s->graph_steps));
   }
-  if (steps_done) *steps_done = s->ctrl_host->steps - start;
+  if (steps_done) *steps_done = s->ctrl_host->steps - s->ctrl_host->ind_base;  // (set at the start)
   return WENOFD_OK;
 }
 
@@ -819,7 +826,7 @@ int wenofd_time_stages(wenofd_solver *s, int reps, double *ms_per_launch) {
       StageArgs a{x.in, x.un, x.out, x.a, x.b, x.c, &s->ctrl->dt, &s->ctrl->active, wenofd::kModeRK,
                   s->precision == WENOFD_LEARNED ? s->flags : nullptr};
       a.form = wenofd::rk_form(x.a, x.b, x.c, x.in, x.un);
-      a.wait_error = s->wait_error;
+      a.wait_error = &s->ctrl->wait_error;
       cudaError_t e = s->precision != WENOFD_FP64
                           ? wenofd::launch_stage_fp32(s->g, a, s->tma[stage_buffer(s, x.in)], s->scheme, s->tile_i,
                                                       s->stage_rows, s->stream)
@@ -835,6 +842,7 @@ int wenofd_time_stages(wenofd_solver *s, int reps, double *ms_per_launch) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   *ms_per_launch = double(ms) / (double(reps) * st.size());
+  if (int rc = read_ctrl(s)) return rc;
   return check_wait(s);
 }
 
@@ -875,13 +883,13 @@ int wenofd_indicator_flags(wenofd_solver *s, unsigned char *host_flags) {
   CUDA_TRY(wenofd::launch_ctrl_open(s->ctrl, s->stream));
   CUDA_TRY(wenofd::launch_bc_fill(s->g, s->S, s->special, nullptr, s->stream));
   CUDA_TRY(wenofd::launch_indicator(s->g, s->S, s->ind_weights, s->ind_logit_threshold, s->ind_guard, s->flags,
-                                    s->wait_error,
+                                    &s->ctrl->wait_error,
                                     nullptr, nullptr, 1, s->stream));
   s->launches += 3;
   CUDA_TRY(cudaMemcpy2DAsync(host_flags, s->ny, s->flags + size_t(wenofd::kGhost) * s->g.pitch + wenofd::kGhost,
                              s->g.pitch, s->ny, s->nx, cudaMemcpyDeviceToHost, s->stream));
   int err = 0;
-  CUDA_TRY(cudaMemcpyAsync(&err, s->wait_error, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CUDA_TRY(cudaMemcpyAsync(&err, &s->ctrl->wait_error, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   if (int rc = sync(s)) return rc;
   if (err) return fail(WENOFD_TIMEOUT, "indicator kernel: a tensor-core completion wait gave up");
   return WENOFD_OK;

@@ -59,6 +59,7 @@ struct Ctrl {
   // a time-step refinement forms dt, the last one of a step's last stage ends
   // the step.
   unsigned arrivals;
+  int wait_error;  // sticky: a device wait (TMA load, tensor-core completion) gave up
 };
 
 // Arguments of one RK stage launch.  uin is read with a 3-node halo (its
