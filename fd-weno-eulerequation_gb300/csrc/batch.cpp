@@ -53,7 +53,7 @@ struct wenofd_batch {
   int *h_flags = nullptr;
   BatchMemberStatus *h_gather = nullptr;
   // configuration
-  wenofd::Fp64Split split{15, 0};  // rows of the stage tiles (FP64 default configuration: fp64_split; else tile_i)
+  wenofd::Fp64Split split{15, 0};  // rows of the stage tiles (default configuration: fp64_split, the learned form 15 or 16; else tile_i)
   int tile_i = 15, blocks_per_sm = 0, steps_setting = 0, steps_per_launch = 1, grid = 0;
   // learned form: (indicator, interval steps) pairs per graph replay, and the
   // members' indicator settings the work plan was made with
@@ -115,7 +115,7 @@ BatchArgs make_args(const wenofd_batch *b, int nsteps) {
 cudaError_t launch_kernel(const wenofd_batch *b, const BatchArgs &a, int *grid) {
   if (b->precision == WENOFD_FP64)
     return wenofd::launch_batch_fp64(a, b->scheme, b->tile_i, b->blocks_per_sm, b->stream, grid);
-  if (b->learned) return wenofd::launch_batch_learned(a, b->scheme, b->tile_i, b->blocks_per_sm, b->stream, grid);
+  if (b->learned) return wenofd::launch_batch_learned(a, b->scheme, b->split.rows, b->blocks_per_sm, b->stream, grid);
   return wenofd::launch_batch_fp32(a, b->scheme, b->tile_i, b->blocks_per_sm, b->stream, grid);
 }
 
@@ -253,6 +253,14 @@ int configure(wenofd_batch *b, int tile_i, int blocks_per_sm, int steps_per_laun
     int sms = 0;
     BATCH_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
     b->split = wenofd::fp64_split(nx.data(), ny.data(), b->n, sms, b->tile_i);
+  }
+  if (b->learned && tile_i == 0) {
+    // the 16 x 32 marching tile where the members' tiles fill the resident blocks
+    // one and a half times, the rule and the reason of the single solve's
+    // stage_rows
+    long long tiles = 0;
+    for (const wenofd_solver *s : b->members) tiles += ceil_div(s->nx, 16) * ceil_div(s->ny, 32);
+    if (tiles > 3LL * 4 * 152 / 2) b->split.rows = 16;
   }
   b->blocks_per_sm = blocks_per_sm;
   b->steps_setting = steps_per_launch;
@@ -555,12 +563,13 @@ int wenofd_batch_autotune(wenofd_batch *b, int steps, double *ms_per_step) {
   int rc = WENOFD_OK;
   double best_ms = -1.0;
   int best_tile = b->tile_i, best_bps = 0;
-  const int tiles[2] = {15, b->precision == WENOFD_FP64 ? 7 : 31};
+  // (learned form: and the default's, which may be the marching tile)
+  const int tiles[3] = {15, b->precision == WENOFD_FP64 ? 7 : 31, 0};
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     rc = fail(WENOFD_CUDA_ERROR, "cudaEventCreate failed");
   }
   if (!rc) rc = copy_all(true);
-  for (int ti = 0; ti < 2 && !rc; ++ti) {
+  for (int ti = 0; ti < (b->learned ? 3 : 2) && !rc; ++ti) {
     // resident blocks per SM the kernel can take at this tile height
     if ((rc = configure(b, tiles[ti], 0, steps))) break;
     int sms = 0;

@@ -30,6 +30,7 @@
 
 #include "aux_device.cuh"
 #include "stage_kernel.cuh"
+#include "stage_routed.cuh"
 
 namespace wenofd {
 
@@ -406,7 +407,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
           a.bounds = M.tile_bounds;
           a.screen = &M.ctrl->screen_bits;
         }
-        if constexpr (F32)
+        if constexpr (ROUTE && TI == RoutedTile::TI)
+          routed_tile<SCHEME, true>(M.g, a, ti * TI, tj * TJ, smem_raw, local, nullptr);
+        else if constexpr (F32)
           stage_tile_f32<SCHEME, TI, TJ, NT, ROUTE, true, !(NT <= 256)>(M.g, a, ti * TI, tj * TJ, smem_raw, local);
         else stage_tile_f64<SCHEME, TI, TJ, NT, true>(M.g, a, ti * b.rows, tj * TJ, b.rows, b.pair != 0, smem_raw);
       });
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
 // from that query.
 template <typename T, int TI, int NT, bool WITHHOLD = false, bool ROUTE = false>
 cudaError_t launch_batch_tile(const BatchArgs &b, int scheme, int blocks_per_sm, cudaStream_t s, int *grid) {
-  constexpr size_t smem = stage_smem_bytes<T, TI, 32, false, NT>();
+  constexpr size_t smem = ROUTE && TI == RoutedTile::TI ? RoutedTile::bytes : stage_smem_bytes<T, TI, 32, false, NT>();
   void (*fn)(BatchArgs) = nullptr;
   if constexpr (WITHHOLD) {
     if (scheme != kWenoZ) return cudaErrorInvalidValue;

@@ -90,19 +90,31 @@ __device__ __forceinline__ void linear_march(const float4 *P, const float4 *M, i
   for (int k = 0; k <= N; ++k) h[k] = join2(lo[k], hi[k]);
 }
 
-// The FP32 state of ghosted node (ei, ej), as the tile's conversion gives it.
-__device__ __forceinline__ float4 node_f32(const Geom &g, const double *U, int ei, int ej) {
-  const double *p = U + WENOFD_GNODE(g, ei, ej);
-  return f64x4_to_f32(__ldg(p), __ldg(p + g.plane), __ldg(p + 2 * g.plane), __ldg(p + 3 * g.plane));
+// A load of state: the batched kernel's (COH) goes to L2, where other blocks'
+// writes of the same launch are; the per-solve kernel's may use L1.
+template <bool COH>
+__device__ __forceinline__ double load_state(const double *p) {
+  if constexpr (COH) return __ldcg(p);
+  else return __ldg(p);
 }
 
-template <int SCHEME>
-__global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
-    k_stage_routed(Geom g, StageArgs a, const __grid_constant__ StageTma tma) {
-  if (*a.active == 0) return;
+// The FP32 state of ghosted node (ei, ej), as the tile's conversion gives it.
+template <bool COH>
+__device__ __forceinline__ float4 node_f32(const Geom &g, const double *U, int ei, int ej) {
+  const double *p = U + WENOFD_GNODE(g, ei, ej);
+  return f64x4_to_f32(load_state<COH>(p), load_state<COH>(p + g.plane), load_state<COH>(p + 2 * g.plane),
+                      load_state<COH>(p + 3 * g.plane));
+}
+
+// The tile of interior nodes from (i0, j0), number `tile` of its grid; all
+// threads of the block.  COH (batched kernel): a thread loads its halo nodes from
+// L2 straight into registers and the flag rows by 16-byte loads, without the
+// boxes and their TMA maps.
+template <int SCHEME, bool COH>
+__device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, const int i0, const int j0,
+                                            unsigned char *smem_raw, const int tile, const StageTma *tma) {
   using S = RoutedTile;
   constexpr int TI = S::TI, TJ = S::TJ, HI = S::HI, NT = S::NT, W = S::kWarps, RW = S::kRows, CW = S::kCols;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char *base = smem_raw + (((tma_smem_addr(smem_raw) + 127u) & ~127u) - tma_smem_addr(smem_raw));
   float4 *Hf = reinterpret_cast<float4 *>(base + S::kRegion);
   __shared__ __align__(128) unsigned char sflag[S::kFlagBoxBytes];
@@ -110,19 +122,21 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
   __shared__ int scount_x, scount_y;
   __shared__ __align__(8) unsigned long long tma_bar;
   const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
-  const int i0 = int(blockIdx.y) * TI, j0 = int(blockIdx.x) * TJ;
   const bool stage1 = a.form == kFormStage1;
 
   if (threadIdx.x == 0) {
-    tma_bar_init(tma_smem_addr(&tma_bar), 1);
     scount_x = scount_y = 0;
-    const unsigned bar = tma_smem_addr(&tma_bar);
-    tma_fence_proxy();
-    tma_bar_expect(bar, S::kBoxBytes + S::kFlagBoxBytes);
-    // first coordinates x * element size a multiple of 16 bytes: j0 is a
-    // multiple of 32 (an unissued copy leaves the wait below to give up)
-    if (WENOFD_REQUIRE(g.guard, (j0 & 1) == 0, j0, 2)) tma_load_3d(tma_smem_addr(base), &tma.u, j0, 1 + i0, 0, bar);
-    if (WENOFD_REQUIRE(g.guard, (j0 & 15) == 0, j0, 16)) tma_load_2d(tma_smem_addr(sflag), &tma.flags, j0, 2 + i0, bar);
+    if constexpr (!COH) {
+      tma_bar_init(tma_smem_addr(&tma_bar), 1);
+      const unsigned bar = tma_smem_addr(&tma_bar);
+      tma_fence_proxy();
+      tma_bar_expect(bar, S::kBoxBytes + S::kFlagBoxBytes);
+      // first coordinates x * element size a multiple of 16 bytes: j0 is a
+      // multiple of 32 (an unissued copy leaves the wait below to give up)
+      if (WENOFD_REQUIRE(g.guard, (j0 & 1) == 0, j0, 2)) tma_load_3d(tma_smem_addr(base), &tma->u, j0, 1 + i0, 0, bar);
+      if (WENOFD_REQUIRE(g.guard, (j0 & 15) == 0, j0, 16))
+        tma_load_2d(tma_smem_addr(sflag), &tma->flags, j0, 2 + i0, bar);
+    }
   }
   // stages 2 and 3: ask L2 for this warp's rows of U^n (stage_tile_f32): lane =
   // component, row, and the line of column 0, 16 or 28
@@ -133,16 +147,18 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
       prefetch_l2(a.un + (t & 3) * g.plane + WENOFD_NODE(g, ii, min(j0 + (l == 2 ? 28 : 16 * l), g.ny - 1)));
     }
   }
-  __syncthreads();  // the barrier is initialised
-  if (threadIdx.x == 0) finish_step(a);
-  const bool landed = tma_bar_wait(tma_smem_addr(&tma_bar), 0, kTmaWaitLimit);
-  if (__syncthreads_or(!landed)) {
-    if (threadIdx.x == 0) {
-      if (a.wait_error) atomicExch(a.wait_error, 1);
-      tma_bar_wait(tma_smem_addr(&tma_bar), 0, kTmaWaitLimit);
+  if constexpr (!COH) {
+    __syncthreads();  // the barrier is initialised
+    if (threadIdx.x == 0) finish_step(a);
+    const bool landed = tma_bar_wait(tma_smem_addr(&tma_bar), 0, kTmaWaitLimit);
+    if (__syncthreads_or(!landed)) {
+      if (threadIdx.x == 0) {
+        if (a.wait_error) atomicExch(a.wait_error, 1);
+        tma_bar_wait(tma_smem_addr(&tma_bar), 0, kTmaWaitLimit);
+      }
+      __syncthreads();
+      return;
     }
-    __syncthreads();
-    return;
   }
 
   // this thread's nodes: column `lane` of halo rows warp, warp + W, ..; and of
@@ -152,7 +168,23 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
   float4 q[NR + 1];
   const int side = int(threadIdx.x) % 6, side_row = int(threadIdx.x) / 6;  // rows below TI only
   const int side_col = side < 3 ? side : TJ + side;                          // halo column
-  {
+  // flag node (fi, fj) is byte fi * 48 + fj + 2 of sflag, a row three 16-byte parts
+  const int flag_row = int(threadIdx.x) / 3, flag_part = int(threadIdx.x) % 3;
+  const bool has_flags = flag_row < TI + 4;
+  uint4 fv = make_uint4(0u, 0u, 0u, 0u);
+  if constexpr (COH) {
+    if (has_flags && 2 + i0 + flag_row < g.nxt && j0 + 16 * flag_part < g.pitch) {  // (rows are a multiple of 32)
+      const long long o = (long long)(2 + i0 + flag_row) * g.pitch + j0 + 16 * flag_part;
+      fv = __ldg(reinterpret_cast<const uint4 *>(a.flags + WENOFD_SPAN(g.guard, o, o + 15, (long long)g.nxt * g.pitch)));
+    }
+    auto node = [&](int hi, int hj) {  // beyond the last ghosts: a node of the last row or column, not used
+      return node_f32<true>(g, a.uin, min(1 + i0 + hi, g.nxt - 1), min(1 + j0 + hj, g.nyt - 1));
+    };
+#pragma unroll
+    for (int m = 0; m < NR; ++m) q[m] = node(min(warp + W * m, HI - 1), lane + 3);
+    q[NR] = node(min(side_row, TI - 1) + 3, side_col);
+    if (has_flags) reinterpret_cast<uint4 *>(sflag)[WENOFD_IX(g.guard, int(threadIdx.x), S::kFlagBoxBytes / 16)] = fv;
+  } else {
     const double *box = reinterpret_cast<const double *>(base);
     auto node = [&](int hi, int hj) {  // box column = halo column + 1
       const int o = hi * S::kBoxJ + hj + 1;
@@ -164,15 +196,12 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
 #pragma unroll
     for (int m = 0; m < NR; ++m) q[m] = node(min(warp + W * m, HI - 1), lane + 3);
     q[NR] = node(min(side_row, TI - 1) + 3, side_col);
+    if (has_flags) fv = reinterpret_cast<const uint4 *>(sflag)[WENOFD_IX(g.guard, int(threadIdx.x), S::kFlagBoxBytes / 16)];
   }
-  // any flag on the tile or within two nodes of it: flag node (fi, fj) is byte
-  // fi * 48 + fj + 2, so the row's first two and last ten bytes do not count
-  unsigned seen = 0;
-  if (threadIdx.x < 3 * (TI + 4)) {
-    const int part = int(threadIdx.x) % 3;
-    const uint4 v = reinterpret_cast<const uint4 *>(sflag)[WENOFD_IX(g.guard, int(threadIdx.x), S::kFlagBoxBytes / 16)];
-    seen = part == 0 ? (v.x & 0xffff0000u) | v.y | v.z | v.w : (part == 1 ? v.x | v.y | v.z | v.w : v.x | (v.y & 0x0000ffffu));
-  }
+  // any flag on the tile or within two nodes of it: the row's first two and last
+  // ten bytes do not count
+  const unsigned seen = flag_part == 0 ? (fv.x & 0xffff0000u) | fv.y | fv.z | fv.w
+                                       : (flag_part == 1 ? fv.x | fv.y | fv.z | fv.w : fv.x | (fv.y & 0x0000ffffu));
   const bool routed = __syncthreads_or(seen != 0u);
 
   const float gamma = g.gamma32, zpl = g.zpl32;
@@ -212,7 +241,7 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int f = t / TJ, j = t - f * TJ;
         const float w = weno_face_lane<0, SCHEME>(
-            gamma, zpl, node_f32(g, a.uin, 3 + i0 + f, 4 + j0 + j), node_f32(g, a.uin, 4 + i0 + f, 4 + j0 + j),
+            gamma, zpl, node_f32<COH>(g, a.uin, 3 + i0 + f, 4 + j0 + j), node_f32<COH>(g, a.uin, 4 + i0 + f, 4 + j0 + j),
             Fp + WENOFD_SPAN(g.guard, t, t + 4 * TJ, S::kX), Fm + WENOFD_SPAN(g.guard, t + TJ, t + 5 * TJ, S::kX), TJ,
             q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
@@ -273,7 +302,7 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int i = t / S::kHS, f = t - i * S::kHS, s = i * S::kYS + f;
         const float w = weno_face_lane<1, SCHEME>(
-            gamma, zpl, node_f32(g, a.uin, 4 + i0 + i, 3 + j0 + f), node_f32(g, a.uin, 4 + i0 + i, 4 + j0 + f),
+            gamma, zpl, node_f32<COH>(g, a.uin, 4 + i0 + i, 3 + j0 + f), node_f32<COH>(g, a.uin, 4 + i0 + i, 4 + j0 + f),
             Fp + WENOFD_SPAN(g.guard, s, s + 4, S::kY), Fm + WENOFD_SPAN(g.guard, s + 1, s + 5, S::kY), 1, q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
       }
@@ -292,13 +321,13 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
     const unsigned at = ok ? unsigned(WENOFD_NODE(g, i0 + i, j0 + lane) - origin) : 0u;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      ui[b][r] = __ldg(in + r * g.plane + at);
-      un[b][r] = stage1 ? 0.0 : __ldg(un0 + r * g.plane + at);
+      ui[b][r] = load_state<COH>(in + r * g.plane + at);
+      un[b][r] = stage1 ? 0.0 : load_state<COH>(un0 + r * g.plane + at);
     }
   };
   load_row(0, 0);
   __syncthreads();
-  const double dt = *a.dt;
+  const double dt = COH ? __ldcg(a.dt) : *a.dt;
   float lo = 0.0f, hi = 0.0f;  // screen bounds of this thread's nodes
   const float2 mi = splat2(-g.inv_dy32);
 #pragma unroll
@@ -329,8 +358,17 @@ __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
       hi = fmaxf(hi, s32 + e);
     }
   }
-  if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, int(blockIdx.y * gridDim.x + blockIdx.x));
-  store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
+  if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, tile);
+  if constexpr (!COH) store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
+}
+
+template <int SCHEME>
+__global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
+    k_stage_routed(Geom g, StageArgs a, const __grid_constant__ StageTma tma) {
+  if (*a.active == 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  routed_tile<SCHEME, false>(g, a, int(blockIdx.y) * RoutedTile::TI, int(blockIdx.x) * RoutedTile::TJ, smem_raw,
+                             int(blockIdx.y * gridDim.x + blockIdx.x), &tma);
 }
 
 }  // namespace dev

@@ -379,3 +379,38 @@ def test_routed_tile_of_large_grids_equals_the_small_tile(nx, ny, testcase, rk):
                 assert s.advance(max_steps=2) == 2
                 got.append(s.get_state())
         assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("rk", [1, 2])
+@pytest.mark.parametrize("sizes", [[(700, 450), (6, 6), (17, 33), (305, 641)], [(97, 95)] * 95])
+@pytest.mark.parametrize("testcase", [1, 2, 4])
+def test_batch_of_many_tiles_equals_the_small_tile(rk, sizes, testcase):
+    """Batches of many tiles march the 16 x 32 tile, loading its halo and flags
+    without TMA: the same operations node by node as the 15 x 32 tile, so the
+    same bits, with routed and unrouted tiles, on ragged members and over a
+    batch of equal ones (95 x 7 x 3 tiles, above the limit of 912)."""
+    params = mlp_oracle.init_params(3)
+
+    def run(tile_i):
+        solvers = [wenofd.Solver({"TESTCASE": testcase, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": rk, "CFL": 0.5,
+                                  "SCHEME": 1, "SEED": k + 1, "PRECISION": wenofd.LEARNED})
+                   for k, (nx, ny) in enumerate(sizes)]
+        for s in solvers:
+            s.initialize()
+            s.set_indicator(params, 0.5)
+        with wenofd.Batch(solvers) as b:
+            if tile_i is not None:
+                b.configure(tile_i=tile_i)
+            try:
+                assert b.advance(4) == 4
+                failed = None
+            except wenofd.WenofdError as e:  # an untrained network may drive a Riemann problem to a NaN time step
+                failed = str(e)
+        out = [(failed, s.info().steps, s.info().now, s.get_state()) for s in solvers]
+        for s in solvers:
+            s.close()
+        return out
+
+    for k, (a, b) in enumerate(zip(run(None), run(15))):
+        assert a[:3] == b[:3], sizes[k]
+        assert np.array_equal(a[3], b[3], equal_nan=True), sizes[k]
