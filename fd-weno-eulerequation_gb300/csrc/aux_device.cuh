@@ -152,15 +152,16 @@ __device__ __forceinline__ void store_images(const Geom &g, double *U, int i, in
 }
 
 // End of a stage tile in the time loop (all NT threads): the ghosts that the
-// tile's nodes determine, so that the loop needs no boundary launch per stage.
+// tile's nodes determine, so that the loop needs no boundary launch (batched
+// kernel: phase) per stage.
 // Read back from the nodes just stored, in the tiles at the grid's edge only:
 // done at each node's store it cost the grids of many tiles 4 to 12 % (a call and
 // the grid's description on the stack of every thread).
-template <int TI, int TJ, int NT>
-__device__ __forceinline__ void store_tile_ghosts(const Geom &g, const StageArgs &a, int i0, int j0) {
-  if (!a.ghosts || (i0 > kGhost && j0 > kGhost && i0 + TI + kGhost < g.nx && j0 + TJ + kGhost < g.ny)) return;
+template <int TJ, int NT>
+__device__ __forceinline__ void store_tile_ghosts(const Geom &g, const StageArgs &a, int i0, int j0, int rows) {
+  if (!a.ghosts || (i0 > kGhost && j0 > kGhost && i0 + rows + kGhost < g.nx && j0 + TJ + kGhost < g.ny)) return;
   __syncthreads();  // the tile's nodes are stored
-  for (int t = threadIdx.x; t < TI * TJ; t += NT) {
+  for (int t = threadIdx.x; t < rows * TJ; t += NT) {
     const int i = i0 + t / TJ, j = j0 + t % TJ;
     if (i < g.nx && j < g.ny) store_images(g, a.uout, i, j);
   }

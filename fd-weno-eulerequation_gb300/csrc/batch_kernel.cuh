@@ -3,8 +3,13 @@
 //
 // Each launch runs `nsteps` time steps of every member.  A step is a fixed
 // sequence of phases separated by grid-wide barriers:
-//   time-step reduction (FP64 exact pass; FP32 forms: screen, then refine)
-//   -> dt of every member -> 3 x (boundary fill -> stage tiles) -> time update.
+//   time-step reduction (FP32 forms: screen, then refine) -> dt of every member
+//   -> 3 x stage tiles -> time update.
+// The stage tiles write the ghosts of their results (store_tile_ghosts); the
+// first step of an advance fills those of U^n, and the SPECIAL ghosts of the
+// stage buffers, beside its time-step reduction (32 uneven members, 8 M nodes: a
+// fill before each stage, with its barrier, took 20 to 26 us).  RK1, whose
+// stage does not write U^n, fills before its stage.
 // As in the single solve, the FP32 forms' last RK stage screens the nodes it
 // writes (per-tile bounds), so from a member's second step on its time-step
 // reduction is the exact FP64 pass over the few tiles whose bound reaches
@@ -173,7 +178,20 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
       }
       all &= __syncthreads_and(ok);
     }
-    if (F32 && threadIdx.x == 0) *b.all_bounds = all;
+    if (threadIdx.x == 0) *b.all_bounds = all;
+  };
+  // ghosts of a member's U^n and, if every, of its stage buffers
+  auto fill = [&](unsigned *counter, bool every) {
+    for_member_items(b, counter, b.work.bc_prefix, sM, [&](int local, const BatchMember &M) {
+      const int first = local * kBcChunk, total = bc_entries(M.g);
+      for (int e = first + int(threadIdx.x); e < first + kBcChunk && e < total; e += NT) {
+        bc_fill_entry(M.g, M.S, M.special, e);
+        if (every) {
+          bc_fill_entry(M.g, M.A, M.special, e);
+          bc_fill_entry(M.g, M.B, M.special, e);
+        }
+      }
+    });
   };
   // dt = min(1, cfl / max s), clipped to t_end - now (src/WENOFD.cpp:401,
   // 426-435); NaN -> error NAN_DT (lines 437-442)
@@ -305,8 +323,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
         if (__ldcg(&M.ctrl->bounds_valid)) return;  // block-uniform: the tile pass covers it
       exact_pass(local, M);
     };
+    const bool all_valid = __ldcg(b.all_bounds) != 0;  // grid-uniform (set before the last release)
+    if (!all_valid && b.rk != 0) fill(cnt + 2, true);
     if constexpr (F32) {
-      const bool all_valid = __ldcg(b.all_bounds) != 0;  // grid-uniform (set before the last release)
       if (!all_valid) {
         // screen of the members without valid bounds: L = max (s32 - e), a
         // lower bound of the member's max s
@@ -337,9 +356,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
     // m_now += dt; count++ (src/WENOFD.cpp:213-224), then the next step's
     // gate; after the launch's last step, the host summary
     const bool last_step = step == b.nsteps - 1;
-    // FP32 forms, SSP-RK2/3: the last stage screens the nodes it writes
-    constexpr bool kFused = F32;
-    const bool fused = kFused && b.rk != 0;
+    // SSP-RK2/3: the stages write their ghosts and, in the FP32 forms, the last
+    // one screens the nodes it writes
+    const bool fused = b.rk != 0;
     auto step_end = [&]() {
       int alive = 0, err = 0, all = 1;
       for (int base = 0; base < n; base += NT) {
@@ -362,7 +381,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
         err |= __syncthreads_or(e);
         all &= __syncthreads_and(!can || (m < n && __ldcg(&b.members[m].ctrl->bounds_valid)));
       }
-      if (F32 && threadIdx.x == 0) *b.all_bounds = all;
+      if (threadIdx.x == 0) *b.all_bounds = all;
       if (last_step && threadIdx.x == 0) {
         b.status[0] = alive;
         b.status[1] = err;
@@ -374,13 +393,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
     // S -> A, then A's interior copied to S.
     const int nst = b.rk + 1;
     for (int st = 0; st < nst; ++st) {
-      for_member_items(b, cnt + 2 + 2 * st, b.work.bc_prefix, sM, [&](int local, const BatchMember &M) {
-        double *in = st == 0 ? M.S : (st == 1 ? M.A : M.B);
-        const int first = local * kBcChunk, total = bc_entries(M.g);
-        for (int e = first + int(threadIdx.x); e < first + kBcChunk && e < total; e += NT)
-          bc_fill_entry(M.g, in, M.special, e);
-      });
-      barrier(Nothing());
+      if (!fused) {
+        fill(cnt + 2, false);
+        barrier(Nothing());
+      }
       for_member_items(b, cnt + 3 + 2 * st, b.work.tile_prefix, sM, [&](int local, const BatchMember &M) {
         const int ti = WENOFD_IX(M.g.guard, local / M.tiles_j, F32 ? (M.g.nx + TI - 1) / TI : M.g.nx),
                   tj = local - (local / M.tiles_j) * M.tiles_j;
@@ -403,7 +419,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
         a.active = &M.ctrl->active;
         a.mode = kModeRK;
         a.flags = ROUTE ? M.flags : nullptr;
-        if (fused && st == nst - 1) {  // screen the new U^n into the member's tile bounds
+        a.ghosts = fused;
+        if (F32 && fused && st == nst - 1) {  // screen the new U^n into the member's tile bounds
           a.bounds = M.tile_bounds;
           a.screen = &M.ctrl->screen_bits;
         }
@@ -431,15 +448,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
     }
   }
   // the ghost nodes of U^n for the indicator launch that follows (members
-  // that can step; `active` was set by the last gate)
-  if (b.fill_end) {
-    for_member_items(b, b.counters + b.nsteps * kBatchPhases, b.work.bc_prefix, sM,
-                     [&](int local, const BatchMember &M) {
-                       const int first = local * kBcChunk, total = bc_entries(M.g);
-                       for (int e = first + int(threadIdx.x); e < first + kBcChunk && e < total; e += NT)
-                         bc_fill_entry(M.g, M.S, M.special, e);
-                     });
-  }
+  // that can step; `active` was set by the last gate), unless the last stage
+  // wrote them
+  if (b.fill_end && (b.nsteps == 0 || b.rk == 0)) fill(b.counters + b.nsteps * kBatchPhases, false);
 }
 
 // Cooperative launch of one kernel instance.  With b.members null: sets the

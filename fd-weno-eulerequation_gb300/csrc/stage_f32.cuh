@@ -553,7 +553,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
     }
   }
   if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, tile);  // block-uniform
-  if constexpr (TMA) store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
+  store_tile_ghosts<TJ, NT>(g, a, i0, j0, TI);
 }
 
 }  // namespace dev

@@ -256,6 +256,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
       }
     }
   }
+  if constexpr (COH) store_tile_ghosts<TJ, NT>(g, a, i0, j0, rows);
 }
 
 // Residency: the FP32 tiles read their FP64 inputs back in the epilogue

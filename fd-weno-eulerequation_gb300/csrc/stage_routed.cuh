@@ -359,7 +359,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
     }
   }
   if (a.bounds) store_tile_bounds<NT>(g, a, lo, hi, tile);
-  if constexpr (!COH) store_tile_ghosts<TI, TJ, NT>(g, a, i0, j0);
+  store_tile_ghosts<TJ, NT>(g, a, i0, j0, TI);
 }
 
 template <int SCHEME>

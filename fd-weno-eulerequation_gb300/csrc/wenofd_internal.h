@@ -50,7 +50,9 @@ struct Ctrl {
   // FP32 forms: the per-tile screen bounds of the current U^n (written by
   // the last RK stage of the previous step, with their maximum lower bound
   // in screen_bits) are valid, so the time-step reduction skips its screen
-  // pass.  Cleared at the start of every advance and by every other entry.
+  // pass.  Batched kernel, every form: also that the ghosts of U^n and of the
+  // stage buffers are filled.  Cleared at the start of every advance and by
+  // every other entry.
   int bounds_valid;
   // Learned form: steps counted from here (set at the start of every
   // advance) decide which steps run the indicator (INDICATOR_INTERVAL).
@@ -86,7 +88,7 @@ struct StageArgs {
   // on this integer instead of comparing the FP64 coefficients on the
   // device, where every FP64 compare issues on the 1/64-rate FP64 pipe.
   int form = 0;
-  // FP32 per-solve kernels in the time loop: the tile also writes the ghost
+  // In the time loop (not the FP64 single solve): the tile also writes the ghost
   // nodes whose values its nodes determine (store_tile_ghosts).
   int ghosts = 0;
   // Last stage of a step in the time loop: its last block to start ends the
@@ -189,7 +191,7 @@ struct BatchWork {
 
 constexpr int kBcChunk = 256;
 constexpr int kPtChunk = 4096;
-constexpr int kBatchPhases = 8;  // work counters per step: dt x 2, (bc, stage) x 3 (RK1: + copy)
+constexpr int kBatchPhases = 8;  // work counters per step: dt x 2, ghosts, stages at 3, 5, 7 (RK1: stage, copy)
 constexpr unsigned kBarrierLimit = 1u << 24;
 // Poll limit of the barrier in the withholding test instance (a few ms).
 constexpr unsigned kBarrierTestLimit = 1u << 12;
@@ -211,10 +213,10 @@ struct BatchArgs {
   // step nsteps (the counter array then holds nsteps + 1 steps).
   int fill_end = 0;
   int rows = 0, pair = 0;  // FP64 members: Fp64Split (rows: the kernel's tile height or fewer)
-  // FP32 forms: set by the block that releases a barrier when every member
-  // that can step holds valid tile bounds of its U^n (Ctrl::bounds_valid):
-  // the next time-step reduction then skips its screen and node passes and
-  // refines only the candidate tiles.
+  // Set by the block that releases a barrier when every member that can step
+  // holds valid tile bounds and ghosts of its U^n (Ctrl::bounds_valid): the next
+  // step then fills no ghosts, and the FP32 forms' time-step reduction skips its
+  // screen and node passes and refines only the candidate tiles.
   int *all_bounds = nullptr;
   // Test instance only (k_batch with WITHHOLD): block `hold_block` skips its
   // arrival at the launch's barrier number `hold_barrier` (counted from 0).

@@ -423,3 +423,46 @@ def test_learned_batch_with_guard_matches_single_solves():
     ref = _learned_run(2, 12, False, weights=(True,) * 4, guard=0.5, members=members)
     got = _learned_run(2, 12, True, weights=(True,) * 4, guard=0.5, members=members)
     _assert_learned_close(got, ref)
+
+
+@pytest.mark.parametrize("bc", [(0, 0, 0), (1, 3, 1), (3, 1, 0), (0, 0, 3), (2, 1, 3), (3, 2, 1), (0, 0, 2), (2, 2, 2),
+                                (1, 1, 2)])
+@pytest.mark.parametrize("rk", [0, 1, 2])
+@pytest.mark.parametrize("precision", [wenofd.FP64, wenofd.FP32, wenofd.LEARNED])
+def test_batched_ghosts_on_every_boundary(bc, rk, precision):
+    """The batch's stage tiles write the ghosts of their results and only the
+    first step of an advance fills them; host-driven single steps fill them
+    before every stage.  The FP64 form is the single solve's to the last bit,
+    the FP32 forms' tiles too on these grids (held to 1e-12; the learned form
+    to the batch's bound)."""
+    sizes = [(6, 6), (7, 9), (9, 40), (33, 65)]
+
+    def make():
+        solvers = []
+        for k, (nx, ny) in enumerate(sizes):
+            s = wenofd.Solver({"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": rk, "CFL": 0.4, "SCHEME": 1,
+                               "SEED": 6 + k, "PRECISION": precision, "BC_LEFT": bc[0], "BC_RIGHT": bc[1],
+                               "BC_BOTTOM": bc[2], "BC_TOP": bc[2]})
+            s.initialize()
+            if precision == wenofd.LEARNED:
+                import mlp_oracle
+
+                s.set_indicator(mlp_oracle.init_params(3), 0.5)
+            solvers.append(s)
+        return solvers
+
+    ref = make()
+    for s in ref:
+        for _ in range(5):
+            s.step()
+    got = make()
+    with wenofd.Batch(got) as b:
+        assert b.advance(2) == 2
+        assert b.advance(3) == 3
+    tol = {wenofd.FP64: 0.0, wenofd.FP32: 1e-12, wenofd.LEARNED: FP32_REL_TOL}[precision]
+    for s, r, size in zip(got, ref, sizes):
+        U, Ur = s.get_state(), r.get_state()
+        assert np.all(np.isfinite(Ur)), size
+        assert np.max(np.abs(U - Ur)) <= tol * np.max(np.abs(Ur)), size
+        s.close()
+        r.close()
