@@ -47,7 +47,7 @@ struct wenofd_batch {
   int counter_steps = 0;
   unsigned *d_ind_counter = nullptr;  // the batched indicator's work counter
   unsigned *d_barrier = nullptr;
-  int *d_flags = nullptr;  // [0] barrier gave up, [1..2] status, [3] indicator wait gave up, [4] all bounds valid
+  int *d_flags = nullptr;  // [0] barrier gave up, [1..2] status, [3] indicator wait gave up, [4] all bounds valid, [5] members that can step
   BatchMemberStatus *d_gather = nullptr;
   // host mirrors (pinned)
   int *h_flags = nullptr;
@@ -106,6 +106,7 @@ BatchArgs make_args(const wenofd_batch *b, int nsteps) {
   a.error = b->d_flags;
   a.status = b->d_flags + 1;
   a.all_bounds = b->d_flags + 4;
+  a.alive = b->d_flags + 5;
   a.guard = wenofd::guard_record();
   return a;
 }

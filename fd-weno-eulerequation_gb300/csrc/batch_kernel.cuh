@@ -144,6 +144,71 @@ __device__ __forceinline__ void for_member_items(const BatchArgs &b, unsigned *c
   }
 }
 
+// The FP64 state of member M's interior node (i, j), from L2.
+__device__ __forceinline__ void load_node(const BatchMember &M, int i, int j, double q[4]) {
+  const long long p = WENOFD_NODE(M.g, i, j);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) q[r] = __ldcg(&M.S[r * M.g.plane + p]);
+}
+
+// FP32 forms, members with valid tile bounds: the exact pass over the tiles
+// whose upper bound reaches L (the last stage raised screen_bits to the member's
+// maximum lower bound), a warp per tile over every member's tiles in a fixed
+// stride (k_dt_refine's tile pass).  Where most tiles remain (a Riemann problem's
+// uniform quadrants) a warp's time is its loads': four rows of them are in
+// flight together (80 -> 61 us for 32 members, 8 M nodes).  Out of line, so that
+// its registers are not the stage tiles' spills.
+template <int TI, int NT>
+__device__ __noinline__ void refine_tiles(const BatchMember *members, const int *prefix, int n,
+                                          unsigned long long *guard) {
+  const int lane = threadIdx.x & 31;
+  const int warps = int(gridDim.x) * (NT / 32);
+  const int total = __ldg(&prefix[n]);
+  for (int t = int(blockIdx.x) * (NT / 32) + int(threadIdx.x >> 5); t < total; t += warps) {
+    const int m = WENOFD_IX(guard, owner(prefix, n, t), n);
+    const BatchMember &M = members[m];
+    Ctrl *c = M.ctrl;
+    if (!__ldcg(&c->active) || !__ldcg(&c->bounds_valid)) continue;  // warp-uniform
+    const float L = __uint_as_float(__ldcg(&c->screen_bits));
+    const int local = t - __ldg(&prefix[m]);
+    const int tiles_j = M.tiles_j;
+    // (bounds are allocated for tiles of 15 rows, the most tiles)
+    if (__ldcg(&M.tile_bounds[WENOFD_IX(guard, local, ((M.g.nx + 14) / 15) * tiles_j)]).y < L) continue;
+    const int i0 = (local / tiles_j) * TI, j = (local - (local / tiles_j) * tiles_j) * 32 + lane;
+    const int i1 = i0 + TI < M.g.nx ? i0 + TI : M.g.nx;
+    double smax = 0.0;
+    int nan_seen = 0;
+    SpeedMemo memo;
+    if (j < M.g.ny) {
+      constexpr int kRows = 4;
+      for (int i = i0; i < i1; i += kRows) {
+        double q[kRows][4];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) load_node(M, min(i + k, i1 - 1), j, q[k]);
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {  // (the last row may come twice)
+          float s32, e;
+          screen_speed(M.g, q[k][0], q[k][1], q[k][2], q[k][3], s32, e);
+          if (s32 + e >= L && !memo.repeat(q[k][0], q[k][1], q[k][2], q[k][3])) {
+            const double sp = exact_speed(M.g.gamma, M.g.dx, M.g.dy, q[k][0], q[k][1], q[k][2], q[k][3]);
+            if (sp != sp) nan_seen = 1;
+            else if (sp > smax) smax = sp;
+          }
+        }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double other = __shfl_xor_sync(0xffffffffu, smax, o);
+      smax = other > smax ? other : smax;
+      nan_seen |= __shfl_xor_sync(0xffffffffu, nan_seen, o);
+    }
+    if (lane == 0) {
+      atomicMax(&c->max_s_bits, (unsigned long long)__double_as_longlong(smax));
+      if (nan_seen) atomicOr(&c->nan_flag, 1);
+    }
+  }
+}
+
 __device__ __forceinline__ int runnable(const Ctrl *c) {
   return (!__ldcg(&c->done) && !__ldcg(&c->error) && __ldcg(&c->steps) < __ldcg(&c->max_steps)) ? 1 : 0;
 }
@@ -166,19 +231,24 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
   // the loop condition of src/WENOFD.cpp:213, per member; FP32 forms: whether
   // every member that can step holds valid tile bounds (BatchArgs::all_bounds)
   auto gate = [&]() {
-    int all = 1;
+    int all = 1, alive = 0;
     for (int base = 0; base < n; base += NT) {
       const int m = base + int(threadIdx.x);
-      int ok = 1;
+      int can = 0, ok = 1;
       if (m < n) {
         Ctrl *c = b.members[m].ctrl;
-        const int can = runnable(c);
+        can = runnable(c);
         c->active = can;
         ok = !can || __ldcg(&c->bounds_valid);
       }
+      alive += __syncthreads_count(can);
       all &= __syncthreads_and(ok);
     }
-    if (threadIdx.x == 0) *b.all_bounds = all;
+    if (threadIdx.x == 0) {
+      *b.all_bounds = all;
+      *b.alive = alive;
+      if (alive == 0) b.status[0] = 0;
+    }
   };
   // ghosts of a member's U^n and, if every, of its stage buffers
   auto fill = [&](unsigned *counter, bool every) {
@@ -224,42 +294,29 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
 
   barrier(gate);
   for (int step = 0; step < b.nsteps; ++step) {
+    // No member can step: the launch is over (grid-uniform, written before the
+    // last release).  The empty phases of a step are 25 us: 2 steps of 8 FP64
+    // members in a launch of up to 16 spent a tenth of their time in the rest.
+    if (__ldcg(b.alive) == 0) break;
     unsigned *cnt = b.counters + step * kBatchPhases;
     // time-step reduction over each member's interior nodes
-    auto node = [&](const BatchMember &M, long long t, double &rho, double &mu, double &mv, double &E) {
-      const int i = int(t / M.g.ny), j = int(t - (t / M.g.ny) * M.g.ny);
-      const long long p = WENOFD_NODE(M.g, i, j);
-      rho = __ldcg(&M.S[p]);
-      mu = __ldcg(&M.S[M.g.plane + p]);
-      mv = __ldcg(&M.S[2 * M.g.plane + p]);
-      E = __ldcg(&M.S[3 * M.g.plane + p]);
-    };
     auto exact_pass = [&](int local, const BatchMember &M) {
       const long long first = (long long)local * kPtChunk;
       const long long npts = (long long)M.g.nx * M.g.ny;
       const long long end = first + kPtChunk < npts ? first + kPtChunk : npts;
       double smax = 0.0;
       int nan_seen = 0;
-      auto offer = [&](double s) {
-        if (s != s) nan_seen = 1;
-        else if (s > smax) smax = s;
-      };
-      if constexpr (F32) {  // refine: only nodes that can hold the maximum
-        const float L = __uint_as_float(__ldcg(&M.ctrl->screen_bits));
-        SpeedMemo memo;
-        for (long long t = first + threadIdx.x; t < end; t += NT) {
-          double rho, mu, mv, E;
-          node(M, t, rho, mu, mv, E);
-          float s32, e;
-          screen_speed(M.g, rho, mu, mv, E, s32, e);
-          if (s32 + e >= L && !memo.repeat(rho, mu, mv, E))
-            offer(exact_speed(M.g.gamma, M.g.dx, M.g.dy, rho, mu, mv, E));
-        }
-      } else {
-        screened_max(
-            M.g, &M.ctrl->screen_bits, first + threadIdx.x, end, NT,
-            [&](long long t, double &rho, double &mu, double &mv, double &E) { node(M, t, rho, mu, mv, E); }, offer);
-      }
+      screened_max(
+          M.g, &M.ctrl->screen_bits, first + threadIdx.x, end, NT,
+          [&](long long t, double &rho, double &mu, double &mv, double &E) {
+            double q[4];
+            load_node(M, int(t / M.g.ny), int(t - (t / M.g.ny) * M.g.ny), q);
+            rho = q[0], mu = q[1], mv = q[2], E = q[3];
+          },
+          [&](double s) {
+            if (s != s) nan_seen = 1;
+            else if (s > smax) smax = s;
+          });
       for (int o = 16; o > 0; o >>= 1) {
         const double other = __shfl_xor_sync(0xffffffffu, smax, o);
         smax = other > smax ? other : smax;
@@ -270,92 +327,19 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
         if (nan_seen) atomicOr(&M.ctrl->nan_flag, 1);
       }
     };
-    // FP32 forms, members with valid tile bounds: the exact pass over the
-    // tiles whose upper bound reaches L (the last stage raised screen_bits to
-    // the member's maximum lower bound), a warp per tile over every member's
-    // tiles in a fixed stride (k_dt_refine's tile pass)
-    auto tile_refine = [&]() {
-      const int lane = threadIdx.x & 31;
-      const int warps = int(gridDim.x) * (NT / 32);
-      const int total = __ldg(&b.work.tile_prefix[n]);
-      for (int t = int(blockIdx.x) * (NT / 32) + int(threadIdx.x >> 5); t < total; t += warps) {
-        const int m = WENOFD_IX(b.guard, owner(b.work.tile_prefix, n, t), n);
-        const BatchMember &M = b.members[m];
-        Ctrl *c = M.ctrl;
-        if (!__ldcg(&c->active) || !__ldcg(&c->bounds_valid)) continue;  // warp-uniform
-        const float L = __uint_as_float(__ldcg(&c->screen_bits));
-        const int local = t - __ldg(&b.work.tile_prefix[m]);
-        const int tiles_j = M.tiles_j;
-        // (bounds are allocated for tiles of 15 rows, the most tiles)
-        if (__ldcg(&M.tile_bounds[WENOFD_IX(b.guard, local, ((M.g.nx + 14) / 15) * tiles_j)]).y < L) continue;
-        const int i0 = (local / tiles_j) * TI, j = (local - (local / tiles_j) * tiles_j) * TJ + lane;
-        const int i1 = i0 + TI < M.g.nx ? i0 + TI : M.g.nx;
-        double smax = 0.0;
-        int nan_seen = 0;
-        SpeedMemo memo;
-        if (j < M.g.ny) {
-          for (int i = i0; i < i1; ++i) {
-            double rho, mu, mv, E;
-            node(M, (long long)i * M.g.ny + j, rho, mu, mv, E);
-            float s32, e;
-            screen_speed(M.g, rho, mu, mv, E, s32, e);
-            if (s32 + e >= L && !memo.repeat(rho, mu, mv, E)) {
-              const double sp = exact_speed(M.g.gamma, M.g.dx, M.g.dy, rho, mu, mv, E);
-              if (sp != sp) nan_seen = 1;
-              else if (sp > smax) smax = sp;
-            }
-          }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const double other = __shfl_xor_sync(0xffffffffu, smax, o);
-          smax = other > smax ? other : smax;
-          nan_seen |= __shfl_xor_sync(0xffffffffu, nan_seen, o);
-        }
-        if (lane == 0) {
-          atomicMax(&c->max_s_bits, (unsigned long long)__double_as_longlong(smax));
-          if (nan_seen) atomicOr(&c->nan_flag, 1);
-        }
-      }
-    };
-    // members without valid bounds: node chunks (FP64 form: every member)
-    auto chunk_pass = [&](int local, const BatchMember &M) {
-      if constexpr (F32)
-        if (__ldcg(&M.ctrl->bounds_valid)) return;  // block-uniform: the tile pass covers it
-      exact_pass(local, M);
-    };
     const bool all_valid = __ldcg(b.all_bounds) != 0;  // grid-uniform (set before the last release)
     if (!all_valid && b.rk != 0) fill(cnt + 2, true);
-    if constexpr (F32) {
-      if (!all_valid) {
-        // screen of the members without valid bounds: L = max (s32 - e), a
-        // lower bound of the member's max s
-        for_member_items(b, cnt + 0, b.work.pt_prefix, sM, [&](int local, const BatchMember &M) {
-          if (__ldcg(&M.ctrl->bounds_valid)) return;  // block-uniform
-          const long long first = (long long)local * kPtChunk;
-          const long long npts = (long long)M.g.nx * M.g.ny;
-          float lo = 0.0f;
-          for (long long t = first + threadIdx.x; t < first + kPtChunk && t < npts; t += NT) {
-            double rho, mu, mv, E;
-            node(M, t, rho, mu, mv, E);
-            float s, e;
-            screen_speed(M.g, rho, mu, mv, E, s, e);
-            lo = fmaxf(lo, s - e);
-          }
-          for (int o = 16; o > 0; o >>= 1) lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-          if ((threadIdx.x & 31) == 0) atomicMax(&M.ctrl->screen_bits, __float_as_uint(lo));
-        });
-        barrier(Nothing());
-        for_member_items(b, cnt + 1, b.work.pt_prefix, sM, chunk_pass);
-      }
-      tile_refine();
-    } else {
-      for_member_items(b, cnt + 1, b.work.pt_prefix, sM, exact_pass);
-    }
+    // node chunks: the members without valid bounds (FP64 form: every member)
+    if (!F32 || !all_valid)
+      for_member_items(b, cnt + 1, b.work.pt_prefix, sM, [&](int local, const BatchMember &M) {
+        if (F32 && __ldcg(&M.ctrl->bounds_valid)) return;  // block-uniform: the tile pass covers it
+        exact_pass(local, M);
+      });
+    if constexpr (F32) refine_tiles<TI, NT>(b.members, b.work.tile_prefix, n, b.guard);
     barrier(finalize);
 
     // m_now += dt; count++ (src/WENOFD.cpp:213-224), then the next step's
-    // gate; after the launch's last step, the host summary
-    const bool last_step = step == b.nsteps - 1;
+    // gate and the host summary
     // SSP-RK2/3: the stages write their ghosts and, in the FP32 forms, the last
     // one screens the nodes it writes
     const bool fused = b.rk != 0;
@@ -381,8 +365,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT <= 256 ? (ROUTE ? 4 :
         err |= __syncthreads_or(e);
         all &= __syncthreads_and(!can || (m < n && __ldcg(&b.members[m].ctrl->bounds_valid)));
       }
-      if (threadIdx.x == 0) *b.all_bounds = all;
-      if (last_step && threadIdx.x == 0) {
+      if (threadIdx.x == 0) {
+        *b.all_bounds = all;
+        *b.alive = alive;
         b.status[0] = alive;
         b.status[1] = err;
       }

@@ -218,6 +218,7 @@ struct BatchArgs {
   // step then fills no ghosts, and the FP32 forms' time-step reduction skips its
   // screen and node passes and refines only the candidate tiles.
   int *all_bounds = nullptr;
+  int *alive = nullptr;  // likewise: members that can step (none: the launch ends)
   // Test instance only (k_batch with WITHHOLD): block `hold_block` skips its
   // arrival at the launch's barrier number `hold_barrier` (counted from 0).
   int hold_block = -1, hold_barrier = -1;
