@@ -267,6 +267,21 @@ int download(wenofd_solver *s, const double *dev_full, double *dst, cudaMemcpyKi
   return copy_interior(s, dst, dev_full, s->ny * sizeof(double), s->g.pitch * sizeof(double), false, kind);
 }
 
+// The state and a caller's dense device array.  Memory that a kernel of this
+// device cannot be given (another device's, the host's, a start that is no
+// multiple of 8 bytes) takes the strided copies.
+int copy_device(wenofd_solver *s, double *dense, bool in) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, dense) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+      at.device == s->device && reinterpret_cast<uintptr_t>(dense) % 8 == 0) {
+    CUDA_TRY(wenofd::launch_copy_state(s->g, s->S, dense, in, s->stream));
+    s->launches += 1;
+    return WENOFD_OK;
+  }
+  cudaGetLastError();
+  return in ? upload(s, dense, cudaMemcpyDeviceToDevice) : download(s, s->S, dense, cudaMemcpyDeviceToDevice);
+}
+
 void release(wenofd_solver *s) {
   if (!s) return;
   cudaSetDevice(s->device);
@@ -582,14 +597,14 @@ int wenofd_set_state_device(wenofd_solver *s, const double *dev_state) {
   if (int rc = check_handle(s)) return rc;
   if (!dev_state) return fail(WENOFD_BAD_ARG, "null state");
   CUDA_TRY(cudaSetDevice(s->device));
-  return upload(s, dev_state, cudaMemcpyDeviceToDevice);
+  return copy_device(s, const_cast<double *>(dev_state), true);
 }
 
 int wenofd_get_state_device(wenofd_solver *s, double *dev_state) {
   if (int rc = check_handle(s)) return rc;
   if (!dev_state) return fail(WENOFD_BAD_ARG, "null state");
   CUDA_TRY(cudaSetDevice(s->device));
-  return download(s, s->S, dev_state, cudaMemcpyDeviceToDevice);
+  return copy_device(s, dev_state, false);
 }
 
 int wenofd_get_state_ghosted(wenofd_solver *s, double *host_full) {

@@ -308,6 +308,7 @@ cudaError_t launch_step_end(Ctrl *c, cudaStream_t s);
 cudaError_t launch_set_dt(Ctrl *c, double dt, cudaStream_t s);
 cudaError_t launch_set_time(Ctrl *c, double now, cudaStream_t s);
 cudaError_t launch_advance_setup(Ctrl *c, long long max_steps, cudaStream_t s);
+cudaError_t launch_copy_state(const Geom &g, double *U, double *dense, bool in, cudaStream_t s);
 cudaError_t launch_copy_interior(const Geom &g, const double *src, double *dst, const int *active, cudaStream_t s);
 // FP64 reductions over interior nodes into partials[nblk*4] then out[4]
 // (deterministic order).  kind 0: {Linf, L1, L2} of density against the

@@ -83,3 +83,27 @@ def test_load_rejects_other_grids_and_other_files(tmp_path):
         with pytest.raises(wenofd.WenofdError) as e:
             c.load_state(str(short))
         assert "truncated" in str(e.value)
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 6), (7, 31), (33, 128), (130, 129), (9, 700)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_device_state_round_trip(nx, ny, offset):
+    """wenofd_set_state_device and wenofd_get_state_device move exactly the
+    interior nodes, from and to any start that is a multiple of 8 bytes."""
+    torch = pytest.importorskip("torch")
+    U = np.random.default_rng(nx).uniform(1.0, 2.0, (4, nx, ny))
+    U[3] += 10.0
+    n = U.size
+    src = torch.full((n + 2,), -1.0, dtype=torch.float64, device="cuda")
+    src[offset:offset + n] = torch.from_numpy(U.ravel()).cuda()
+    dst = torch.full((n + 2,), -2.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with wenofd.Solver({"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.5, "SCHEME": 1}) as s:
+        lib = wenofd.lib()
+        assert lib.wenofd_set_state_device(s.handle, src.data_ptr() + 8 * offset) == wenofd.OK
+        assert np.array_equal(s.get_state(), U)
+        assert lib.wenofd_get_state_device(s.handle, dst.data_ptr() + 8 * offset) == wenofd.OK
+        s.info()  # waits for the solver's stream
+        got = dst.cpu().numpy()
+    assert np.array_equal(got[offset:offset + n], U.ravel())
+    assert np.all(got[:offset] == -2.0) and np.all(got[offset + n:] == -2.0)
