@@ -4,6 +4,7 @@
 #pragma once
 
 #include "approx.cuh"
+#include "chain.cuh"
 #include "convert.cuh"
 #include "guard.cuh"
 #include "int_f64.cuh"

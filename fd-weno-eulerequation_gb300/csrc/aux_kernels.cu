@@ -18,6 +18,8 @@ constexpr int kDtBlocks = 4;            // blocks of k_dt_reduce per SM
 
 
 __global__ void k_bc_fill(Geom g, double *U, const double *special, const int *active) {
+  dev::chain_wait();
+  dev::chain_release();
   if (active && *active == 0) return;
   const int total = dev::bc_entries(g);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
@@ -49,6 +51,8 @@ __device__ __forceinline__ void dt_finalize(Ctrl *c) {
   c->dt = timestep;
 }
 __global__ void k_dt_finalize(Ctrl *c) {
+  dev::chain_wait();
+  dev::chain_release();
   if (c->active) dt_finalize(c);
 }
 
@@ -62,6 +66,7 @@ __global__ void k_dt_finalize(Ctrl *c) {
 // All blocks are resident, so that their first passes run together and the
 // second ones meet a bound that is nearly the maximum.
 __global__ void __launch_bounds__(256, kDtBlocks) k_dt_reduce(Geom g, const double *U, Ctrl *c) {
+  dev::chain_wait();
   if (!c->active) return;
   double smax = 0.0;
   int nan_seen = 0;
@@ -77,6 +82,7 @@ __global__ void __launch_bounds__(256, kDtBlocks) k_dt_reduce(Geom g, const doub
         if (s != s) nan_seen = 1;
         else if (s > smax) smax = s;
       });
+  dev::chain_release();
   for (int o = 16; o > 0; o >>= 1) {
     const double other = __shfl_xor_sync(0xffffffffu, smax, o);
     smax = other > smax ? other : smax;
@@ -135,6 +141,7 @@ __global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
 // tiles remain, and a warp per tile (15 nodes a lane, one FP64 evaluation after
 // the other) took 37 us at 257 x 193 where this takes 9.
 __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *bounds, int tile_i) {
+  dev::chain_wait();
   if (!c->active) return;
   const float L = __uint_as_float(c->screen_bits);
   double smax = 0.0;
@@ -178,6 +185,7 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
       visit(i, j);
     }
   }
+  dev::chain_release();
   for (int o = 16; o > 0; o >>= 1) {
     const double other = __shfl_xor_sync(0xffffffffu, smax, o);
     smax = other > smax ? other : smax;
@@ -221,10 +229,16 @@ __global__ void k_ctrl_open(Ctrl *c) {
 
 // Start of a graph-driven step whose predecessor's last stage did not end it
 // (end_step).
-__global__ void k_step_begin(Ctrl *c) { dev::gate_step(c); }
+__global__ void k_step_begin(Ctrl *c) {
+  dev::chain_wait();
+  dev::chain_release();
+  dev::gate_step(c);
+}
 
 // The time update by itself: RK1, the FP64 form and the host-driven step.
 __global__ void k_step_end(Ctrl *c) {
+  dev::chain_wait();
+  dev::chain_release();
   if (c->active) dev::end_step(c, 0);
 }
 
@@ -453,14 +467,12 @@ unsigned long long *guard_record() { return nullptr; }
 
 cudaError_t launch_bc_fill(const Geom &g, double *U, const double *special, const int *active, cudaStream_t s) {
   const long long work = dev::bc_entries(g);
-  k_bc_fill<<<grid_for(work, 256), 256, 0, s>>>(g, U, special, active);
-  return cudaGetLastError();
+  return launch_chained(k_bc_fill, grid_for(work, 256), 256, 0, s, g, U, special, active);
 }
 
 cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream_t s) {
   const long long blocks = ((long long)g.nx * g.ny + 255) / 256;
-  k_dt_reduce<<<int(blocks < 152 * kDtBlocks ? blocks : 152 * kDtBlocks), 256, 0, s>>>(g, U, c);
-  return cudaGetLastError();
+  return launch_chained(k_dt_reduce, int(blocks < 152 * kDtBlocks ? blocks : 152 * kDtBlocks), 256, 0, s, g, U, c);
 }
 
 cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream_t s) {
@@ -473,8 +485,7 @@ cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const floa
   // arrival on the same word
   const int rows = tile_i > 0 ? tile_i : 15;
   const long long tiles = (long long)((g.nx + rows - 1) / rows) * ((g.ny + 31) / 32);
-  k_dt_refine<<<int(tiles < 152 * 8 ? tiles : 152 * 8), 256, 0, s>>>(g, U, c, bounds, rows);
-  return cudaGetLastError();
+  return launch_chained(k_dt_refine, int(tiles < 152 * 8 ? tiles : 152 * 8), 256, 0, s, g, U, c, bounds, rows);
 }
 
 cudaError_t launch_ctrl_open(Ctrl *c, cudaStream_t s) {
@@ -482,16 +493,13 @@ cudaError_t launch_ctrl_open(Ctrl *c, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_step_begin(Ctrl *c, cudaStream_t s) {
-  k_step_begin<<<1, 1, 0, s>>>(c);
-  return cudaGetLastError();
+  return launch_chained(k_step_begin, 1, 1, 0, s, c);
 }
 cudaError_t launch_dt_finalize(Ctrl *c, cudaStream_t s) {
-  k_dt_finalize<<<1, 1, 0, s>>>(c);
-  return cudaGetLastError();
+  return launch_chained(k_dt_finalize, 1, 1, 0, s, c);
 }
 cudaError_t launch_step_end(Ctrl *c, cudaStream_t s) {
-  k_step_end<<<1, 1, 0, s>>>(c);
-  return cudaGetLastError();
+  return launch_chained(k_step_end, 1, 1, 0, s, c);
 }
 cudaError_t launch_set_dt(Ctrl *c, double dt, cudaStream_t s) {
   k_set_dt<<<1, 1, 0, s>>>(c, dt);

@@ -286,7 +286,8 @@ void release(wenofd_solver *s) {
   if (!s) return;
   cudaSetDevice(s->device);
   if (s->graph) cudaGraphExecDestroy(s->graph);
-  if (s->graph1) cudaGraphExecDestroy(s->graph1);
+  for (cudaGraphExec_t t : s->tail)
+    if (t) cudaGraphExecDestroy(t);
   cudaFree(s->S);
   cudaFree(s->A);
   cudaFree(s->B);
@@ -734,9 +735,11 @@ int capture_steps(wenofd_solver *s, int nsteps, cudaGraphExec_t *exec, long long
 
 void drop_graphs(wenofd_solver *s) {
   if (s->graph) cudaGraphExecDestroy(s->graph);
-  if (s->graph1) cudaGraphExecDestroy(s->graph1);
   s->graph = nullptr;
-  s->graph1 = nullptr;
+  for (cudaGraphExec_t &t : s->tail) {
+    if (t) cudaGraphExecDestroy(t);
+    t = nullptr;
+  }
 }
 
 }  // namespace
@@ -761,9 +764,10 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
   CUDA_TRY(wenofd::launch_advance_setup(s->ctrl, max_steps, s->stream));
   s->launches += 1;
   if (int rc = prepare_loop(s)) return rc;
-  // Steps this call may still take (-1: no cap).  A chunk past the cap runs
-  // gated-off launches that return at once; when fewer steps than a chunk
-  // remain, one-step graphs are replayed instead.
+  // Steps this call may still take (-1: no cap).  A chunk past the cap would run
+  // gated-off launches; when fewer steps than a chunk remain, graphs of 1, 2, 4,
+  // .. steps that add up to them are replayed instead (one-step graphs, one after
+  // the other, left the GPU idle between them for longer than a kernel takes).
   long long left = max_steps < 0 ? -1 : max_steps;
   // Graphs launched between two looks at the control block: one, until a step
   // has shown how many are left; then as many as half of those fill, at most 8
@@ -771,12 +775,13 @@ int wenofd_advance(wenofd_solver *s, long long max_steps, long long *steps_done)
   long long ahead = 1;
   for (;;) {
     if (left >= 0 && left < s->graph_steps) {
-      if (!s->graph1) {
-        if (int rc = capture_steps(s, 1, &s->graph1, &s->graph1_kernels)) return rc;
-      }
-      for (long long k = 0; k < left; ++k) {
-        CUDA_TRY(cudaGraphLaunch(s->graph1, s->stream));
-        s->launches += s->graph1_kernels;
+      for (int k = 5; k >= 0; --k) {  // (a chunk has 64 steps at most)
+        if (!(left >> k & 1)) continue;
+        if (!s->tail[k]) {
+          if (int rc = capture_steps(s, 1 << k, &s->tail[k], &s->tail_kernels[k])) return rc;
+        }
+        CUDA_TRY(cudaGraphLaunch(s->tail[k], s->stream));
+        s->launches += s->tail_kernels[k];
       }
     } else {
       for (long long k = 0; k < ahead; ++k) {

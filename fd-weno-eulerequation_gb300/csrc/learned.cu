@@ -561,7 +561,7 @@ __device__ __forceinline__ bool indicator_band(const Geom &g, const double *U, f
         ok[q] = k < count && ei < g.nxt && ej < g.nyt;
         const double *src = U + WENOFD_GNODE_IF(g, ok[q], ei, ej);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) v[q][r] = ok[q] ? __ldg(src + r * g.plane) : 0.0;
+        for (int r = 0; r < 4; ++r) v[q][r] = ok[q] ? __ldcg(src + r * g.plane) : 0.0;
       }
 #pragma unroll
       for (int q = 0; q < NP; ++q) {
@@ -682,6 +682,7 @@ __global__ void __launch_bounds__(kCells, kResident) k_indicator_tc(Geom g, cons
                                                             float logit_threshold, float guard, unsigned char *flags,
                                                             int flag_pitch, int *error, const int *active,
                                                             const Ctrl *ctrl, int interval) {
+  dev::chain_wait();
   if (active && *active == 0) return;
   if (ctrl && interval > 1 && (ctrl->steps - ctrl->ind_base) % interval != 0) return;
   __shared__ __align__(128) __nv_bfloat16 sA[kCells * kK1];
@@ -704,6 +705,7 @@ __global__ void __launch_bounds__(kCells, kResident) k_indicator_tc(Geom g, cons
   const int first = int((long long)tiles_i * band / bands), last = int((long long)tiles_i * (band + 1) / bands);
   const IndSmem sm{sA, sW.w1, sW.w2, sW.w3, sRho, sPre};
   indicator_band(g, U, logit_threshold, guard, flags, flag_pitch, error, strip, first, last, sm, tc);
+  dev::chain_release();
   indicator_close(tc);
 }
 
@@ -843,10 +845,9 @@ cudaError_t launch_indicator(const Geom &g, const double *U, const void *weights
   // runs 64 bands of 2 tiles, not 76 of which some have 2 and some 1
   bands = (tiles_i + (tiles_i + bands - 1) / bands - 1) / ((tiles_i + bands - 1) / bands);
   const int grid = tiles_j * bands;
-  lrn::k_indicator_tc<<<grid, lrn::kCells, 0, s>>>(g, U, static_cast<const lrn::IndicatorWeights *>(weights),
-                                                   logit_threshold, guard, flags, g.pitch, error, active, ctrl,
-                                                   interval);
-  return cudaGetLastError();
+  return launch_chained(lrn::k_indicator_tc, grid, lrn::kCells, 0, s, g, U,
+                        static_cast<const lrn::IndicatorWeights *>(weights), logit_threshold, guard, flags, int(g.pitch),
+                        error, active, ctrl, interval);
 }
 
 cudaError_t launch_indicator_batch(const BatchMember *members, const int *ind_prefix, int n, unsigned *counter,

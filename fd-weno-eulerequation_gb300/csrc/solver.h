@@ -37,10 +37,10 @@ struct wenofd_solver {
   float ind_guard = 0.0f;          // INDICATOR_GUARD: relative window range that flags a node (0: off)
   bool ind_ready = false;
   cudaGraphExec_t graph = nullptr;   // graph_steps steps of the time loop
-  cudaGraphExec_t graph1 = nullptr;  // one step, for the tail of a capped advance
+  cudaGraphExec_t tail[6] = {};      // 1, 2, 4, .. 32 steps, for the tail of a capped advance
   int graph_steps = 0;
   long long graph_kernels = 0;   // kernel nodes in the graph
-  long long graph1_kernels = 0;  // kernel nodes in graph1
+  long long tail_kernels[6] = {};  // kernel nodes in each of `tail`
   long long launches = 0;       // kernels enqueued so far (graph replays included)
 };
 

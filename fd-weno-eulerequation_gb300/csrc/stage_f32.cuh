@@ -501,6 +501,7 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
   }
 
   // --- y term, source, RK combination in FP64, store
+  if constexpr (!COH) chain_release();
   const double dt = COH ? __ldcg(a.dt) : *a.dt;
   if constexpr (!COH && KEEP) {
     cp_async_wait_all_f32();
@@ -537,8 +538,8 @@ __device__ __forceinline__ void stage_tile_f32(const Geom &g, const StageArgs &a
         ui[r] = __ldcg(&a.uin[ix]);
         un[r] = __ldcg(&a.un[ix]);
       } else {
-        ui[r] = __ldg(&a.uin[ix]);
-        if (!stage1) un[r] = __ldg(&a.un[ix]);
+        ui[r] = __ldcg(&a.uin[ix]);
+        if (!stage1) un[r] = __ldcg(&a.un[ix]);
       }
     }
     double w[4];

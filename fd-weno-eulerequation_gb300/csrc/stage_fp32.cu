@@ -27,8 +27,7 @@ cudaError_t launch_routed(const Geom &g, const StageArgs &a, const StageTma &tma
     configured |= bit;
   }
   const dim3 grid((g.ny + T::TJ - 1) / T::TJ, (g.nx + T::TI - 1) / T::TI);
-  dev::k_stage_routed<SCHEME><<<grid, T::NT, T::bytes, s>>>(g, a, tma);
-  return cudaGetLastError();
+  return launch_chained(dev::k_stage_routed<SCHEME>, grid, T::NT, T::bytes, s, g, a, tma);
 }
 
 }  // namespace

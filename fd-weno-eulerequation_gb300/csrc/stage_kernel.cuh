@@ -229,6 +229,7 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
   }
 
   // --- source, RK combination, store
+  if constexpr (!COH) chain_release();
   const double dt = COH ? __ldcg(a.dt) : *a.dt;
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
@@ -281,6 +282,7 @@ __host__ __device__ constexpr bool stage_keeps_inputs() {
 template <typename T, int SCHEME, int TI, int TJ, int NT, bool ROUTE>
 __global__ void __launch_bounds__(NT, stage_blocks_per_sm<T, ROUTE, NT>())
     k_stage(Geom g, StageArgs a, const __grid_constant__ StageTma tma) {
+  chain_wait();
   if (*a.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // first interior node of the tile (0-based)
@@ -333,8 +335,7 @@ cudaError_t launch_stage_tile(const Geom &g, const StageArgs &args, const StageT
     if (e != cudaSuccess) return e;
     configured[scheme & 3] |= bit;
   }
-  fn<<<grid, NT, smem, s>>>(g, a, tma);
-  return cudaGetLastError();
+  return launch_chained(fn, grid, NT, smem, s, g, a, tma);
 }
 
 }  // namespace dev

@@ -90,20 +90,10 @@ __device__ __forceinline__ void linear_march(const float4 *P, const float4 *M, i
   for (int k = 0; k <= N; ++k) h[k] = join2(lo[k], hi[k]);
 }
 
-// A load of state: the batched kernel's (COH) goes to L2, where other blocks'
-// writes of the same launch are; the per-solve kernel's may use L1.
-template <bool COH>
-__device__ __forceinline__ double load_state(const double *p) {
-  if constexpr (COH) return __ldcg(p);
-  else return __ldg(p);
-}
-
 // The FP32 state of ghosted node (ei, ej), as the tile's conversion gives it.
-template <bool COH>
 __device__ __forceinline__ float4 node_f32(const Geom &g, const double *U, int ei, int ej) {
   const double *p = U + WENOFD_GNODE(g, ei, ej);
-  return f64x4_to_f32(load_state<COH>(p), load_state<COH>(p + g.plane), load_state<COH>(p + 2 * g.plane),
-                      load_state<COH>(p + 3 * g.plane));
+  return f64x4_to_f32(__ldcg(p), __ldcg(p + g.plane), __ldcg(p + 2 * g.plane), __ldcg(p + 3 * g.plane));
 }
 
 // The tile of interior nodes from (i0, j0), number `tile` of its grid; all
@@ -178,7 +168,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
       fv = __ldg(reinterpret_cast<const uint4 *>(a.flags + WENOFD_SPAN(g.guard, o, o + 15, (long long)g.nxt * g.pitch)));
     }
     auto node = [&](int hi, int hj) {  // beyond the last ghosts: a node of the last row or column, not used
-      return node_f32<true>(g, a.uin, min(1 + i0 + hi, g.nxt - 1), min(1 + j0 + hj, g.nyt - 1));
+      return node_f32(g, a.uin, min(1 + i0 + hi, g.nxt - 1), min(1 + j0 + hj, g.nyt - 1));
     };
 #pragma unroll
     for (int m = 0; m < NR; ++m) q[m] = node(min(warp + W * m, HI - 1), lane + 3);
@@ -241,7 +231,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int f = t / TJ, j = t - f * TJ;
         const float w = weno_face_lane<0, SCHEME>(
-            gamma, zpl, node_f32<COH>(g, a.uin, 3 + i0 + f, 4 + j0 + j), node_f32<COH>(g, a.uin, 4 + i0 + f, 4 + j0 + j),
+            gamma, zpl, node_f32(g, a.uin, 3 + i0 + f, 4 + j0 + j), node_f32(g, a.uin, 4 + i0 + f, 4 + j0 + j),
             Fp + WENOFD_SPAN(g.guard, t, t + 4 * TJ, S::kX), Fm + WENOFD_SPAN(g.guard, t + TJ, t + 5 * TJ, S::kX), TJ,
             q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
@@ -302,7 +292,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int i = t / S::kHS, f = t - i * S::kHS, s = i * S::kYS + f;
         const float w = weno_face_lane<1, SCHEME>(
-            gamma, zpl, node_f32<COH>(g, a.uin, 4 + i0 + i, 3 + j0 + f), node_f32<COH>(g, a.uin, 4 + i0 + i, 4 + j0 + f),
+            gamma, zpl, node_f32(g, a.uin, 4 + i0 + i, 3 + j0 + f), node_f32(g, a.uin, 4 + i0 + i, 4 + j0 + f),
             Fp + WENOFD_SPAN(g.guard, s, s + 4, S::kY), Fm + WENOFD_SPAN(g.guard, s + 1, s + 5, S::kY), 1, q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
       }
@@ -321,12 +311,13 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
     const unsigned at = ok ? unsigned(WENOFD_NODE(g, i0 + i, j0 + lane) - origin) : 0u;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      ui[b][r] = load_state<COH>(in + r * g.plane + at);
-      un[b][r] = stage1 ? 0.0 : load_state<COH>(un0 + r * g.plane + at);
+      ui[b][r] = __ldcg(in + r * g.plane + at);
+      un[b][r] = stage1 ? 0.0 : __ldcg(un0 + r * g.plane + at);
     }
   };
   load_row(0, 0);
   __syncthreads();
+  if constexpr (!COH) chain_release();
   const double dt = COH ? __ldcg(a.dt) : *a.dt;
   float lo = 0.0f, hi = 0.0f;  // screen bounds of this thread's nodes
   const float2 mi = splat2(-g.inv_dy32);
@@ -365,6 +356,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
 template <int SCHEME>
 __global__ void __launch_bounds__(RoutedTile::NT, RoutedTile::kBlocks)
     k_stage_routed(Geom g, StageArgs a, const __grid_constant__ StageTma tma) {
+  chain_wait();
   if (*a.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   routed_tile<SCHEME, false>(g, a, int(blockIdx.y) * RoutedTile::TI, int(blockIdx.x) * RoutedTile::TJ, smem_raw,
