@@ -109,8 +109,7 @@ __global__ void __launch_bounds__(256, kDtBlocks) k_dt_reduce(Geom g, const doub
 }
 
 // Pass 1: L = max over nodes of (s32 - e), a lower bound of max s.
-__global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
-  if (!c->active || c->bounds_valid) return;
+__device__ __forceinline__ void screen_nodes(const Geom &g, const double *U, Ctrl *c) {
   const long long n = (long long)g.nx * g.ny;
   float lo = 0.0f;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -129,6 +128,26 @@ __global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, wl[w]);
     atomicMax(&c->screen_bits, __float_as_uint(m));
   }
+}
+
+__global__ void k_dt_screen(Geom g, const double *U, Ctrl *c) {
+  if (!c->active || c->bounds_valid) return;
+  screen_nodes(g, U, c);
+}
+
+// Before the steps of a fused time loop: the ghosts of U^n, the SPECIAL ghosts of
+// the stage buffers (constants that no stage writes) and the screen of U^n, in
+// one launch (four of 3 to 6 us on small grids).
+__global__ void k_loop_open(Geom g, double *S, double *A, double *B, const double *special, Ctrl *c) {
+  dev::chain_wait();
+  if (!c->active) return;
+  const int total = dev::bc_entries(g);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    dev::bc_fill_entry(g, S, special, t);
+    dev::bc_fill_entry(g, A, special, t);
+    dev::bc_fill_entry(g, B, special, t);
+  }
+  screen_nodes(g, S, c);
 }
 
 // Pass 2: the exact FP64 s of every node with s32 + e >= L (the node holding
@@ -478,6 +497,12 @@ cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream
 cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream_t s) {
   k_dt_screen<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, s>>>(g, U, c);
   return cudaGetLastError();
+}
+
+cudaError_t launch_loop_open(const Geom &g, double *S, double *A, double *B, const double *special, Ctrl *c,
+                             cudaStream_t s) {
+  const long long work = std::max((long long)g.nx * g.ny, (long long)dev::bc_entries(g));
+  return launch_chained(k_loop_open, grid_for(work, 256), 256, 0, s, g, S, A, B, special, c);
 }
 
 cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i, cudaStream_t s) {

@@ -211,10 +211,8 @@ int enqueue_dt(wenofd_solver *s, bool screened = false) {
 // where a gate, a screen, a dt, an end and a ghost fill per stage made 11 or 12.
 int prepare_loop(wenofd_solver *s) {
   if (!fused_loop(s)) return WENOFD_OK;
-  for (double *buf : {s->S, s->A, s->B})
-    CUDA_TRY(wenofd::launch_bc_fill(s->g, buf, s->special, &s->ctrl->active, s->stream));
-  CUDA_TRY(wenofd::launch_dt_screen(s->g, s->S, s->ctrl, s->stream));
-  s->launches += 4;
+  CUDA_TRY(wenofd::launch_loop_open(s->g, s->S, s->A, s->B, s->special, s->ctrl, s->stream));
+  s->launches += 1;
   return WENOFD_OK;
 }
 

@@ -300,6 +300,8 @@ cudaError_t launch_dt_reduce(const Geom &g, const double *U, Ctrl *c, cudaStream
 // Ctrl::bounds_valid set, the screen pass is skipped and the refine pass
 // visits only the tiles whose upper bound reaches the maximum lower bound.
 cudaError_t launch_dt_screen(const Geom &g, const double *U, Ctrl *c, cudaStream_t s);
+cudaError_t launch_loop_open(const Geom &g, double *S, double *A, double *B, const double *special, Ctrl *c,
+                             cudaStream_t s);
 cudaError_t launch_dt_refine(const Geom &g, const double *U, Ctrl *c, const float2 *bounds, int tile_i, cudaStream_t s);
 cudaError_t launch_ctrl_open(Ctrl *c, cudaStream_t s);
 cudaError_t launch_step_begin(Ctrl *c, cudaStream_t s);
