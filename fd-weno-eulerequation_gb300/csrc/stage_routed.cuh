@@ -13,7 +13,7 @@
 // it), and the state stays in registers between the two splits.
 // A tile with a flag on or around it (block-uniform) also stores the faces,
 // recomputes the listed ones with characteristic WENO (weno_face_lane, four
-// lanes a face, the faces' two nodes from global memory) and takes the
+// lanes a face, the faces' nodes from the state it keeps) and takes the
 // differences from the stored faces.
 //
 // What bounds it, 4096^2, mean of the three stages, without the time-step
@@ -22,7 +22,12 @@
 // combination 424: the FP64 pipe (262 us of it) and the copies' latency, partly
 // overlapped.  Stages 1 / 2 / 3 in the time loop: 444 / 497 / 587 us with the 15 x
 // 32 tile of stage_f32.cuh, 339 / 408 / 526 here with no flag in the interior; 487
-// / 550 / 638 and 441 / 522 / 637 with 0.7 % of the nodes flagged one by one.
+// / 550 / 638 and 441 / 522 / 637 with 0.7 % of the nodes flagged one by one.  Those
+// with the listed faces' nodes loaded from global memory; kept in shared memory, a
+// step at 2400^2 with 10 / 28 / 100 % of the nodes flagged takes 0.89 / 1.20 / 1.49
+// ms instead of 1.08 / 1.55 / 2.01 (15 x 32: 0.94 / 1.24 / 1.52), and 4096^2 with
+// few flags 1.68 instead of 1.73; placed behind the box instead of over its end,
+// 12 % less L1 for the spills cost the batched kernel 5 %.
 // Other shapes (rows, threads, blocks per SM): (32, 256, 3) 319 / 440 / 541, (32,
 // 512, 2) 375 / 483 / 640, (16, 256, 5) 390 / 482 / 557, (16, 128, 5) 332 / 449 /
 // 553; the next tile's copies under this one's combination (persistent blocks)
@@ -47,9 +52,14 @@ struct RoutedTile {
   static constexpr int kY = TI * kYS;
   static constexpr int kHS = TJ + 1;           // row stride of the y faces and differences
   static constexpr int kFace = (TI + 1) * TJ > TI * kHS ? (TI + 1) * TJ : TI * kHS;
-  static constexpr size_t kRegion = kBoxBytes;  // box, then F+ and F- of a sweep
-  static_assert(2 * sizeof(float4) * (kX > kY ? kX : kY) <= kRegion, "both split fluxes fit over the box");
-  static constexpr size_t bytes = 128 + kRegion + sizeof(float4) * kFace;
+  // shared memory: F+ and F- of a sweep, the state of a tile with a flag, the
+  // faces; the box lies over the first two and is in registers before either is
+  // written.  (The L1 cache has what four blocks leave: spills live there.)
+  static constexpr size_t kSplits = 2 * sizeof(float4) * (kX > kY ? kX : kY);
+  static constexpr int kUS = TJ + 6, kU = HI * kUS;  // FP32 state with halo [HI][TJ + 6], kept by tiles with a flag
+  static constexpr size_t kFaces = kSplits + sizeof(float4) * kU;  // offset of the faces
+  static_assert(kBoxBytes <= kFaces && kSplits % 16 == 0, "the box ends before the faces");
+  static constexpr size_t bytes = 128 + kFaces + sizeof(float4) * kFace;
 };
 
 // N + 1 consecutive faces of one line of nodes: faces f0 .. f0 + N from F+ at
@@ -106,7 +116,7 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
   using S = RoutedTile;
   constexpr int TI = S::TI, TJ = S::TJ, HI = S::HI, NT = S::NT, W = S::kWarps, RW = S::kRows, CW = S::kCols;
   unsigned char *base = smem_raw + (((tma_smem_addr(smem_raw) + 127u) & ~127u) - tma_smem_addr(smem_raw));
-  float4 *Hf = reinterpret_cast<float4 *>(base + S::kRegion);
+  float4 *Us = reinterpret_cast<float4 *>(base + S::kSplits), *Hf = reinterpret_cast<float4 *>(base + S::kFaces);
   __shared__ __align__(128) unsigned char sflag[S::kFlagBoxBytes];
   __shared__ short slist[S::kFace];
   __shared__ int scount_x, scount_y;
@@ -193,6 +203,12 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
   const unsigned seen = flag_part == 0 ? (fv.x & 0xffff0000u) | fv.y | fv.z | fv.w
                                        : (flag_part == 1 ? fv.x | fv.y | fv.z | fv.w : fv.x | (fv.y & 0x0000ffffu));
   const bool routed = __syncthreads_or(seen != 0u);
+  if (routed) {  // the listed faces' nodes
+#pragma unroll
+    for (int m = 0; m < NR; ++m)
+      if (warp + W * m < HI) Us[WENOFD_IX(g.guard, (warp + W * m) * S::kUS + lane + 3, S::kU)] = q[m];
+    if (side_row < TI) Us[WENOFD_IX(g.guard, (side_row + 3) * S::kUS + side_col, S::kU)] = q[NR];
+  }
 
   const float gamma = g.gamma32, zpl = g.zpl32;
   float4 *Fp = reinterpret_cast<float4 *>(base), *Fm = Fp + S::kX;
@@ -231,7 +247,8 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int f = t / TJ, j = t - f * TJ;
         const float w = weno_face_lane<0, SCHEME>(
-            gamma, zpl, node_f32(g, a.uin, 3 + i0 + f, 4 + j0 + j), node_f32(g, a.uin, 4 + i0 + f, 4 + j0 + j),
+            gamma, zpl, Us[WENOFD_IX(g.guard, (f + 2) * S::kUS + j + 3, S::kU)],
+            Us[WENOFD_IX(g.guard, (f + 3) * S::kUS + j + 3, S::kU)],
             Fp + WENOFD_SPAN(g.guard, t, t + 4 * TJ, S::kX), Fm + WENOFD_SPAN(g.guard, t + TJ, t + 5 * TJ, S::kX), TJ,
             q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
@@ -292,7 +309,8 @@ __device__ __forceinline__ void routed_tile(const Geom &g, const StageArgs &a, c
         const int t = slist[WENOFD_IX(g.guard, q4 < 4 * nw ? q4 >> 2 : 0, S::kFace)];
         const int i = t / S::kHS, f = t - i * S::kHS, s = i * S::kYS + f;
         const float w = weno_face_lane<1, SCHEME>(
-            gamma, zpl, node_f32(g, a.uin, 4 + i0 + i, 3 + j0 + f), node_f32(g, a.uin, 4 + i0 + i, 4 + j0 + f),
+            gamma, zpl, Us[WENOFD_IX(g.guard, (i + 3) * S::kUS + f + 2, S::kU)],
+            Us[WENOFD_IX(g.guard, (i + 3) * S::kUS + f + 3, S::kU)],
             Fp + WENOFD_SPAN(g.guard, s, s + 4, S::kY), Fm + WENOFD_SPAN(g.guard, s + 1, s + 5, S::kY), 1, q4 & 3);
         if (q4 < 4 * nw) reinterpret_cast<float *>(&Hf[WENOFD_IX(g.guard, t, S::kFace)])[q4 & 3] = w;
       }
