@@ -184,8 +184,8 @@ __global__ void k_dt_refine(Geom g, const double *U, Ctrl *c, const float2 *boun
       if (threadIdx.x == 0) nkept = 0;
       __syncthreads();
       const long long t = first + (long long)threadIdx.x * gridDim.x;
-      // (bounds are allocated for tiles of 15 rows, the most tiles)
-      if (t < ntiles && !(bounds[WENOFD_IX(g.guard, t, ((g.nx + 14) / 15) * tiles_j)].y < L))
+      // (bounds are allocated for tiles of 7 rows, the most tiles)
+      if (t < ntiles && !(bounds[WENOFD_IX(g.guard, t, ((g.nx + 6) / 7) * tiles_j)].y < L))
         kept[WENOFD_IX(g.guard, atomicAdd(&nkept, 1), 256)] = int(t);
       __syncthreads();
       const int count = nkept;

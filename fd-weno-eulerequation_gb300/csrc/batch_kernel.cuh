@@ -172,8 +172,8 @@ __device__ __noinline__ void refine_tiles(const BatchMember *members, const int 
     const float L = __uint_as_float(__ldcg(&c->screen_bits));
     const int local = t - __ldg(&prefix[m]);
     const int tiles_j = M.tiles_j;
-    // (bounds are allocated for tiles of 15 rows, the most tiles)
-    if (__ldcg(&M.tile_bounds[WENOFD_IX(guard, local, ((M.g.nx + 14) / 15) * tiles_j)]).y < L) continue;
+    // (bounds are allocated for tiles of 7 rows, the most tiles)
+    if (__ldcg(&M.tile_bounds[WENOFD_IX(guard, local, ((M.g.nx + 6) / 7) * tiles_j)]).y < L) continue;
     const int i0 = (local / tiles_j) * TI, j = (local - (local / tiles_j) * tiles_j) * 32 + lane;
     const int i1 = i0 + TI < M.g.nx ? i0 + TI : M.g.nx;
     double smax = 0.0;

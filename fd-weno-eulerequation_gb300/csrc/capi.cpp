@@ -414,8 +414,8 @@ int create_from_map(const std::map<std::string, std::string> &opt, wenofd_solver
             cudaMalloc(&s->ctrl, sizeof(Ctrl)) == cudaSuccess &&
             cudaMallocHost(&s->ctrl_host, sizeof(Ctrl)) == cudaSuccess &&
             cudaMallocHost(&s->red_host, 4 * sizeof(double)) == cudaSuccess;
-  if (ok && precision != WENOFD_FP64) {  // stage tiles of 15 (or 16, or 31) x 32 nodes
-    const size_t tiles = size_t((nx + 14) / 15) * size_t((ny + 31) / 32);
+  if (ok && precision != WENOFD_FP64) {  // stage tiles of 7 (or 15, 16, 31) x 32 nodes
+    const size_t tiles = size_t((nx + 6) / 7) * size_t((ny + 31) / 32);
     ok = cudaMalloc(&s->tile_bounds, tiles * sizeof(float2)) == cudaSuccess;
   }
   if (ok && precision == WENOFD_LEARNED) {

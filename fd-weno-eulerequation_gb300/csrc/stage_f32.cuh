@@ -172,8 +172,8 @@ __device__ __forceinline__ void store_tile_bounds(const Geom &g, const StageArgs
     float2 b = sred[0];
 #pragma unroll
     for (int w = 1; w < NT / 32; ++w) b = make_float2(fmaxf(b.x, sred[w].x), fmaxf(b.y, sred[w].y));
-    // (allocated for tiles of 15 rows, the most tiles)
-    a.bounds[WENOFD_IX(g.guard, tile, ((g.nx + 14) / 15) * ((g.ny + 31) / 32))] = b;
+    // (allocated for tiles of 7 rows, the most tiles)
+    a.bounds[WENOFD_IX(g.guard, tile, ((g.nx + 6) / 7) * ((g.ny + 31) / 32))] = b;
     atomicMax(a.screen, __float_as_uint(b.x));
   }
 }

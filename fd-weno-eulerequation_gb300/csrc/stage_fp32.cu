@@ -36,8 +36,17 @@ cudaError_t launch_routed(const Geom &g, const StageArgs &a, const StageTma &tma
 // resident blocks (four on each of 152 SMs) one and a half times, else 15 x 32,
 // whose block is done sooner.  Measured, 8 steps (k_stage_routed / 15 x 32): 512^2
 // 920 / 911 us, 700^2 1,133 / 1,145, 1024^2 1,694 / 1,764, 2048^2 4,538 / 4,801.
+// Grids whose tiles of 7 rows fit the resident blocks at once (three on each SM in
+// the FP32 form, four in the learned form) take those: a tile's time is the
+// latency of its rounds of faces, and a short tile has two instead of four.  A step,
+// 7 rows / 15: FP32 100^2 25 / 36 us, 257 x 193 31 / 38, 300^2 (430 tiles of 456) 34
+// / 44; learned 100^2 33 / 44, 257 x 193 39 / 49, 350^2 (550 of 608) 52 / 63.
 int stage_rows(const Geom &g, int precision, int tile_i) {
   using T = dev::RoutedTile;
+  if (precision != 0 && tile_i == 0) {
+    const long long tiles = (long long)((g.nx + 6) / 7) * ((g.ny + 31) / 32);
+    if (tiles <= (precision == 2 ? 4 : 3) * 152LL) return 7;
+  }
   if (precision == 2 && tile_i == 0) {
     const long long tiles = (long long)((g.nx + T::TI - 1) / T::TI) * ((g.ny + T::TJ - 1) / T::TJ);
     if (tiles > 3LL * T::kBlocks * 152 / 2) return T::TI;
@@ -58,6 +67,9 @@ cudaError_t launch_stage_fp32(const Geom &g, const StageArgs &a, const StageTma 
     }
     return cudaErrorInvalidValue;
   }
+  if (rows == 7 && tile_i == 0)
+    return a.flags ? dev::launch_stage_tile<float, 7, 256, true>(g, a, tma, scheme, s)
+                   : dev::launch_stage_tile<float, 7, 256>(g, a, tma, scheme, s);
   if (a.flags) {
     switch (tile_i) {
       case 0:

@@ -111,7 +111,7 @@ struct StageTma {
   CUtensorMap flags;
 };
 // Encodes the maps of one state array (and of the flag array, if not null)
-// for stage tiles of up to `rows` rows (FP32 tiles 15 or 31, the learned form's
+// for stage tiles of up to `rows` rows (FP32 tiles 7, 15 or 31, the learned form's
 // 16, FP64 tiles 15 or 7; stage_rows).
 cudaError_t make_stage_tma(const Geom &g, const double *state, const unsigned char *flags, int rows, StageTma *out);
 // Rows of the per-solve stage tiles of a precision form with TILE_I = tile_i.

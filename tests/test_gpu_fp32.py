@@ -126,6 +126,28 @@ def test_fused_screen_steps_equal_separate_steps(precision, tile_i):
     assert np.array_equal(Ua, Ub)
 
 
+@pytest.mark.parametrize("nx,ny", [(6, 6), (7, 32), (8, 33), (14, 64), (15, 97), (300, 300), (307, 321)])
+@pytest.mark.parametrize("precision", [wenofd.FP32, wenofd.LEARNED])
+def test_short_tiles_of_small_grids_equal_the_default_height(nx, ny, precision):
+    """Grids whose 7-row tiles are resident at once take those (300^2: 430 of
+    456 FP32 tiles; 307 x 321: 484, past the FP32 form's limit and within the
+    learned form's); every node's operations are those of the 15-row tile, so
+    the states and the times are the same bits."""
+    import mlp_oracle
+
+    got = []
+    for tile_i in (0, 15):
+        with wenofd.Solver({"TESTCASE": 5, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.5, "SCHEME": 1,
+                            "SEED": 8, "PRECISION": precision, "TILE_I": tile_i}) as s:
+            s.initialize()
+            if precision == wenofd.LEARNED:
+                s.set_indicator(mlp_oracle.init_params(3), 0.5)
+            assert s.advance(max_steps=6) == 6
+            got.append((s.info().now, s.get_state()))
+    assert got[0][0] == got[1][0]
+    assert np.all(np.isfinite(got[0][1])) and np.array_equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("bc", [(0, 0, 0), (1, 3, 1), (3, 1, 0), (0, 0, 3), (2, 1, 3), (3, 2, 1), (0, 0, 2), (2, 2, 2),
                                 (1, 1, 2)])
 @pytest.mark.parametrize("rk", [0, 1, 2])
