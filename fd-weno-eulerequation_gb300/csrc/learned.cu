@@ -95,6 +95,23 @@ __global__ void __launch_bounds__(kBackThreads)
   extern __shared__ __align__(16) unsigned char back_raw[];
   BackSmem &S = *reinterpret_cast<BackSmem *>(back_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long groups = (n + kGroup - 1) / kGroup;
+  auto gather = [&](long long grp) {  // the group's inputs
+    const long long s0 = grp * kGroup;
+    for (int e = tid; e < kGroup * kIn; e += kBackThreads) {
+      const int s = e / kIn, k = e - s * kIn;
+      float v = 0.0f;
+      if (s0 + s < n) {
+        const long long row = idx ? (long long)WENOFD_IX(guard, idx[s0 + s], rows) : s0 + s;
+        v = X[row * kIn + k];
+      }
+      S.x[k * kSS + s] = v;
+    }
+  };
+  // In the training loop the launch before writes the parameters, not the
+  // samples: the first group's come in beside its end.
+  if (blockIdx.x < groups) gather(blockIdx.x);
+  dev::chain_wait();
   for (int e = tid; e < kHid * kIn; e += kBackThreads) S.w1[(e / kIn) * kWS + e % kIn] = P[oW1 + e];
   for (int e = tid; e < kHid * (kWS - kIn); e += kBackThreads) S.w1[(e / 2) * kWS + kIn + (e & 1)] = 0.0f;
   for (int e = tid; e < kHid * kHid; e += kBackThreads) S.w2[e] = P[oW2 + e];
@@ -109,20 +126,13 @@ __global__ void __launch_bounds__(kBackThreads)
   // also the biases, the output layer and the loss
   float g1[7] = {0, 0, 0, 0, 0, 0, 0}, g2[4] = {0, 0, 0, 0}, gb1 = 0, gb2 = 0, g3 = 0, gs = 0;
   const int k0 = 7 * warp, kn = warp < 7 ? 7 : 1;
-  const long long groups = (n + kGroup - 1) / kGroup;
   for (long long grp = blockIdx.x; grp < groups; grp += gridDim.x) {
     const long long s0 = grp * kGroup;
-    __syncthreads();  // the last group's sums are done (and the weights are in)
-    for (int e = tid; e < kGroup * kIn; e += kBackThreads) {
-      const int s = e / kIn, k = e - s * kIn;
-      float v = 0.0f;
-      if (s0 + s < n) {
-        const long long row = idx ? (long long)WENOFD_IX(guard, idx[s0 + s], rows) : s0 + s;
-        v = X[row * kIn + k];
-      }
-      S.x[k * kSS + s] = v;
+    if (grp != blockIdx.x) {
+      __syncthreads();  // the last group's sums are done
+      gather(grp);
     }
-    __syncthreads();
+    __syncthreads();  // the weights and the group are in
     const bool valid = s0 + lane < n;
     const int u0 = 4 * warp;  // this thread's hidden units u0 .. u0 + 3 of sample `lane`
     float z1[4], z2[4];
@@ -203,6 +213,7 @@ __global__ void __launch_bounds__(kBackThreads)
       }
     }
   }
+  dev::chain_release();
   float *row = part ? part + (long long)blockIdx.x * (kParams + 1) : nullptr;
   auto emit = [&](int e, float v) {
     if (row) row[e] = v;
@@ -248,6 +259,8 @@ __global__ void __launch_bounds__(4 * kStepParams)
   __shared__ float quarter[4][kStepParams];
   const int c = threadIdx.x % kStepParams, q = threadIdx.x / kStepParams, e = blockIdx.x * kStepParams + c;
   const int first = int((long long)blocks * q / 4), last = int((long long)blocks * (q + 1) / 4);
+  dev::chain_wait();
+  dev::chain_release();
   float acc = 0.0f;
   if (e <= kParams) {
 #pragma unroll 8
@@ -916,9 +929,10 @@ int back_blocks(long long n) {
 // One backward pass over n samples: with part null the blocks add their
 // gradients into grad / loss with atomics (after zeroing them); with part
 // (room for one row of kParams + 1 floats per block) they write partials.
-// (rows: the rows of x and y that idx indexes)
+// (rows: the rows of x and y that idx indexes; chained: the launch before in the
+// stream writes nothing that the samples' gather reads, launch_chained)
 int launch_backward(const float *params, const float *x, const float *y, long long n, float *grad, float *loss,
-                    float *part, cudaStream_t s, const unsigned *idx = nullptr, long long rows = 0) {
+                    float *part, cudaStream_t s, const unsigned *idx = nullptr, long long rows = 0, bool chained = false) {
   using namespace wenofd::lrn;
   const size_t smem = sizeof(BackSmem);
   int dev = 0;
@@ -933,6 +947,11 @@ int launch_backward(const float *params, const float *x, const float *y, long lo
   if (!part && (cudaMemsetAsync(grad, 0, kParams * sizeof(float), s) != cudaSuccess ||
                 cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess))
     return WENOFD_CUDA_ERROR;
+  if (chained)
+    return wenofd::launch_chained(k_mlp_backward, back_blocks(n), kBackThreads, smem, s, params, x, y, n, 1.0f / float(n),
+                                  grad, loss, part, idx, idx ? rows : n, wenofd::guard_record()) == cudaSuccess
+               ? WENOFD_OK
+               : WENOFD_CUDA_ERROR;
   k_mlp_backward<<<back_blocks(n), kBackThreads, smem, s>>>(params, x, y, n, 1.0f / float(n), grad, loss, part, idx,
                                                             idx ? rows : n, wenofd::guard_record());
   return cudaGetLastError() == cudaSuccess ? WENOFD_OK : WENOFD_CUDA_ERROR;
@@ -1001,7 +1020,9 @@ void shuffle(std::vector<unsigned> &perm, unsigned long long &st) {
 // loss is estimated from every 16th mini-batch's loss (and the last).
 // 131,072 samples in mini-batches of 4,096, one epoch: 4.06 ms with 32 blocks a
 // mini-batch, a reduction, an Adam launch and a loss read-back each.
-// Now 1.4 ms, a third of it the shuffle on the host.
+// Now 1.23 ms: 32 times 17 us of chained launches, the rest the shuffle on the host,
+// the allocation and the copies (unchained, without the gather beside the step
+// before: 1.41).
 extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const float *dev_y, long long n, int epochs,
                                 int batch, float lr, unsigned long long seed, float *host_epoch_loss, void *stream) {
   WENOFD_TRACE("wenofd_mlp_train");
@@ -1035,11 +1056,11 @@ extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const flo
     for (long long k = 0; k < nb && rc == WENOFD_OK; ++k) {
       const long long off = k * batch;
       const long long cnt = off + batch <= n ? batch : n - off;
-      rc = launch_backward(dev_params, dev_x, dev_y, cnt, nullptr, nullptr, part, s, perm_dev + off, n);
+      rc = launch_backward(dev_params, dev_x, dev_y, cnt, nullptr, nullptr, part, s, perm_dev + off, n, k > 0);
       if (rc != WENOFD_OK) break;
-      k_train_step<<<(kParams + kStepParams) / kStepParams, 4 * kStepParams, 0, s>>>(part, back_blocks(cnt), dev_params, m, v,
-                                                                                    ++step, lr, losses + k);
-      if (cudaGetLastError() != cudaSuccess) rc = WENOFD_CUDA_ERROR;
+      if (wenofd::launch_chained(k_train_step, (kParams + kStepParams) / kStepParams, 4 * kStepParams, 0, s, part,
+                                 back_blocks(cnt), dev_params, m, v, ++step, lr, losses + k) != cudaSuccess)
+        rc = WENOFD_CUDA_ERROR;
     }
     if (rc == WENOFD_OK && host_epoch_loss) {
       if (cudaMemcpyAsync(host_losses.data(), losses, sizeof(float) * size_t(nb), cudaMemcpyDeviceToHost, s) !=
