@@ -98,6 +98,12 @@ WENOFD_HD float bits_float(u32 u) {
 #endif
 }
 
+// A seed in [1/2, 1) as 2^32 times itself.  The exact value lies in that interval,
+// but an approximation may fall short of 1/2 by its error; unclamped, its exponent
+// would be read as part of the fraction, off by a factor of two.  (At the upper
+// end the callers keep clear of 1.)  2^8 times the bits drops the exponent field.
+WENOFD_HD u32 seed_fixed(u32 bits) { return (bits < 0x3f000000u ? 0x3f000000u : bits) * 256u + 0x80000000u; }
+
 // x is a zero or |x| in [2^lo, 2^hi) (exponents unbiased)
 template <int LO, int HI>
 WENOFD_HD bool in_range(double x) {
@@ -160,9 +166,10 @@ struct IntDivisor {
     X = (u & 0xfffffffffffffull) | 0x10000000000000ull;
     const u64 XL = X << 11;  // in [2^63, 2^64)
     const u32 xh = u32(XL >> 32), xl = u32(XL);
-    // seed: 1 / (the leading 24 bits of the significand, rounded up), below 1
-    const float r = rcp_seed(bits_float(0x3f800001u + ((xh >> 8) & 0x7fffffu)));
-    const u32 y0 = (float_bits(r) << 8) | 0x80000000u;  // 2^32 / significand
+    // seed: 1 / (the leading 24 bits of the significand, rounded up by two), below
+    // 1 whatever its error
+    const float r = rcp_seed(bits_float(0x3f800002u + ((xh >> 8) & 0x7fffffu)));
+    const u32 y0 = seed_fixed(float_bits(r));  // 2^32 / significand
     const u64 P = u64(xh) * y0 + ((u64(xl) * y0) >> 32);                   // 2^63 (1 - e)
     const int E = int((long long)(0x8000000000000000ull - P) >> 11);       // e 2^52
     const u64 Y1 = (u64(y0) << 32) + u64(((long long)(int(y0 >> 1)) * E) >> 19);
@@ -208,7 +215,7 @@ WENOFD_HD double int_sqrt(double x) {
   const u64 A = M << 10;                                                 // f 2^62
   const u32 f32 = (u32(u >> 29) & 0x7fffffu) + (odd ? 0x40000001u : 0x3f800001u);
   const u32 yb = float_bits(rsqrt_seed(bits_float(f32)));
-  const u32 y = ((yb < 0x3f7fffffu ? yb : 0x3f7fffffu) << 8) | 0x80000000u;  // 2^32 / sqrt(f)
+  const u32 y = seed_fixed(yb < 0x3f7fffffu ? yb : 0x3f7fffffu);  // 2^32 / sqrt(f)
   const u32 s0 = u32((u64(u32(A >> 32)) * y) >> 32);                         // s 2^30
   const long long R0 = (long long)(A - ((u64(s0) * s0) << 2));               // (f - s^2) 2^62
   const u64 S1 = (u64(s0) << 32) + u64(((long long)int(R0 >> 13) * int(y >> 1)) >> 19);  // s 2^62
