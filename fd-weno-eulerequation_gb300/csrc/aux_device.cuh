@@ -244,12 +244,14 @@ __device__ __noinline__ double exact_speed(double gamma, double dx, double dy, d
       return IntDivisor(dx).quotient(fabs(u) + c) + IntDivisor(dy).quotient(fabs(v) + c);
     }
   }
-  const double u = mu / rho, v = mv / rho;
-  const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
-  const double cs = sqrt(gamma * p / rho);
-  const double lx = fabs(u * 1.0 + v * 0.0) + cs;
-  const double ly = fabs(u * 0.0 + v * 1.0) + cs;
-  return lx / dx + ly / dy;
+  // Rounded operation by operation: the FP32 batches are compiled with contraction.
+  const double u = __ddiv_rn(mu, rho), v = __ddiv_rn(mv, rho);
+  const double K = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
+  const double p = __dmul_rn(gamma - 1.0, __dsub_rn(E, __dmul_rn(__dmul_rn(0.5, rho), K)));
+  const double cs = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, p), rho));
+  const double lx = __dadd_rn(fabs(__dadd_rn(u, __dmul_rn(v, 0.0))), cs);
+  const double ly = __dadd_rn(fabs(__dadd_rn(__dmul_rn(u, 0.0), v)), cs);
+  return __dadd_rn(__ddiv_rn(lx, dx), __ddiv_rn(ly, dy));
 }
 
 // FP32 estimate s32 of a node's s and a bound e with |s32 - s| <= e.  Error

@@ -145,3 +145,28 @@ def test_time_step_is_the_exact_maximum(nx, ny, precision):
                 with wenofd.Batch([s]) as b:
                     assert b.advance(1) == 1
                 assert s.info().now == want, name
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 6), (33, 65), (257, 193), (300, 411)])
+@pytest.mark.parametrize("precision", [wenofd.FP64, wenofd.FP32, wenofd.LEARNED])
+def test_batched_time_step_outside_the_integer_domain(nx, ny, precision):
+    """The first time step of a batch whose member holds values outside the
+    integer forms' exponents, against the formula as above, bit for bit: the FP64
+    instructions that take over round every operation, also in the units that
+    may contract multiply-adds."""
+    cfg = {"TESTCASE": 4, "ELEMNUMX": nx, "ELEMNUMY": ny, "RKMETH": 2, "CFL": 0.6, "SCHEME": 1, "SEED": 2,
+           "PRECISION": precision}
+    states = dict(_speed_states(nx, ny))
+    for name, U in (("huge", states["huge"]), ("mixed", states["mixed"]), ("cancelling", states["cancelling"] * 2.0 ** 140),
+                    ("thin", states["cancelling"] * 2.0 ** -150)):
+        with wenofd.Solver(cfg) as s:
+            s.initialize()
+            inf = s.info()
+            with np.errstate(all="ignore"):
+                u, v = U[1] / U[0], U[2] / U[0]
+                c = np.sqrt(inf.gamma * ((inf.gamma - 1.0) * (U[3] - 0.5 * U[0] * (u * u + v * v))) / U[0])
+                want = min(1.0, np.min(0.6 / ((np.abs(u) + c) / inf.dx + (np.abs(v) + c) / inf.dy)), inf.t_end)
+            s.set_state(U)
+            with wenofd.Batch([s]) as b:
+                assert b.advance(1) == 1
+            assert s.info().now == want, name
