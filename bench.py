@@ -493,7 +493,7 @@ def batching_leg(wenofd, precision: int, device: int, steps: int, warmup: int, p
     t0 = time.perf_counter()
     assert b.advance(steps) == steps
     t_batch = time.perf_counter() - t0
-    info = b.info()
+    info, (rows, lanes) = b.info(), b.tile()
     diff, l1 = 0.0, 0.0
     flagged, flags_differ = 0.0, 0
     for m, a in zip(members, alone):
@@ -518,7 +518,7 @@ def batching_leg(wenofd, precision: int, device: int, steps: int, warmup: int, p
             "one_at_a_time": {"value": steps * cells / t_alone, "unit": "cell-updates/s",
                               "ms_per_step": 1e3 * t_alone / steps},
             "speedup": t_alone / t_batch,
-            "autotuned": {"tile_i": info.tile_i, "blocks_per_sm": info.blocks_per_sm, "grid": info.grid,
+            "autotuned": {"tile_i": info.tile_i, "tile_rows": rows, "lanes_per_face": lanes, "blocks_per_sm": info.blocks_per_sm, "grid": info.grid,
                           "steps_per_launch": info.steps_per_launch, "graph": info.graph,
                           "tuned_ms_per_step": tuned_ms},
             "max_rel_diff_vs_one_at_a_time": diff, "max_l1_rel_diff_vs_one_at_a_time": l1}

@@ -445,6 +445,13 @@ int wenofd_batch_get_info(const wenofd_batch *b, wenofd_batch_info *info) {
   return WENOFD_OK;
 }
 
+int wenofd_batch_get_tile(const wenofd_batch *b, int *rows, int *lanes_per_face) {
+  if (!b) return fail(WENOFD_BAD_ARG, "null batch handle");
+  if (rows) *rows = b->split.rows;
+  if (lanes_per_face) *lanes_per_face = b->split.pair ? 2 : 1;
+  return WENOFD_OK;
+}
+
 int wenofd_batch_advance(wenofd_batch *b, long long max_steps, long long *steps_done) {
   WENOFD_TRACE("wenofd_batch_advance");
   if (!b) return fail(WENOFD_BAD_ARG, "null batch handle");

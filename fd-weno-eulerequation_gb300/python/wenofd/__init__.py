@@ -110,6 +110,7 @@ def lib() -> C.CDLL:
         L.wenofd_batch_autotune.argtypes = [H, C.c_int, P]
         L.wenofd_batch_advance.argtypes = [H, C.c_longlong, C.POINTER(C.c_longlong)]
         L.wenofd_batch_get_info.argtypes = [H, C.POINTER(BatchInfo)]
+        L.wenofd_batch_get_tile.argtypes = [H, C.POINTER(C.c_int), C.POINTER(C.c_int)]
         L.wenofd_batch_test_withhold.argtypes = [H, C.c_int, C.c_int]
         L.wenofd_output_variables.argtypes = [H, P]
         L.wenofd_indicator_sample.argtypes = [H, C.c_longlong, C.c_ulonglong, VP, VP, C.c_longlong,
@@ -120,7 +121,7 @@ def lib() -> C.CDLL:
         L.wenofd_bounds_report.argtypes = [C.POINTER(C.c_longlong), C.c_char_p, C.c_int, C.c_int]
         L.wenofd_bounds_selftest.argtypes = [C.POINTER(C.c_longlong), C.c_char_p, C.c_int]
         for f in ("wenofd_batch_create", "wenofd_batch_destroy", "wenofd_batch_configure", "wenofd_batch_autotune",
-                  "wenofd_batch_advance", "wenofd_batch_get_info", "wenofd_batch_test_withhold"):
+                  "wenofd_batch_advance", "wenofd_batch_get_info", "wenofd_batch_get_tile", "wenofd_batch_test_withhold"):
             getattr(L, f).restype = C.c_int
         for f in ("wenofd_create", "wenofd_create_from_file", "wenofd_destroy", "wenofd_set_stream",
                   "wenofd_get_info", "wenofd_initialize", "wenofd_fill_boundary", "wenofd_set_state",
@@ -358,6 +359,12 @@ class Batch:
         _check(lib().wenofd_batch_get_info(self._h, C.byref(i)))
         return i
 
+    def tile(self) -> tuple[int, int]:
+        """(rows, lanes per face) of the stage tiles that the batch runs."""
+        rows, lanes = C.c_int(), C.c_int()
+        _check(lib().wenofd_batch_get_tile(self._h, C.byref(rows), C.byref(lanes)))
+        return rows.value, lanes.value
+
     def test_withhold(self, block: int = 0, barrier: int = 1) -> None:
         """Arm the barrier give-up test (wenofd_batch_test_withhold)."""
         _check(lib().wenofd_batch_test_withhold(self._h, block, barrier))
@@ -373,7 +380,7 @@ EXPORTED = [
     "wenofd_routing_flags",
     "wenofd_indicator_data", "wenofd_mlp_forward", "wenofd_mlp_backward", "wenofd_mlp_adam", "wenofd_mlp_train",
     "wenofd_batch_create", "wenofd_batch_destroy", "wenofd_batch_configure", "wenofd_batch_autotune",
-    "wenofd_batch_advance", "wenofd_batch_get_info", "wenofd_batch_test_withhold", "wenofd_output_variables",
+    "wenofd_batch_advance", "wenofd_batch_get_info", "wenofd_batch_get_tile", "wenofd_batch_test_withhold", "wenofd_output_variables",
     "wenofd_save_state", "wenofd_load_state", "wenofd_indicator_sample", "wenofd_mlp_init",
     "wenofd_bounds_report", "wenofd_bounds_selftest",
 ]

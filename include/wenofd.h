@@ -262,8 +262,10 @@ int wenofd_mlp_init(float *host_params, unsigned long long seed);
  * WENO.  Weights loaded on a member reach the batch's next call.
  *
  * wenofd_batch_configure: tile rows per stage tile (FP64: 7 or 15, FP32 and
- *   learned: 15 or 31; 0 = default 15), resident blocks per SM (0 = as many
- *   as fit) and steps per launch (0 = chosen from the batch's size; learned
+ *   learned: 15 or 31; 0 = default: FP64 1 to 15 rows and one or two lanes a
+ *   face, chosen from the members' sizes and the number of SMs, learned 15, or
+ *   16 where the members have many tiles, FP32 15), resident blocks per SM (0 =
+ *   as many as fit) and steps per launch (0 = chosen from the batch's size; learned
  *   batches round it up to whole INDICATOR_INTERVAL runs of steps, each its
  *   own launch after an indicator launch).
  * wenofd_batch_autotune: times each (tile, blocks per SM) candidate over
@@ -281,7 +283,7 @@ typedef struct wenofd_batch wenofd_batch;
 typedef struct wenofd_batch_info {
   int members;
   int precision;
-  int tile_i;            /* tile rows of the stage tiles */
+  int tile_i;            /* configured tile rows; 15 for the default, whose rows wenofd_batch_get_tile gives */
   int blocks_per_sm;     /* resident blocks per SM of the persistent kernel */
   int grid;              /* blocks per launch */
   int steps_per_launch;  /* time steps one launch (learned: one graph replay) runs */
@@ -297,6 +299,9 @@ int wenofd_batch_configure(wenofd_batch *b, int tile_i, int blocks_per_sm, int s
 int wenofd_batch_autotune(wenofd_batch *b, int steps, double *ms_per_step);
 int wenofd_batch_advance(wenofd_batch *b, long long max_steps, long long *steps_done);
 int wenofd_batch_get_info(const wenofd_batch *b, wenofd_batch_info *info);
+/* The stage tiles that the batch runs: their rows, and the lanes that share a
+ * face (FP64: 1 or 2; else 1).  Either pointer may be NULL. */
+int wenofd_batch_get_tile(const wenofd_batch *b, int *rows, int *lanes_per_face);
 /* Test hook, no counterpart in the reference (whose failures abort,
  * src/WENOFD.cpp:437-442): arms the next wenofd_batch_advance to run its
  * first launch on a separately compiled instance of the batched kernel

@@ -466,3 +466,23 @@ def test_batched_ghosts_on_every_boundary(bc, rk, precision):
         assert np.max(np.abs(U - Ur)) <= tol * np.max(np.abs(Ur)), size
         s.close()
         r.close()
+
+
+@pytest.mark.parametrize("precision,nx,ny,tile_i,want", [
+    (wenofd.FP64, 800, 800, 0, (15, 1)), (wenofd.FP64, 100, 100, 15, (15, 1)), (wenofd.FP64, 100, 100, 7, (7, 1)),
+    (wenofd.FP64, 100, 100, 0, None), (wenofd.FP32, 100, 100, 0, (15, 1)), (wenofd.FP32, 100, 100, 31, (31, 1)),
+    (wenofd.LEARNED, 100, 100, 0, (15, 1)), (wenofd.LEARNED, 701, 707, 0, (16, 1)),
+    (wenofd.LEARNED, 701, 707, 15, (15, 1)), (wenofd.LEARNED, 701, 707, 31, (31, 1))])
+def test_batch_tells_the_tiles_that_it_runs(precision, nx, ny, tile_i, want):
+    """The default's tiles: FP64 short ones with two lanes a face on a grid of few
+    tiles (their exact height is the cost model's), learned 16 rows from 912
+    tiles on."""
+    with wenofd.Solver(_cfg(4, nx, ny, 1, {}, precision)) as s, wenofd.Batch([s]) as b:
+        if tile_i:
+            b.configure(tile_i=tile_i)
+        rows, lanes = b.tile()
+        assert b.info().tile_i == (tile_i or 15)
+        if want is None:
+            assert 1 <= rows < 7 and lanes == 2
+        else:
+            assert (rows, lanes) == want
