@@ -571,13 +571,14 @@ int wenofd_batch_autotune(wenofd_batch *b, int steps, double *ms_per_step) {
   int rc = WENOFD_OK;
   double best_ms = -1.0;
   int best_tile = b->tile_i, best_bps = 0;
-  // (learned form: and the default's, which may be the marching tile)
+  // FP64 and learned: and the default, whose tiles no explicit height gives (short
+  // ones with two lanes a face; the marching tile)
   const int tiles[3] = {15, b->precision == WENOFD_FP64 ? 7 : 31, 0};
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     rc = fail(WENOFD_CUDA_ERROR, "cudaEventCreate failed");
   }
   if (!rc) rc = copy_all(true);
-  for (int ti = 0; ti < (b->learned ? 3 : 2) && !rc; ++ti) {
+  for (int ti = 0; ti < (b->precision == WENOFD_FP32 ? 2 : 3) && !rc; ++ti) {
     // resident blocks per SM the kernel can take at this tile height
     if ((rc = configure(b, tiles[ti], 0, steps))) break;
     int sms = 0;

@@ -268,9 +268,10 @@ int wenofd_mlp_init(float *host_params, unsigned long long seed);
  *   as many as fit) and steps per launch (0 = chosen from the batch's size; learned
  *   batches round it up to whole INDICATOR_INTERVAL runs of steps, each its
  *   own launch after an indicator launch).
- * wenofd_batch_autotune: times each (tile, blocks per SM) candidate over
- *   `steps` steps, keeps the fastest and returns its milliseconds per step;
- *   the members' states and times are restored after every trial.
+ * wenofd_batch_autotune: times each (tile, blocks per SM) candidate, the default's
+ *   tiles and the explicit heights, over `steps` steps, keeps the fastest and
+ *   returns its milliseconds per step; the members' states and times are restored
+ *   after every trial.
  * wenofd_batch_advance: like wenofd_advance for every member: each member
  *   steps until its TEND or `max_steps` more steps (-1: no limit).
  *   *steps_done receives the largest number of steps a member took.

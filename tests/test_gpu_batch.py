@@ -486,3 +486,21 @@ def test_batch_tells_the_tiles_that_it_runs(precision, nx, ny, tile_i, want):
             assert 1 <= rows < 7 and lanes == 2
         else:
             assert (rows, lanes) == want
+
+
+def test_autotune_may_keep_the_default_split_of_small_fp64_members():
+    """Four members of 96^2: at that size a step takes 473 us with the default's
+    tiles (4 rows) and 566 with the better of 15 and 7 rows; the tuner keeps the
+    default."""
+    solvers = [wenofd.Solver(_cfg(4, 96, 96, k, {}, wenofd.FP64)) for k in range(4)]
+    try:
+        for s in solvers:
+            s.initialize()
+        with wenofd.Batch(solvers) as b:
+            default = b.tile()
+            assert default not in ((7, 1), (15, 1))
+            b.autotune(5)
+            assert b.tile() == default
+    finally:
+        for s in solvers:
+            s.close()
