@@ -89,9 +89,10 @@ __device__ __forceinline__ float dot4(const float4 a, const float4 b, float c) {
 
 // rows: with idx set, sample s of the mini-batch is row idx[s] of X and Y
 // (rows of them in all).
+template <typename Index>
 __global__ void __launch_bounds__(kBackThreads)
     k_mlp_backward(const float *P, const float *X, const float *Y, long long n, float inv_n, float *grad, float *loss,
-                   float *part, const unsigned *idx, long long rows, unsigned long long *guard) {
+                   float *part, const Index *idx, long long rows, unsigned long long *guard) {
   extern __shared__ __align__(16) unsigned char back_raw[];
   BackSmem &S = *reinterpret_cast<BackSmem *>(back_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -931,16 +932,19 @@ int back_blocks(long long n) {
 // (room for one row of kParams + 1 floats per block) they write partials.
 // (rows: the rows of x and y that idx indexes; chained: the launch before in the
 // stream writes nothing that the samples' gather reads, launch_chained)
+template <typename Index>
 int launch_backward(const float *params, const float *x, const float *y, long long n, float *grad, float *loss,
-                    float *part, cudaStream_t s, const unsigned *idx = nullptr, long long rows = 0, bool chained = false) {
+                    float *part, cudaStream_t s, const Index *idx = nullptr, long long rows = 0, bool chained = false) {
   using namespace wenofd::lrn;
+  void (*const kernel)(const float *, const float *, const float *, long long, float, float *, float *, float *,
+                       const Index *, long long, unsigned long long *) = k_mlp_backward<Index>;
   const size_t smem = sizeof(BackSmem);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return WENOFD_CUDA_ERROR;
   static unsigned long long configured = 0;  // one bit per device
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(configured & bit)) {
-    if (cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
       return WENOFD_CUDA_ERROR;
     configured |= bit;
   }
@@ -948,12 +952,12 @@ int launch_backward(const float *params, const float *x, const float *y, long lo
                 cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess))
     return WENOFD_CUDA_ERROR;
   if (chained)
-    return wenofd::launch_chained(k_mlp_backward, back_blocks(n), kBackThreads, smem, s, params, x, y, n, 1.0f / float(n),
-                                  grad, loss, part, idx, idx ? rows : n, wenofd::guard_record()) == cudaSuccess
+    return wenofd::launch_chained(kernel, back_blocks(n), kBackThreads, smem, s, params, x, y, n, 1.0f / float(n), grad,
+                                  loss, part, idx, idx ? rows : n, wenofd::guard_record()) == cudaSuccess
                ? WENOFD_OK
                : WENOFD_CUDA_ERROR;
-  k_mlp_backward<<<back_blocks(n), kBackThreads, smem, s>>>(params, x, y, n, 1.0f / float(n), grad, loss, part, idx,
-                                                            idx ? rows : n, wenofd::guard_record());
+  kernel<<<back_blocks(n), kBackThreads, smem, s>>>(params, x, y, n, 1.0f / float(n), grad, loss, part, idx,
+                                                    idx ? rows : n, wenofd::guard_record());
   return cudaGetLastError() == cudaSuccess ? WENOFD_OK : WENOFD_CUDA_ERROR;
 }
 
@@ -962,7 +966,8 @@ int launch_backward(const float *params, const float *x, const float *y, long lo
 extern "C" int wenofd_mlp_backward(const float *dev_params, const float *dev_x, const float *dev_y, long long n,
                                    float *dev_grad, float *dev_loss, void *stream) {
   if (!dev_params || !dev_x || !dev_y || !dev_grad || !dev_loss || n <= 0) return WENOFD_BAD_ARG;
-  return launch_backward(dev_params, dev_x, dev_y, n, dev_grad, dev_loss, nullptr, static_cast<cudaStream_t>(stream));
+  return launch_backward<unsigned>(dev_params, dev_x, dev_y, n, dev_grad, dev_loss, nullptr,
+                                   static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int wenofd_mlp_adam(float *dev_params, const float *dev_grad, float *dev_m, float *dev_v, int step,
@@ -991,10 +996,11 @@ inline unsigned mod_by(unsigned long long z, unsigned d) {
 // Fisher-Yates with splitmix64, from the last entry down.  The draws of a block
 // of entries are formed before its swaps, so that their arithmetic overlaps
 // (131,072 entries 710 -> 440 us on the GPU's host).
-void shuffle(std::vector<unsigned> &perm, unsigned long long &st) {
+template <typename Index>
+void shuffle(std::vector<Index> &perm, unsigned long long &st) {
   constexpr unsigned long long kStep = 0x9E3779B97F4A7C15ULL;
   constexpr int kBlock = 64;
-  unsigned pick[kBlock];
+  Index pick[kBlock];
   for (long long r = static_cast<long long>(perm.size()) - 1; r > 0;) {
     const int count = int(std::min<long long>(r, kBlock));
     for (int k = 0; k < count; ++k) {
@@ -1002,15 +1008,14 @@ void shuffle(std::vector<unsigned> &perm, unsigned long long &st) {
       z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
       z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
       z ^= z >> 31;
-      pick[k] = mod_by(z, static_cast<unsigned>(r - k + 1));
+      const unsigned long long left = static_cast<unsigned long long>(r - k + 1);
+      pick[k] = left <= 0xffffffffu ? mod_by(z, static_cast<unsigned>(left)) : static_cast<Index>(z % left);
     }
     st += kStep * static_cast<unsigned long long>(count);
     for (int k = 0; k < count; ++k) std::swap(perm[r - k], perm[pick[k]]);
     r -= count;
   }
 }
-
-}  // namespace
 
 // Training loop: per epoch a seeded permutation of the samples (so the data
 // may come in any order, e.g. grouped by snapshot and node), cut into
@@ -1023,26 +1028,23 @@ void shuffle(std::vector<unsigned> &perm, unsigned long long &st) {
 // Now 1.23 ms: 32 times 17 us of chained launches, the rest the shuffle on the host,
 // the allocation and the copies (unchained, without the gather beside the step
 // before: 1.41).
-extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const float *dev_y, long long n, int epochs,
-                                int batch, float lr, unsigned long long seed, float *host_epoch_loss, void *stream) {
-  WENOFD_TRACE("wenofd_mlp_train");
+template <typename Index>
+int train(float *dev_params, const float *dev_x, const float *dev_y, long long n, int epochs, int batch, float lr,
+          unsigned long long seed, float *host_epoch_loss, cudaStream_t s) {
   using namespace wenofd::lrn;
-  if (!dev_params || !dev_x || !dev_y || n <= 0 || epochs < 1 || batch < 1) return WENOFD_BAD_ARG;
-  if (n > 0xffffffffLL) return WENOFD_BAD_ARG;  // 32-bit row indices (as many rows take 860 GB)
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const long long nb = (n + batch - 1) / batch;
-  // m | v | the mini-batches' losses | the backward blocks' partial rows | permutation
+  // permutation | m | v | the mini-batches' losses | the backward blocks' partial rows
   const size_t part_floats = size_t(back_blocks(std::min<long long>(batch, n))) * (kParams + 1);
-  float *buf = nullptr;
-  if (cudaMalloc(&buf, sizeof(float) * (2 * kParams + size_t(nb) + part_floats + size_t(n))) != cudaSuccess)
+  Index *perm_dev = nullptr;
+  if (cudaMalloc(&perm_dev, sizeof(Index) * size_t(n) + sizeof(float) * (2 * kParams + size_t(nb) + part_floats)) !=
+      cudaSuccess)
     return WENOFD_CUDA_ERROR;
-  float *m = buf, *v = m + kParams, *losses = v + kParams, *part = losses + nb;
-  unsigned *perm_dev = reinterpret_cast<unsigned *>(part + part_floats);
+  float *m = reinterpret_cast<float *>(perm_dev + n), *v = m + kParams, *losses = v + kParams, *part = losses + nb;
   int rc = WENOFD_OK;
   if (cudaMemsetAsync(m, 0, sizeof(float) * 2 * kParams, s) != cudaSuccess) rc = WENOFD_CUDA_ERROR;
-  std::vector<unsigned> perm(static_cast<size_t>(n));
+  std::vector<Index> perm(static_cast<size_t>(n));
   std::vector<float> host_losses(host_epoch_loss ? size_t(nb) : 0);
-  for (long long r = 0; r < n; ++r) perm[r] = unsigned(r);
+  for (long long r = 0; r < n; ++r) perm[r] = Index(r);
   unsigned long long st = seed ? seed : 0x9E3779B97F4A7C15ULL;
   int step = 0;
   for (int e = 0; e < epochs && rc == WENOFD_OK; ++e) {
@@ -1050,7 +1052,7 @@ extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const flo
     // the previous epoch's mini-batches read the permutation buffer: copy
     // after they ran (same stream; the copy from pageable memory returns
     // once the host buffer is staged)
-    if (cudaMemcpyAsync(perm_dev, perm.data(), sizeof(unsigned) * size_t(n), cudaMemcpyHostToDevice, s) !=
+    if (cudaMemcpyAsync(perm_dev, perm.data(), sizeof(Index) * size_t(n), cudaMemcpyHostToDevice, s) !=
         cudaSuccess)
       rc = WENOFD_CUDA_ERROR;
     for (long long k = 0; k < nb && rc == WENOFD_OK; ++k) {
@@ -1080,6 +1082,19 @@ extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const flo
     }
   }
   if (cudaStreamSynchronize(s) != cudaSuccess) rc = WENOFD_CUDA_ERROR;
-  cudaFree(buf);
+  cudaFree(perm_dev);
   return rc;
+}
+
+}  // namespace
+
+extern "C" int wenofd_mlp_train(float *dev_params, const float *dev_x, const float *dev_y, long long n, int epochs,
+                                int batch, float lr, unsigned long long seed, float *host_epoch_loss, void *stream) {
+  WENOFD_TRACE("wenofd_mlp_train");
+  if (!dev_params || !dev_x || !dev_y || n <= 0 || epochs < 1 || batch < 1) return WENOFD_BAD_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // 32-bit row indices (half the copy and the gather's loads) as far as they reach
+  return n <= 0xffffffffLL
+             ? train<unsigned>(dev_params, dev_x, dev_y, n, epochs, batch, lr, seed, host_epoch_loss, s)
+             : train<unsigned long long>(dev_params, dev_x, dev_y, n, epochs, batch, lr, seed, host_epoch_loss, s);
 }

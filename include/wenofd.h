@@ -224,7 +224,8 @@ int wenofd_indicator_sample(wenofd_solver *s, long long per_snapshot, unsigned l
  *          (may be NULL); each mini-batch's gradient is summed in a fixed
  *          order, so the same data and seed give the same parameters bit for
  *          bit (the standalone backward accumulates with atomics).  It
- *          allocates its optimiser state and an 8-byte index per sample. */
+ *          allocates its optimiser state and a 4-byte index per sample (8 bytes
+ *          from 2^32 samples on). */
 int wenofd_mlp_forward(const float *dev_params, const float *dev_x, long long n, float *dev_logits, void *stream);
 int wenofd_mlp_backward(const float *dev_params, const float *dev_x, const float *dev_y, long long n,
                         float *dev_grad, float *dev_loss, void *stream);

@@ -102,3 +102,18 @@ def test_bounds_report_release_and_checked_exports():
     L = ctypes.CDLL(checked)
     for name in wenofd.EXPORTED:
         assert hasattr(L, name), name
+
+
+def test_training_takes_more_samples_than_32_bits_count():
+    """2^32 samples are no bad argument; without a GPU the first allocation fails
+    (nothing is read: with one this call would train on these addresses)."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    if torch.cuda.is_available():
+        pytest.skip("for a machine without a GPU")
+    fake = C.c_void_p(256)
+    train = wenofd.lib().wenofd_mlp_train
+    for n in (1 << 32, (1 << 32) - 1, 1):
+        assert train(fake, fake, fake, n, 1, 4096, 1e-3, 1, None, None) == wenofd.CUDA_ERROR
+    assert train(fake, fake, fake, 0, 1, 4096, 1e-3, 1, None, None) == wenofd.BAD_ARG
