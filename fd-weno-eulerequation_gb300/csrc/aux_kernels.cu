@@ -308,7 +308,9 @@ __global__ void k_copy_state(Geom g, double *U, double *dense, int in) {
   for (long long row = (long long)blockIdx.x * warps + (threadIdx.x >> 5); row < rows;
        row += (long long)gridDim.x * warps) {
     const int r = int(row / g.nx), i = int(row - (long long)r * g.nx);
-    double *u = U + dev::at(g, r, kGhost + i, kGhost), *d = dense + row * g.ny;
+    const long long first = dev::at(g, r, kGhost + i, kGhost);
+    double *u = U + WENOFD_SPAN(g.guard, first, first + g.ny - 1, 4 * g.plane);
+    double *d = dense + WENOFD_SPAN(g.guard, row * g.ny, (row + 1) * g.ny - 1, rows * g.ny);
     const double *src = in ? d : u;
     double *dst = in ? u : d;
     for (int j0 = 0; j0 < g.ny; j0 += 128) {
@@ -316,12 +318,12 @@ __global__ void k_copy_state(Geom g, double *U, double *dense, int in) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int j = j0 + 32 * k + lane;
-        if (j < g.ny) v[k] = src[j];
+        if (j < g.ny) v[k] = src[WENOFD_IX(g.guard, j, g.ny)];
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int j = j0 + 32 * k + lane;
-        if (j < g.ny) dst[j] = v[k];
+        if (j < g.ny) dst[WENOFD_IX(g.guard, j, g.ny)] = v[k];
       }
     }
   }
