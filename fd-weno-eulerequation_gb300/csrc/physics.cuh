@@ -631,7 +631,7 @@ __device__ __forceinline__ bool face_flux_f64(int dir, bool pair, double gamma, 
     // the - side is mirrored: from its last node down
     const double *f = side == 0 ? fp : fm + 4 * ss;
     const int step = side == 0 ? ss : -ss;
-    double x[4][5];
+    double x[4][5] = {};  // (the first four shifts move what no node has set yet)
 #pragma unroll 1
     for (int q = 0; q < 5; ++q, f += step) {
 #pragma unroll
