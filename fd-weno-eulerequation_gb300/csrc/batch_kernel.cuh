@@ -103,7 +103,9 @@ struct Nothing {
 // the barrier first took two each: a phase of 281 tiles on 304 blocks ran two
 // tiles one after the other.)  f(local item, member)
 // runs with the whole block for items of active members, with the member's
-// record staged in shared memory (sM).
+// record staged in shared memory (sM).  The barrier at the top keeps a call's
+// first claim behind every thread's last look at the claims of the call before
+// (calls with one type of f share them).
 template <typename F>
 __device__ __forceinline__ void for_member_items(const BatchArgs &b, unsigned *counter, const int *prefix,
                                                  BatchMember &sM, F f) {
@@ -118,6 +120,7 @@ __device__ __forceinline__ void for_member_items(const BatchArgs &b, unsigned *c
     }
   };
   const int blocks = int(gridDim.x);
+  __syncthreads();
   if (threadIdx.x == 0) resolve(0, int(blockIdx.x));
   __syncthreads();
   int cur = -1;
