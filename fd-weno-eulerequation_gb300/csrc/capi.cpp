@@ -105,6 +105,7 @@ int stage_buffer(const wenofd_solver *s, const double *in) { return in == s->A ?
 
 int sync(wenofd_solver *s) {
   CUDA_TRY(cudaStreamSynchronize(s->stream));
+  s->lent = false;
   return WENOFD_OK;
 }
 
@@ -269,6 +270,7 @@ int download(wenofd_solver *s, const double *dev_full, double *dst, cudaMemcpyKi
 // device cannot be given (another device's, the host's, a start that is no
 // multiple of 8 bytes) takes the strided copies.
 int copy_device(wenofd_solver *s, double *dense, bool in) {
+  s->lent = true;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, dense) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
       at.device == s->device && reinterpret_cast<uintptr_t>(dense) % 8 == 0) {
@@ -624,8 +626,12 @@ int wenofd_set_time(wenofd_solver *s, double now) {
   CUDA_TRY(wenofd::launch_set_time(s->ctrl, now, s->stream));
   // In stream order like wenofd_set_state_device: what follows on this stream,
   // or in a batch (which waits for its members' streams), sees it.  A wait here
-  // cost each call about 20 us, 32 times per pass over a batch of 32.  A stream
-  // under capture is refused by the wait, as before.
+  // cost each call about 20 us, 32 times per pass over a batch of 32.  It stays on
+  // the handle's own stream while a copy from or to a caller's device array may
+  // still run: a caller has no other stream to order its next use of that array
+  // by, and this call's return has always been the copy's end.  A stream under
+  // capture is refused by the wait, as before.
+  if (s->lent && s->stream == s->own_stream) return sync(s);
   cudaStreamCaptureStatus capture;
   CUDA_TRY(cudaStreamIsCapturing(s->stream, &capture));
   return capture == cudaStreamCaptureStatusNone ? WENOFD_OK : sync(s);

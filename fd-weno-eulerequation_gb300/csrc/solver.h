@@ -14,6 +14,7 @@ struct wenofd_solver {
   int device = 0;
   cudaStream_t stream = nullptr;      // stream in use
   cudaStream_t own_stream = nullptr;  // created by the handle
+  bool lent = false;  // a copy from or to a caller's device array may still run
   int testcase = 0, nx = 0, ny = 0, rk = 2, scheme = 1, precision = 0, tile_i = 0;
   int stage_rows = 15;  // rows of the stage tiles (wenofd::stage_rows)
   double cfl = 0.5;

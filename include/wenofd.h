@@ -102,11 +102,17 @@ int wenofd_initialize(wenofd_solver *s);
 /* Upload / download the interior state (host pointers, [4][NX][NY]). */
 int wenofd_set_state(wenofd_solver *s, const double *host_state);
 int wenofd_get_state(wenofd_solver *s, double *host_state);
-/* Same with device pointers (no host round trip; stream-ordered). */
+/* Same with device pointers (no host round trip), stream-ordered: the copy may
+ * still run on return.  Work on the handle's stream comes after it; on the
+ * handle's own stream the next call that waits ends it (wenofd_set_time and
+ * wenofd_get_info among them). */
 int wenofd_set_state_device(wenofd_solver *s, const double *dev_state);
 int wenofd_get_state_device(wenofd_solver *s, double *dev_state);
 /* Full state including the 4 ghost layers, [4][NX+8][NY+8] (host). */
 int wenofd_get_state_ghosted(wenofd_solver *s, double *host_full);
+/* Sets the time, stream-ordered.  On the handle's own stream it returns after a
+ * copy of wenofd_set_state_device or wenofd_get_state_device has ended; on a
+ * caller's stream (wenofd_set_stream) it does not wait. */
 int wenofd_set_time(wenofd_solver *s, double now);
 
 /* Values of SPECIAL boundaries (getU0 at fixed boundary nodes,

@@ -107,3 +107,24 @@ def test_device_state_round_trip(nx, ny, offset):
         got = dst.cpu().numpy()
     assert np.array_equal(got[offset:offset + n], U.ravel())
     assert np.all(got[:offset] == -2.0) and np.all(got[offset + n:] == -2.0)
+
+
+def test_set_time_ends_device_copies_of_the_own_stream():
+    """On the handle's own stream, to which a caller can order nothing, its device
+    arrays are its own again when wenofd_set_time returns: what it writes to the
+    one handed in, or reads from the one filled, on another stream is no race."""
+    torch = pytest.importorskip("torch")
+    n = 2048
+    U = torch.rand((4, n, n), dtype=torch.float64, device="cuda") + 1.0
+    x, y = U.clone(), torch.zeros_like(U)
+    torch.cuda.synchronize()
+    with wenofd.Solver({"TESTCASE": 5, "ELEMNUMX": n, "ELEMNUMY": n, "RKMETH": 2, "CFL": 0.5, "SCHEME": 1}) as s:
+        lib = wenofd.lib()
+        assert lib.wenofd_set_state_device(s.handle, x.data_ptr()) == wenofd.OK
+        s.set_time(0.25)
+        x.fill_(-1.0)
+        assert lib.wenofd_get_state_device(s.handle, y.data_ptr()) == wenofd.OK
+        s.set_time(0.5)
+        assert torch.equal(y, U)
+        assert s.info().now == 0.5
+        assert np.array_equal(s.get_state(), U.cpu().numpy())
