@@ -257,8 +257,8 @@ int configure(wenofd_batch *b, int tile_i, int blocks_per_sm, int steps_per_laun
   }
   if (b->learned && tile_i == 0) {
     // the 16 x 32 marching tile where the members' tiles fill the resident blocks
-    // one and a half times, the rule and the reason of the single solve's
-    // stage_rows
+    // one and a half times, the single solve's rule for it (stage_rows).  The 7-row
+    // tiles that a single solve takes on small grids have no batched instance.
     long long tiles = 0;
     for (const wenofd_solver *s : b->members) tiles += ceil_div(s->nx, 16) * ceil_div(s->ny, 32);
     if (tiles > 3LL * 4 * 152 / 2) b->split.rows = 16;

@@ -36,8 +36,14 @@ struct Geom {
   unsigned long long *guard;
 };
 
-// Device-resident control block of the time loop.  All fields are written
-// by single-thread control kernels or by the host between launches.
+// Device-resident control block of the time loop.  Written by single-thread
+// control kernels, by the host between launches, by the last block to arrive in a
+// time-step refinement (k_dt_refine: dt or the error, the reduction's words back
+// to zero) and in a step's last stage (finish_step: time, step count, done, the
+// next step's gate), and in a batch by the block that releases a grid barrier.
+// Within a launch only the reduction's words, the arrivals and wait_error are
+// written by many blocks (atomics); finish_step may change `active` while the
+// stage runs, after every block has passed its gate.
 struct Ctrl {
   double now, t_end, cfl, dt;
   unsigned long long max_s_bits;  // max over nodes of lx/dx + ly/dy, as IEEE bits (all >= 0)
