@@ -53,6 +53,21 @@ def test_warmup_below_three_is_rejected():
     assert "--warmup" in r.stderr
 
 
+def test_roofline_names_the_stage_kernel_that_runs():
+    """The default tile at the bench's size is the marching one, and the committed
+    traffic under its key is of that kernel; explicit heights and small grids take
+    the other tile."""
+    import bench
+
+    name, key = bench.stage_kernel(4096, 0)
+    assert name.startswith("k_stage_routed")
+    record = bench.committed_traffic()[key]
+    assert record["kernel"].startswith("k_stage_routed") and "k_stage_routed" in record["command"]
+    assert record["dram_bytes_per_launch"] == pytest.approx(4096 ** 2 * 256 / 3, rel=0.01)  # 256 B a node and RK3 step
+    for n, tile_i in ((4096, 15), (4096, 31), (512, 0)):
+        assert bench.stage_kernel(n, tile_i)[0].startswith("k_stage<float")
+
+
 @pytest.mark.gpu
 def test_kernel_tour_runs():
     """Every kernel of the path once at a small size (the per-kernel counter
