@@ -17,9 +17,9 @@
 //
 // Bound of the FP32 form: issue and the FMA pipe.  With the reconstruction on
 // the stencil's differences, eigenvector rows sharing Q and D and bare hardware
-// reciprocals (physics.cuh) a node takes 1,364 thread instructions a stage
-// instead of 2,725; stage 1 at 2048^2 (WENO-Z) 283 -> 212 us, FMA pipe 56 %,
-// issue 69 %.
+// reciprocals (physics.cuh) a node takes 1,250 thread instructions in stage 1
+// instead of 2,725; stage 1 at 2048^2 (WENO-Z) 283 -> 206 us, FMA pipe 58 %,
+// issue 65 %.
 #pragma once
 
 #include "aux_device.cuh"

@@ -136,8 +136,9 @@ __device__ __forceinline__ void stage_tile_f64(const Geom &g, const StageArgs &a
   // (WENO-Z, one stage): all arithmetic on the FP64 pipe 98.7 M warp
   // instructions on it and 6.11 ms; with fewer operations, still all there, 79.9
   // M and 4.95 ms; with products, quotients and roots on the integer pipes 33.0
-  // M and 2.47 ms (FP64 pipe at 82 % of the rate it reaches, ALU pipe 56 %).
-  // 4096^2 SSP-RK3 step: 285 -> 115 ms.
+  // M and 2.47 ms.  Counters at 2048^2, 9.39 ms: FP64 pipe at 84 % of the rate it
+  // reaches, ALU pipe 58 %, FMA pipe 22 %, issue 50 %.  4096^2 SSP-RK3 step: 285 ->
+  // 112 ms.
   constexpr int PPT = (TI * TJ + NT - 1) / NT;
   T rhs[PPT][4];
 #pragma unroll
